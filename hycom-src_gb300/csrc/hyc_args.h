@@ -49,6 +49,7 @@ struct TileArgs {
   // advem mode (single slice)
   const double *fco, *fcn;
   double dt2;
+  double qdt2;  // 1/dt2, divided once on the host (the same IEEE quotient)
   int nfld;
   FieldDesc f[kMaxFields];
   // output: out + (fi*kdm + k)*slice; sea cells of the interior are written
@@ -70,6 +71,7 @@ struct Fct2cArgs {
   const double *uflx, *vflx, *dpn, *oneta;  // mode 0: per layer k (+k*slice); oneta may be null
   const double *fco, *fcn;                  // mode 1
   double dt2;
+  double qdt2;  // 1/dt2
   int npair;
   double *work;     // A_N * npair slices
   uint8_t *lcalc;   // npair slices

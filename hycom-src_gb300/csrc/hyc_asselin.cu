@@ -32,7 +32,7 @@ __device__ __forceinline__ long long acell(const AsselinArgs &A, long long t) {
 
 // oneta(:,:,l) = max(oneta0, 1 + pbavg(:,:,l)/pbot) (mod_asselin.F90:50-51, :114-115)
 __device__ __forceinline__ double oneta_of(const AsselinArgs &A, long long c, int l) {
-  return kmax(A.oneta0, 1.0 + A.pbavg[(long long)l * A.slice + c] / A.pbot[c]);
+  return kmax(A.oneta0, 1.0 + div_rn(A.pbavg[(long long)l * A.slice + c], A.pbot[c]));
 }
 
 // asselin_save: oneta/onetao at sea points, level n of every scalar into the
@@ -85,7 +85,7 @@ __global__ void asselin_filter_kernel(const AsselinArgs A) {
     const double on = oneta_of(A, c, nn), om = oneta_of(A, c, mm);
     A.oneta[nn * sl + c] = on;
     A.oneta[mm * sl + c] = om;
-    const double ron = __drcp_rn(om);
+    const double ron = rcp_rn(om);
     const double oon = A.onetao[nn * sl + c], oom = A.onetao[mm * sl + c];
     for (int k = 0; k < kk; k++) {
       const long long lk = k * sl + c, lm = ((long long)k + (long long)mm * kk) * sl + c,
@@ -95,7 +95,7 @@ __global__ void asselin_filter_kernel(const AsselinArgs A) {
       const double dpmidn = dpmid + q;
       A.dp[lm] = div_rcp(dpmidn, om, ron);
       if (!(dpmidn > kOnezm)) continue;
-      const double qdpmidn = __drcp_rn(dpmidn);
+      const double qdpmidn = rcp_rn(dpmidn);
       const double s = ra_scalar(A.osaln[lk], A.saln[lm], A.saln[ln], dpold, dpmid, dpnew, hra, qdpmidn);
       const double tm = ra_scalar(A.otemp[lk], A.temp[lm], A.temp[ln], dpold, dpmid, dpnew, hra, qdpmidn);
       A.saln[lm] = s;

@@ -180,10 +180,10 @@ __global__ void cn_ratio(const CnuityArgs A, int k) {
   const double u1 = mx(mx(mx(mx(d, dk[ca]), dk[cb]), dk[cja]), dk[cjb]);
   const double u2 = mx(0., mn(mn(mn(mn(d, dk[ca]), dk[cb]), dk[cja]), dk[cjb]));
   const double *f2u = W(A, W_UF2), *f2v = W(A, W_VF2);
-  W(A, W_U1)[c] = (u1 - d) / ((((pos0(f2u[c]) - neg0(f2u[c + 1])) + (pos0(f2v[c]) - neg0(f2v[c + ld]))) + kEpsilCb) *
-                              A.delt1 * A.scp2i[c]);
-  W(A, W_U2)[c] = (u2 - d) / ((((neg0(f2u[c]) - pos0(f2u[c + 1])) + (neg0(f2v[c]) - pos0(f2v[c + ld]))) - kEpsilCb) *
-                              A.delt1 * A.scp2i[c]);
+  W(A, W_U1)[c] = div_rn(u1 - d, (((pos0(f2u[c]) - neg0(f2u[c + 1])) + (pos0(f2v[c]) - neg0(f2v[c + ld]))) + kEpsilCb) *
+                                     A.delt1 * A.scp2i[c]);
+  W(A, W_U2)[c] = div_rn(u2 - d, (((neg0(f2u[c]) - pos0(f2u[c + 1])) + (neg0(f2v[c]) - pos0(f2v[c + ld]))) - kEpsilCb) *
+                                     A.delt1 * A.scp2i[c]);
 }
 
 // :442-472 at margin 3: clip the antidiffusive fluxes
@@ -240,7 +240,7 @@ __global__ void cn_rpb(const CnuityArgs A) {
   if (!cell_of(A, 2, x)) return;
   const long long c = x.c;
   if (!(A.msk[c] & kIP)) return;
-  W(A, W_U1)[c] = 1. / A.p[(long long)A.kdm * A.slice + c];
+  W(A, W_U1)[c] = rcp_rn(A.p[(long long)A.kdm * A.slice + c]);
 }
 
 // loop 77, :595-645 at margin 1: the barotropic correction fluxes of layer k.
@@ -277,7 +277,7 @@ __global__ void cn_bottom(const CnuityArgs A) {
   const long long c = x.c, sl = A.slice;
   if (!(A.msk[c] & kIP)) return;
   const int nn = A.n - 1;
-  const double q = A.pbot[c] / A.p[(long long)A.kdm * sl + c];
+  const double q = div_rn(A.pbot[c], A.p[(long long)A.kdm * sl + c]);
   for (int k = 0; k < A.kdm; k++) {
     double *d = A.dp + ((long long)k + (long long)nn * A.kdm) * sl + c;
     *d = *d * q;
@@ -462,11 +462,11 @@ __global__ void cn_btrmas(const CnuityArgs A) {
   const long long c = x.c, sl = A.slice;
   if (!(A.msk[c] & kIP)) return;
   const int nn = A.n - 1;
-  const double cnt = A.p[(long long)A.kdm * sl + c] / A.pbot[c];
+  const double cnt = div_rn(A.p[(long long)A.kdm * sl + c], A.pbot[c]);
   A.onetacnt[c] = cnt;
   double *dn = A.dp + (long long)nn * A.kdm * sl + c;
   if (cnt > kEpsilCn) {
-    const double q = 1.0 / cnt;
+    const double q = rcp_rn(cnt);
     for (int k = 0; k < A.kdm; k++) {
       dn[(long long)k * sl] = dn[(long long)k * sl] * q;
       A.p[(long long)(k + 1) * sl + c] = A.p[(long long)k * sl + c] + dn[(long long)k * sl];

@@ -17,6 +17,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "hyc_div.cuh"
+
 namespace hyc {
 
 constexpr double kOnemu = 9806.e-12;  // 1 micrometre in Pa, mod_tsadvc.F90:236
@@ -55,17 +57,20 @@ __device__ __forceinline__ bool gt0(float x) { return x > 0.0f; }
 __device__ __forceinline__ bool klt(float a, float b) { return a < b; }
 
 // Correctly rounded q/h given r = RN(1/h) (one reciprocal per cell shared by
-// every tracer of the layer).  y0 = RN(q*r) is within 1.5 ulp; one
-// residual correction makes it faithful; a second one is Markstein's
-// theorem (y faithful, r = RN(1/h)  =>  RN(y + r*RN(q - h*y)) = RN(q/h)),
-// so the result equals IEEE q/h bit for bit for normal operands.  1 DMUL +
-// 4 DFMA instead of a full division.
+// every tracer of the layer): y = RN(q*r) and one residual correction,
+// RN(y + r*RN(q - h*y)) = RN(q/h) bit for bit for normal operands.
+// Markstein's theorem gives this for a faithful y (below 1 ulp off), which
+// RN(q*r) is where the significands satisfy q >= h.  Where q < h (take
+// 1 <= h, q < 2, ulp(q/h) = 2^-53), y may be up to (q+1)/2 < 1.5 ulp off.
+// With q/h = m + K*2^-106/h, m a midpoint and K odd, rounding to the wrong
+// side of m needs |K| < 2|RN(e) - e|*2^105 + 2|RN(e)|*|r - 1/h|*h*2^105 for the
+// residual e: with y at the nearer distance of 1/2 ulp from m, e is exact
+// and the bound is below 1, and |K| >= 1; at 3/2 ulp it is below 2 + 3, but
+// y lies there only if q >= 2 - |K|*2^-52/h, and q <= h - 2^-52 < 2 - 2^-52 then
+// requires |K| >= 5.  1 DMUL + 2 DFMA.
 __device__ __forceinline__ double div_rcp(double q, double h, double r) {
-  double y = __dmul_rn(q, r);
-  double e = __fma_rn(-y, h, q);
-  y = __fma_rn(e, r, y);
-  e = __fma_rn(-y, h, q);
-  return __fma_rn(e, r, y);
+  const double y = __dmul_rn(q, r);
+  return __fma_rn(__fma_rn(-y, h, q), r, y);
 }
 
 }  // namespace hyc

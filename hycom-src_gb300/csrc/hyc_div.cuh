@@ -1,0 +1,156 @@
+// hyc_div.cuh -- IEEE double division (round to nearest) on the integer pipes.
+//
+// GB300 issues FP64 at about 1/70 of the FP32 rate (1.6 operations per SM
+// and clock), so a hardware double division, a chain of dependent FP64
+// FMAs, holds the FP64 pipe longer than the ~60 integer instructions of a
+// long division hold the integer pipes -- and the FP64 pipe is what bounds
+// the kernels that divide.  div_rn forms the same correctly rounded
+// quotient with no FP64 operation: 287e9 divisions/s against the hardware
+// division's 69e9 in a loop of nothing else.  In the kernels (FCT2 on
+// 4500x3298x41: 179.7 -> 139.3 ms; cnuity on 1500x1100x41: 25.0 -> 20.1 ms;
+// the tracer step there: 42.2 -> 34.0 ms) it comes with the three-operation
+// div_rcp of hyc_device.cuh.
+//
+// Method: schoolbook long division of the 53-bit significands in two digits
+// (31 and 27 bits), each digit estimated from a 32-bit reciprocal that is
+// never too large (hardware FP32 seed, one integer Newton step), then one
+// exact remainder comparison.  With N/m in [1,2) (N the dividend's
+// significand, doubled when it is the smaller):
+//   R  in (r-6.1, r],  r = 2^84/m            (32 bits)
+//   Q1 in (t-8.1, t],  t = N*2^30/m          remainder N*2^30 - Q1*m < 8.1 m
+//   Q2 within 1.3 below the second digit      remainder < 1.3 m
+// so floor(N*2^53/m) = Q1*2^23 + Q2 + (remainder >= m), 54 bits, and the
+// result is that number rounded at its last bit (a tie would need m to be a
+// multiple of 2^53).  The remainders are small, so 64-bit arithmetic modulo
+// 2^64 holds them.  Operands outside 2^-500 .. 2^500 (other than a zero
+// dividend) take the hardware division, which covers infinities, NaNs,
+// subnormals and over- and underflow.
+#pragma once
+#include <cstdint>
+#include <cstring>
+
+#ifdef __CUDACC__
+#define HYC_HD __host__ __device__ __forceinline__
+#else
+#define HYC_HD inline
+#endif
+
+namespace hyc {
+
+namespace idiv {
+
+HYC_HD uint32_t f2u(float f) {
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(f);
+#else
+  uint32_t u;
+  memcpy(&u, &f, 4);
+  return u;
+#endif
+}
+HYC_HD float u2f(uint32_t u) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(u);
+#else
+  float f;
+  memcpy(&f, &u, 4);
+  return f;
+#endif
+}
+HYC_HD uint64_t bits(double x) {
+#ifdef __CUDA_ARCH__
+  return (uint64_t)__double_as_longlong(x);
+#else
+  uint64_t u;
+  memcpy(&u, &x, 8);
+  return u;
+#endif
+}
+HYC_HD double from_bits(uint64_t u) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)u);
+#else
+  double x;
+  memcpy(&x, &u, 8);
+  return x;
+#endif
+}
+HYC_HD uint32_t mulhi(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+  return __umulhi(a, b);
+#else
+  return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+HYC_HD int32_t mulhi_s(int32_t a, int32_t b) {
+#ifdef __CUDA_ARCH__
+  return __mulhi(a, b);
+#else
+  return (int32_t)(((int64_t)a * b) >> 32);
+#endif
+}
+// q*m modulo 2^64
+HYC_HD uint64_t mul_lo(uint32_t q, uint64_t m) {
+  return (uint64_t)q * (uint32_t)m + ((uint64_t)(q * (uint32_t)(m >> 32)) << 32);
+}
+// FP32 reciprocal seed of x in [1,2), relative error below 2^-22 (the
+// hardware's approximate reciprocal is within 1 ulp)
+HYC_HD float seed(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return 1.0f / x;
+#endif
+}
+HYC_HD uint64_t significand(uint64_t b) { return (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull; }
+
+// 32-bit reciprocal of a significand m in [2^52, 2^53): in (r-6.1, r], r = 2^84/m.
+// The seed's argument is m's top 24 bits with the last one set: at least
+// 1 + 2^-23, so the seed is below 1 and its significand is all of R0.
+HYC_HD uint32_t recip32(uint64_t m) {
+  const float rf = seed(u2f(0x3F800001u | ((uint32_t)(m >> 29) & 0x7FFFFFu)));
+  const uint32_t R0 = 0x80000000u | (f2u(rf) << 8);
+  const uint32_t x = (uint32_t)(m >> 21);
+  // e = 2^63 - R0*x, |e| < 2^42; R0*(1 + e/2^63) is the Newton step
+  const int32_t e = (int32_t)((0x8000000000000000ull - (uint64_t)R0 * x) >> 32);
+  return R0 + (uint32_t)mulhi_s((int32_t)(R0 >> 1), e * 4) - 3u;
+}
+
+// significand of RN(N/m) (bit 52 set), N/m in [1,2), R = recip32(m)
+HYC_HD uint64_t quotient(uint64_t N, uint64_t m, uint32_t R) {
+  const uint32_t q1 = mulhi((uint32_t)(N >> 22), R);
+  const uint64_t r1 = (N << 30) - mul_lo(q1, m);
+  const uint32_t q2 = mulhi((uint32_t)(r1 >> 25), R) >> 4;
+  const uint64_t r2 = (r1 << 23) - mul_lo(q2, m);
+  const uint64_t q = ((uint64_t)q1 << 23) + q2 + (r2 >= m ? 1u : 0u);
+  return (q + 1) >> 1;
+}
+
+// exponent field in [1023-500, 1023+500): every quotient of two such values is normal
+HYC_HD bool mid_range(uint32_t hi) { return (hi & 0x7FFFFFFFu) - 0x20B00000u < 0x3E800000u; }
+
+}  // namespace idiv
+
+// a/b, correctly rounded
+HYC_HD double div_rn(double a, double b) {
+  using namespace idiv;
+  const uint64_t ia = bits(a), ib = bits(b);
+  const uint32_t ha = (uint32_t)(ia >> 32), hb = (uint32_t)(ib >> 32);
+  const bool zero = (ia << 1) == 0;
+  if (!(mid_range(hb) && (mid_range(ha) || zero))) return a / b;
+  const uint64_t ma = significand(ia), mb = significand(ib);
+  const bool less = ma < mb;
+  const uint64_t q = quotient(less ? ma << 1 : ma, mb, recip32(mb));
+  const uint32_t sgn = (ha ^ hb) & 0x80000000u;
+  // (exponent - 1) << 20, added onto the significand's own bit 52
+  const uint32_t ex = (ha & 0x7FF00000u) - (hb & 0x7FF00000u) + (less ? 0x3FD00000u : 0x3FE00000u);
+  const uint64_t r = q + ((uint64_t)(ex | sgn) << 32);
+  return from_bits(zero ? (uint64_t)sgn << 32 : r);
+}
+
+// 1/b, correctly rounded
+HYC_HD double rcp_rn(double b) { return div_rn(1.0, b); }
+
+}  // namespace hyc

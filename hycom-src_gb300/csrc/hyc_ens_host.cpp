@@ -291,6 +291,7 @@ int build_tables(hyc_ens *e, double dt2) {
         a.vflx = (const double *)b.vflx;
         a.dpn = b.dp;
         a.dt2 = dt2;
+        a.qdt2 = 1.0 / dt2;
         a.nfld = b.ntr;
         for (int q = 0; q < b.ntr; q++) {
           a.f[q].nbase = (double *)b.lev[lo] + (long long)q * b.kdm * b.slice;

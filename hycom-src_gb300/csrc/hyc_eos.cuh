@@ -34,7 +34,7 @@ __device__ __forceinline__ double sig17(double t, double s) {
   const double sn = c101 + t * (c002 + t * (c103 + t * c004)) + s * (c105 - t * c006 + s * c007);
   const double sd = c108 + t * (c109 + t * (c010 + t * (c111 + t * c012))) +
                     s * (c013 - t * (c014 + t * t * c015) + sqrt(pos0(s)) * (c016 + t * t * c017));
-  const double sq = __drcp_rn(sd);  // aone/sig_d, correctly rounded
+  const double sq = rcp_rn(sd);  // aone/sig_d, correctly rounded
   return sn * sq - 1000.0;
 }
 

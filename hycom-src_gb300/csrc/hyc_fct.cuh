@@ -169,11 +169,11 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
     FCN[t] = fcn;
     HO[t] = fco + kOnemu;
     HN[t] = hn;
-    RH[t] = __drcp_rn(hn);
+    RH[t] = rcp_rn(hn);
   }
   __syncthreads();
 
-  const double qdt2 = 1.0 / dt2;  // mod_tsadvc.F90:865
+  const double qdt2 = A.qdt2;  // mod_tsadvc.F90:865
   for (int fi = 0; fi < A.nfld; fi++) {
     const FieldDesc fd = A.f[fi];
     if (k + 1 > fd.kmax || k + 1 < fd.kmin) continue;
@@ -298,11 +298,11 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
       double rp = 0.0, rm = 0.0;
       if (gt0(famax)) {
         const double qp = (fqmax - lo) * FCN[e] * SCL[e] * qdt2;
-        rp = klt(qp, famax) ? qp / famax : 1.0;
+        rp = klt(qp, famax) ? div_rn(qp, famax) : 1.0;
       }
       if (gt0(famin)) {
         const double qm = (lo - fqmin) * FCN[e] * SCL[e] * qdt2;
-        rm = klt(qm, famin) ? qm / famin : 1.0;
+        rm = klt(qm, famin) ? div_rn(qm, famin) : 1.0;
       }
       RP[e] = rp;
       RM[e] = rm;

@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "hyc_args.h"
+#include "hyc_div.cuh"
 #include "hyc_internal.h"
 
 namespace hyc {
@@ -110,7 +111,7 @@ __global__ void fct2c_dt(Fct2cArgs A) {
   const double q = mx2(u[c + 1], 0.0) - mn2(u[c], 0.0) + mx2(v[c + ld], 0.0) - mn2(v[c], 0.0);
   double *dt = W(A, A_DTLOC, p);
   if (q > 0.0)
-    dt[c] = mn2(A.dt2, W(A, A_HLOC, p)[c] / (q * A.scali[c]));
+    dt[c] = mn2(A.dt2, div_rn(W(A, A_HLOC, p)[c], q * A.scali[c]));
   else
     dt[c] = A.dt2;
 }
@@ -180,7 +181,7 @@ __global__ void fct2c_cell(Fct2cArgs A) {
   const double *ucum = W(A, A_UCUM, p), *vcum = W(A, A_VCUM, p);
   const double qp = h[c] - (uloc[c + 1] - uloc[c] + vloc[c + ld] - vloc[c]) * A.scali[c];
   if (qp > 0.0)
-    lo[c] = ((kEps + h[c]) * lo[c] - (flx[c + 1] - flx[c] + fly[c + ld] - fly[c]) * A.scali[c]) / (kEps + qp);
+    lo[c] = div_rn((kEps + h[c]) * lo[c] - (flx[c + 1] - flx[c] + fly[c + ld] - fly[c]) * A.scali[c], kEps + qp);
   h[c] = qp;
   lc[c] = ucum[c + 1] != dt2 || ucum[c] != dt2 || vcum[c + ld] != dt2 || vcum[c] != dt2;
 }
@@ -202,13 +203,13 @@ __global__ void fct2c_anti(Fct2cArgs A) {
   const double *fxc = W(A, A_FXC, p), *fyc = W(A, A_FYC, p);
   if (m & kIU) {
     const double fhx = u[c] * 0.5 * (fc[c] + fc[c - 1]);
-    fax[c] = fhx - fxc[c] / dt2;
+    fax[c] = fhx - div_rn(fxc[c], dt2);
   } else {
     fax[c] = 0.0;
   }
   if (m & kIV) {
     const double fhy = v[c] * 0.5 * (fc[c] + fc[c - ld]);
-    fay[c] = fhy - fyc[c] / dt2;
+    fay[c] = fhy - div_rn(fyc[c], dt2);
   } else {
     fay[c] = 0.0;
   }
@@ -229,17 +230,17 @@ __global__ void fct2c_ratio(Fct2cArgs A) {
   const double fqmin = mn2(mn2(mn2(mn2(lo[c], lo[ca]), lo[cb]), lo[cja]), lo[cjb]);
   const double famax = mx2(0.0, fax[c]) - mn2(0.0, fax[c + 1]) + mx2(0.0, fay[c]) - mn2(0.0, fay[c + ld]);
   const double famin = mx2(0.0, fax[c + 1]) - mn2(0.0, fax[c]) + mx2(0.0, fay[c + ld]) - mn2(0.0, fay[c]);
-  const double qdt2 = 1.0 / A.dt2;
+  const double qdt2 = A.qdt2;
   double rp, rm;
   if (famax > kEps) {
     const double qp = (fqmax - lo[c]) * h[c] * A.scal[c] * qdt2;
-    rp = (qp < famax) ? qp / famax : 1.0;
+    rp = (qp < famax) ? div_rn(qp, famax) : 1.0;
   } else {
     rp = 0.0;
   }
   if (famin > kEps) {
     const double qm = (lo[c] - fqmin) * h[c] * A.scal[c] * qdt2;
-    rm = (qm < famin) ? qm / famin : 1.0;
+    rm = (qm < famin) ? div_rn(qm, famin) : 1.0;
   } else {
     rm = 0.0;
   }
@@ -279,7 +280,7 @@ __global__ void fct2c_update(Fct2cArgs A) {
   const double flxdiv = ((fax[c + 1] - fax[c]) + (fay[c + ld] - fay[c])) * A.dt2 * A.scali[c];
   double *f = A.fld[p];
   if (h[c] > 0.)
-    f[c] = ((kEps + h[c]) * lo[c] - flxdiv) / (kEps + h[c]);
+    f[c] = div_rn((kEps + h[c]) * lo[c] - flxdiv, kEps + h[c]);
   else
     f[c] = lo[c];
 }

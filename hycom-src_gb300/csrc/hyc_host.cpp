@@ -680,6 +680,7 @@ int hyc_advem(hyc_ctx *c, int32_t advtyp, double *fld, const double *fldc, const
     f.fco = dfco;
     f.fcn = dfcn;
     f.dt2 = dt2;
+    f.qdt2 = 1.0 / dt2;
     fct2c_bind(f, c, 1);
     f.fld[0] = dfld;
     f.fldc[0] = dfldc;
@@ -716,6 +717,7 @@ int hyc_advem(hyc_ctx *c, int32_t advtyp, double *fld, const double *fldc, const
   a.fco = dfco;
   a.fcn = dfcn;
   a.dt2 = dt2;
+  a.qdt2 = 1.0 / dt2;
   a.nfld = 1;
   a.f[0].nbase = dfld;
   a.f[0].mbase = dfldc ? dfldc : dfld;
@@ -882,6 +884,7 @@ int hyc_tsadvc(hyc_ctx *c, int32_t m, int32_t n, const hyc_tsadvc_params *p, dou
   a.dpn = F[HYC_F_DP].dev + (long long)nn * kk * sl;
   a.oneta_n = p->btrmas ? F[HYC_F_ONETA].dev + (long long)nn * sl : nullptr;
   a.dt2 = p->delt1;
+  a.qdt2 = 1.0 / p->delt1;
   a.kdm = kk;
   if (at == 2 && p->btrmas) {  // advem_fct2c per (field, layer), mod_tsadvc.F90:154-155
     std::vector<std::pair<int, int>> pairs;  // (layer, field) in the reference's call order
@@ -907,6 +910,7 @@ int hyc_tsadvc(hyc_ctx *c, int32_t m, int32_t n, const hyc_tsadvc_params *p, dou
     f.dpn = a.dpn;
     f.oneta = a.oneta_n;
     f.dt2 = p->delt1;
+    f.qdt2 = 1.0 / p->delt1;
     for (size_t p0 = 0; p0 < pairs.size(); p0 += nb) {
       const int np = (int)std::min(pairs.size() - p0, (size_t)nb);
       fct2c_bind(f, c, np);

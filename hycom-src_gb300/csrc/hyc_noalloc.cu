@@ -139,6 +139,7 @@ extern "C" int hyc_advem_noalloc(int32_t idm, int32_t jdm, int32_t nbdy, int32_t
   a.fco = fco;
   a.fcn = fcn;
   a.dt2 = dt2;
+  a.qdt2 = 1.0 / dt2;
   a.nfld = 1;
   a.f[0].nbase = fld;
   a.f[0].mbase = fldc ? fldc : fld;

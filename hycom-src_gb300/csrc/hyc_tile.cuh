@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
   for (int t = threadIdx.x; t < NR; t += blockDim.x) {
     double hn = FCN[t] + kOnemu;
     HN[t] = hn;
-    RH[t] = __drcp_rn(hn);
+    RH[t] = rcp_rn(hn);
   }
   __syncthreads();
 
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
       if (SCHEME == kMPDATA) {  // :377-381
         double fco2 = FCO[e] + FCO[e - 1];
         double fcn2 = FCN[e] + FCN[e - 1];
-        FX[e] = FXL[e] - uu * (FLDC[e] + FLDC[e - 1]) / ((fco2 + fcn2) + kOnemu);
+        FX[e] = FXL[e] - div_rn(uu * (FLDC[e] + FLDC[e - 1]), (fco2 + fcn2) + kOnemu);
       } else if (SCHEME == kFCT4 && (MSK[e - 1] & kIU) && (MSK[e + 1] & kIU)) {  // :1540-1541
         const double ft14 = 7.0 / 12.0, ft24 = -1.0 / 12.0;
         double fhx = uu * (ft14 * (FLDC[e] + FLDC[e - 1]) + ft24 * (FLDC[e + 1] + FLDC[e - 2]));
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
       if (SCHEME == kMPDATA) {  // :383-387
         double fco2 = FCO[e] + FCO[e - RX];
         double fcn2 = FCN[e] + FCN[e - RX];
-        FY[e] = FNL[e] - vv * (FLDC[e] + FLDC[e - RX]) / ((fco2 + fcn2) + kOnemu);
+        FY[e] = FNL[e] - div_rn(vv * (FLDC[e] + FLDC[e - RX]), (fco2 + fcn2) + kOnemu);
       } else if (SCHEME == kFCT4 && (MSK[e - RX] & kIV) && (MSK[e + RX] & kIV)) {  // :1551-1552
         const double ft14 = 7.0 / 12.0, ft24 = -1.0 / 12.0;
         double fhy = vv * (ft14 * (FLDC[e] + FLDC[e - RX]) + ft24 * (FLDC[e + RX] + FLDC[e - 2 * RX]));
@@ -339,8 +339,8 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
         double flydn = pos0(fy1) - neg0(fy0);
         double lo = FLO[e];
         double fs = FCN[e] * SCL[e];
-        RP[e] = (QX[e] - lo) * fs / ((kOnemu - (flxdp + flydp)) * dt2);
-        RM[e] = (lo - QN[e]) * fs / ((kOnemu + (flxdn + flydn)) * dt2);
+        RP[e] = div_rn((QX[e] - lo) * fs, (kOnemu - (flxdp + flydp)) * dt2);
+        RM[e] = div_rn((lo - QN[e]) * fs, (kOnemu + (flxdn + flydn)) * dt2);
         return;
       }
       const bool mw = MSK[e - 1] & kIP, me = MSK[e + 1] & kIP, ms = MSK[e - RX] & kIP, mn = MSK[e + RX] & kIP;
@@ -361,15 +361,15 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
       double famax = pos0(fxa) - neg0(fxb) + pos0(fya) - neg0(fyb);
       double famin = pos0(fxb) - neg0(fxa) + pos0(fyb) - neg0(fya);
       double lo = FLO[e];
-      double qdt2 = 1.0 / dt2;
+      double qdt2 = A.qdt2;
       double rp = 0.0, rm = 0.0;
       if (gt0(famax)) {
         double qp = (fqmax - lo) * FCN[e] * SCL[e] * qdt2;
-        rp = klt(qp, famax) ? qp / famax : 1.0;
+        rp = klt(qp, famax) ? div_rn(qp, famax) : 1.0;
       }
       if (gt0(famin)) {
         double qm = (lo - fqmin) * FCN[e] * SCL[e] * qdt2;
-        rm = klt(qm, famin) ? qm / famin : 1.0;
+        rm = klt(qm, famin) ? div_rn(qm, famin) : 1.0;
       }
       RP[e] = rp;
       RM[e] = rm;

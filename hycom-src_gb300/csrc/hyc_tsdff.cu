@@ -37,7 +37,7 @@ constexpr double kEpsHar = 1.0e-20;      // eps_har, mod_tsadvc.F90:1762-1763
 
 // harmonic means, mod_tsadvc.F90:1770-1771 (max on the integer pipes,
 // kmax/pos0 of hyc_device.cuh)
-__device__ __forceinline__ double harmonz(double a, double b) { return 2.0 * a * b / kmax((a + b), 2.0 * kEpsHar); }
+__device__ __forceinline__ double harmonz(double a, double b) { return div_rn(2.0 * a * b, kmax((a + b), 2.0 * kEpsHar)); }
 __device__ __forceinline__ double harmonc(double aa, double bb) { return harmonz(pos0(aa), pos0(bb)); }
 
 __device__ __forceinline__ long long cell(const TsdffArgs &A, int i, int j) {
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kThreads) tsdff_tile_kernel(const TsdffArgs A,
   for (int r = 0; r < 4; r++) {
     const int b = b0 + 8 * r, j = j0 + b;
     sea[r] = i <= A.ii && j <= A.jj && (sm[b + 1][a + 1] & kIP);
-    fac[r] = sea[r] ? -A.delt1 / (A.scp2[cell(A, i, j)] * kmax(sh[b + 1][a + 1], kEpsHar)) : 0.0;
+    fac[r] = sea[r] ? div_rn(-A.delt1, A.scp2[cell(A, i, j)] * kmax(sh[b + 1][a + 1], kEpsHar)) : 0.0;
   }
   for (int q = 0; q < A.nfld; q++) {
     const double *f = A.fld[q] + lk;
