@@ -28,6 +28,10 @@ __device__ __forceinline__ long long dkey(double x) {
   long long b = __double_as_longlong(x);
   return b ^ ((long long)((unsigned long long)(b >> 63) >> 1));
 }
+__device__ __forceinline__ double from_dkey(long long k) {  // dkey is its own inverse
+  return __longlong_as_double(k ^ (long long)((unsigned long long)(k >> 63) >> 1));
+}
+constexpr long long kOneBits = 0x3FF0000000000000LL;  // 1.0
 // max(a,b) / min(a,b) of the reference (mod_tsadvc.F90 passim)
 __device__ __forceinline__ double kmax(double a, double b) { return dkey(a) > dkey(b) ? a : b; }
 __device__ __forceinline__ double kmin(double a, double b) { return dkey(a) < dkey(b) ? a : b; }
@@ -45,6 +49,24 @@ __device__ __forceinline__ bool lt0(double x) {
 }
 __device__ __forceinline__ bool gt0(double x) { return __double_as_longlong(x) > 0; }
 __device__ __forceinline__ bool klt(double a, double b) { return dkey(a) < dkey(b); }
+
+// FP32 bounds of a double for tests that need no exact value (integer pipes:
+// a conversion instruction would issue at the FP64 rate).  Both truncate
+// (relative error below 2^-23).  f32_below: of a value >= 0, at most x, and 0
+// where x is negative, NaN or outside FP32's normal range.
+__device__ __forceinline__ float f32_below(double x) {
+  const uint32_t h = (uint32_t)__double2hiint(x);
+  const uint32_t f = __funnelshift_l((uint32_t)__double2loint(x), h, 3) + 0x40000000u;
+  return h - 0x38100000u < 0x0FE00000u ? __uint_as_float(f) : 0.0f;
+}
+// f32_away: 0 only where x is 0; below FP32's normal range the smallest
+// normal, above it (and for NaN) infinity
+__device__ __forceinline__ float f32_away(double x) {
+  const uint32_t h = (uint32_t)__double2hiint(x), l = (uint32_t)__double2loint(x), m = h & 0x7FFFFFFFu;
+  uint32_t f = __funnelshift_l(l, h, 3) + 0x40000000u;
+  if (m - 0x38100000u >= 0x0FE00000u) f = m > 0x38100000u ? 0x7F800000u : (m | l) != 0 ? 0x00800000u : 0u;
+  return __uint_as_float(f | (h & 0x80000000u));
+}
 
 // FP32 versions (FMNMX is cheap on the FP32 pipe)
 __device__ __forceinline__ float kmax(float a, float b) { return fmaxf(a, b); }

@@ -153,4 +153,54 @@ HYC_HD double div_rn(double a, double b) {
 // 1/b, correctly rounded
 HYC_HD double rcp_rn(double b) { return div_rn(1.0, b); }
 
+// R of a divisor that several dividends share; 0 sends them to the hardware division
+HYC_HD uint32_t recip_of(double b) {
+  const uint64_t ib = idiv::bits(b);
+  return idiv::mid_range((uint32_t)(ib >> 32)) ? idiv::recip32(idiv::significand(ib)) : 0u;
+}
+
+// a/b, correctly rounded, R = recip_of(b)
+HYC_HD double div_by(double a, double b, uint32_t R) {
+  using namespace idiv;
+  const uint64_t ia = bits(a), ib = bits(b);
+  const uint32_t ha = (uint32_t)(ia >> 32), hb = (uint32_t)(ib >> 32);
+  const bool zero = (ia << 1) == 0;
+  if (!(R != 0 && (mid_range(ha) || zero))) return a / b;
+  const uint64_t ma = significand(ia), mb = significand(ib);
+  const bool less = ma < mb;
+  const uint64_t q = quotient(less ? ma << 1 : ma, mb, R);
+  const uint32_t sgn = (ha ^ hb) & 0x80000000u;
+  const uint32_t ex = (ha & 0x7FF00000u) - (hb & 0x7FF00000u) + (less ? 0x3FD00000u : 0x3FE00000u);
+  const uint64_t r = q + ((uint64_t)(ex | sgn) << 32);
+  return from_bits(zero ? (uint64_t)sgn << 32 : r);
+}
+
+// a*b, correctly rounded, on the integer pipes: the 106-bit product of the
+// significands from four 32x32-bit ones (b's shifted up 11 bits, so that the
+// product's top 53 or 54 bits are its upper 64-bit half), shifted to 53 bits
+// and rounded half to even.  Operands outside 2^-500 .. 2^500 (zeros too)
+// take the FP64 multiply.
+HYC_HD double mul_rn(double a, double b) {
+  using namespace idiv;
+  const uint64_t ia = bits(a), ib = bits(b);
+  const uint32_t ha = (uint32_t)(ia >> 32), hb = (uint32_t)(ib >> 32), al = (uint32_t)ia;
+  if (!(mid_range(ha) && mid_range(hb))) return a * b;
+  const uint32_t ah = (ha & 0xFFFFFu) | 0x100000u;
+  const uint32_t bh = (hb << 11 | (uint32_t)ib >> 21) | 0x80000000u, bl = (uint32_t)ib << 11;
+  const uint64_t t0 = (uint64_t)al * bl;
+  const uint64_t t1 = (uint64_t)al * bh + (t0 >> 32);
+  const uint64_t t2 = (uint64_t)ah * bl + (uint32_t)t1;
+  const uint64_t hi = (uint64_t)ah * bh + (t1 >> 32) + (t2 >> 32);  // in [2^51, 2^53)
+  const uint32_t m = (uint32_t)t2;
+  const uint32_t up = (uint32_t)(hi >> 52);        // 1: 53 bits already
+  const uint32_t sh = 1u ^ up;
+  const uint64_t q = hi << sh | (sh & (m >> 31));  // 53 bits
+  // the rest, its sticky bits folded into the last one
+  const uint32_t rest = m << sh | ((uint32_t)t0 != 0 ? 1u : 0u);
+  const uint64_t c = ((uint64_t)rest + 0x7FFFFFFFu + ((uint32_t)q & 1u)) >> 32;
+  // exponents and signs add; -1 for the significand's own bit 52
+  const uint32_t ex = (ha & 0xFFF00000u) + (hb & 0xFFF00000u) - 0x3FF00000u - (sh << 20);
+  return from_bits(q + c + ((uint64_t)ex << 32));
+}
+
 }  // namespace hyc

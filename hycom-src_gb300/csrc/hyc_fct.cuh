@@ -34,9 +34,10 @@ struct FctGeom {
   static constexpr int RW = TX + 6, RX = TX + 8, RY = TY + 6;
   static constexpr int NR = RX * RY;                     // cells of a staged box
   static constexpr int N = (NR + 1 + 15) / 16 * 16;      // one array's slot (128-byte multiple)
-  static constexpr int NARR = 15;  // U V FCN HO HN RH SCL SCI | FLD FLDC FX FY FLO RP RM
+  // doubles U V HO HN SCI | FLD FLDC FX FY FLO RP RM, 4-byte RC QF FXF FYF, bytes MSK NBR
+  static constexpr int NARR = 12;
   static constexpr unsigned BOX = NR * 8;                // bytes of one TMA box
-  static constexpr size_t smem_bytes = 128 + (size_t)NARR * N * sizeof(double) + ((NR + 15) / 16) * 16;
+  static constexpr size_t smem_bytes = 128 + (size_t)N * (NARR * 8 + 4 * 4 + 2);
 };
 
 // Compile-time rectangle [A0,A1) x [B0,B1) of a region of width RX, spread
@@ -73,11 +74,16 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
   const int x0 = ib0 + nb - 1, y0 = jb0 + nb - 1;  // padded column / row of the region origin
   const int off = x0 & 1;                           // TMA boxes start at the even column x0 - off
   double *sal = reinterpret_cast<double *>((reinterpret_cast<uintptr_t>(sm) + 127) & ~uintptr_t(127));
-  double *U = sal + off, *V = U + N, *FCN = V + N, *HO = FCN + N, *HN = HO + N, *RH = HN + N, *SCL = RH + N,
-         *SCI = SCL + N;
+  double *U = sal + off, *V = U + N, *HO = V + N, *HN = HO + N, *SCI = HN + N;
   double *FLD = SCI + N, *FLDC = FLD + N, *FX = FLDC + N, *FY = FX + N, *FLO = FY + N, *RP = FLO + N,
          *RM = RP + N;
-  uint8_t *MSK = reinterpret_cast<uint8_t *>(sal + G::NARR * N);
+  double *FCN = RP, *SCL = RM;  // staged there: dead before the first field's ratios
+  uint32_t *RC = reinterpret_cast<uint32_t *>(sal + G::NARR * N);
+  float *QF = reinterpret_cast<float *>(RC + N), *FXF = QF + N, *FYF = FXF + N;
+  uint8_t *MSK = reinterpret_cast<uint8_t *>(FYF + N), *NBR = MSK + N;
+  // fmxlo/fmnlo, as keys, in FLD/FLDC once those are dead
+  auto kmx_at = [&](int e) { return __double_as_longlong(FLD[e]); };
+  auto kmn_at = [&](int e) { return __double_as_longlong(FLDC[e]); };
   const CUtensorMap *tm = reinterpret_cast<const CUtensorMap *>(A.tmaps);
   const long long sl = A.slice;
   const double dt2 = A.dt2;
@@ -138,11 +144,18 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
     }
   }
   __syncthreads();
+  const float qdt2f = f32_below(A.qdt2);
   for (int t = threadIdx.x; t < NR; t += 256) {
     const int bb = t / RX, aa = t - bb * RX;
     double fco, fcn;
+    FX[t] = 0.0;  // faces that are not between two sea cells keep these zeros
+    FY[t] = 0.0;
+    FXF[t] = 0.0f;
+    FYF[t] = 0.0f;
+    if (aa > 0 && aa < RX - 1 && bb > 0 && bb < RY - 1)
+      NBR[t] = (MSK[t - 1] & kIP) | (MSK[t + 1] & kIP) << 1 | (MSK[t - RX] & kIP) << 2 | (MSK[t + RX] & kIP) << 3;
     if (A.mode == 0) {  // mod_tsadvc.F90:1931-1938
-      const double o = HO[t] * FCN[t];
+      const double o = A.oneta_n ? HO[t] * FCN[t] : FCN[t];  // 1.0*x == x
       double fdv = 0.0;
       if (aa < RX - 1 && bb < RY - 1) {
         if (A.ufco) {
@@ -166,14 +179,25 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
       fcn = FCN[t];
     }
     const double hn = fcn + kOnemu;
-    FCN[t] = fcn;
     HO[t] = fco + kOnemu;
     HN[t] = hn;
-    RH[t] = rcp_rn(hn);
+    RC[t] = recip_of(hn);
+    // fcn*scal/dt2 from below, 0 where FP32 could lose it
+    const float fs = f32_below(fcn) * f32_below(SCL[t]), qf = fs * qdt2f;
+    QF[t] = fs > 1e-30f && fs < 1e30f && qf > 1e-30f && qf < 1e30f ? qf : 0.0f;
   }
   __syncthreads();
 
   const double qdt2 = A.qdt2;  // mod_tsadvc.F90:865
+  // fcn and scal of a region cell again, for the few ratios that need them
+  auto cell = [&](int a, int b) { return (long long)(x0 + a) + (long long)(y0 + b) * ld1; };
+  auto fcn_of = [&](int a, int b) {
+    const long long o = cell(a, b);
+    if (A.mode != 0) return A.fcn[o];
+    const double d = A.dpn[k * sl + o];
+    return kmax(A.oneta_n ? A.oneta_n[o] * d : d, 0.0);
+  };
+  auto scl_of = [&](int a, int b) { return A.scal[cell(a, b)]; };
   for (int fi = 0; fi < A.nfld; fi++) {
     const FieldDesc fd = A.f[fi];
     if (k + 1 > fd.kmax || k + 1 < fd.kmin) continue;
@@ -187,10 +211,6 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
         tma::load3(FLD - off, tm + 6 + 2 * fi, bar, x0 - off, y0, k + fd.k_off);
         tma::load3(FLDC - off, tm + 7 + 2 * fi, bar, x0 - off, y0, k + fd.k_off);
       }
-      for (int t = threadIdx.x; t < NR; t += 256) {
-        FX[t] = 0.0;
-        FY[t] = 0.0;
-      }
       if (!landed()) return false;
     } else {
       for (int t = threadIdx.x; t < NR; t += 256) {
@@ -200,8 +220,6 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
         const long long o = in ? (long long)(i + nb - 1) + (long long)(j + nb - 1) * ld1 : 0;
         FLD[t] = in ? fn[o] : 0.0;
         FLDC[t] = in ? fm[o] : 0.0;
-        FX[t] = 0.0;
-        FY[t] = 0.0;
       }
       __syncthreads();
     }
@@ -223,18 +241,16 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
 
     // S2: low-order solution on [1,RX-1)^2, :778-791
     rect<RX, 1, RW - 1, 1, RY - 1>([&](int a, int b, int e, int) {
-      const uint8_t m = MSK[e];
-      if (!(m & kIP)) return;
+      if (!(MSK[e] & kIP)) return;
+      const int nbr = NBR[e];
       const double c = FLD[e];
-      const double w = (MSK[e - 1] & kIP) ? FLD[e - 1] : c;
-      const double ea = (MSK[e + 1] & kIP) ? FLD[e + 1] : c;
-      const double s = (MSK[e - RX] & kIP) ? FLD[e - RX] : c;
-      const double n = (MSK[e + RX] & kIP) ? FLD[e + RX] : c;
-      const double fmx = kmax(kmax(kmax(kmax(c, w), ea), s), n);
-      const double fmn = kmin(kmin(kmin(kmin(c, w), ea), s), n);
-      const double fdv = ((FX[e + 1] - FX[e]) + (FY[e + RX] - FY[e])) * dt2 * SCI[e];
-      const double q = c * HO[e] - fdv;
-      FLO[e] = kmax(fmn, kmin(fmx, div_rcp(q, HN[e], RH[e])));
+      const long long kc = dkey(c), kw = dkey(FLD[nbr & 1 ? e - 1 : e]), ke = dkey(FLD[nbr & 2 ? e + 1 : e]),
+                      ks = dkey(FLD[nbr & 4 ? e - RX : e]), kn = dkey(FLD[nbr & 8 ? e + RX : e]);
+      const long long fmx = max(max(max(max(kc, kw), ke), ks), kn);
+      const long long fmn = min(min(min(min(kc, kw), ke), ks), kn);
+      const double fdv = mul_rn(mul_rn((FX[e + 1] - FX[e]) + (FY[e + RX] - FY[e]), dt2), SCI[e]);
+      const double q = mul_rn(c, HO[e]) - fdv;
+      FLO[e] = from_dkey(max(fmn, min(fmx, dkey(div_by(q, HN[e], RC[e])))));
     });
     __syncthreads();
 
@@ -249,7 +265,9 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
       } else {
         fhx = uu * 0.5 * (FLDC[e] + FLDC[e - 1]);
       }
-      FX[e] = fhx - FX[e];
+      const double fa = fhx - FX[e];
+      FX[e] = fa;
+      FXF[e] = f32_away(fa);
     });
     rect<RX, 2, RW - 2, 2, RY - 1>([&](int a, int b, int e, int) {
       if (!(MSK[e] & kIV)) return;
@@ -261,54 +279,56 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
       } else {
         fhy = vv * 0.5 * (FLDC[e] + FLDC[e - RX]);
       }
-      FY[e] = fhy - FY[e];
+      const double fa = fhy - FY[e];
+      FY[e] = fa;
+      FYF[e] = f32_away(fa);
     });
     __syncthreads();
 
     // fmxlo/fmnlo (:792-793) in place over fld/fldc, now dead
     rect<RX, 1, RW - 1, 1, RY - 1>([&](int a, int b, int e, int) {
       if (!(MSK[e] & kIP)) return;
-      const double c = FLD[e], cc = FLDC[e], lo = FLO[e];
-      FLD[e] = kmax(kmax(c, cc), lo);
-      FLDC[e] = kmin(kmin(c, cc), lo);
+      const long long c = dkey(FLD[e]), cc = dkey(FLDC[e]), lo = dkey(FLO[e]);
+      FLD[e] = __longlong_as_double(max(max(c, cc), lo));
+      FLDC[e] = __longlong_as_double(min(min(c, cc), lo));
     });
     __syncthreads();
 
     // S4: Zalesak bounds and ratios, :863-909.  Output cells keep
-    // fqmax/fqmin in registers for S6 (same thread-to-cell map).
-    double qx[NOUT_IT], qn[NOUT_IT];
-    auto zalesak = [&](int e, double &fqmax, double &fqmin) {
-      const bool mw = MSK[e - 1] & kIP, me = MSK[e + 1] & kIP, ms = MSK[e - RX] & kIP, mn = MSK[e + RX] & kIP;
-      fqmax = FLD[e];
-      fqmin = FLDC[e];
-      fqmax = kmax(fqmax, mw ? FLD[e - 1] : FLD[e]);
-      fqmax = kmax(fqmax, me ? FLD[e + 1] : FLD[e]);
-      fqmax = kmax(fqmax, ms ? FLD[e - RX] : FLD[e]);
-      fqmax = kmax(fqmax, mn ? FLD[e + RX] : FLD[e]);
-      fqmin = kmin(fqmin, mw ? FLDC[e - 1] : FLDC[e]);
-      fqmin = kmin(fqmin, me ? FLDC[e + 1] : FLDC[e]);
-      fqmin = kmin(fqmin, ms ? FLDC[e - RX] : FLDC[e]);
-      fqmin = kmin(fqmin, mn ? FLDC[e + RX] : FLDC[e]);
-      // ib=ipip1, jb=ipjp1 (:873-875): land to the E/N -> own face twice
-      const double fxa = FX[e], fxb = me ? FX[e + 1] : FX[e];
-      const double fya = FY[e], fyb = mn ? FY[e + RX] : FY[e];
-      const double famax = pos0(fxa) - neg0(fxb) + pos0(fya) - neg0(fyb);
-      const double famin = pos0(fxb) - neg0(fxa) + pos0(fyb) - neg0(fya);
+    // fqmax/fqmin (as keys) in registers for S6 (same thread-to-cell map).
+    // A ratio is 1 unless qp < famax, which holds at a few cells only, those
+    // near an extremum of the field: FP32 bounds of the two sides (below qp,
+    // above famax, 2^-18 apart where the roundings of either are below
+    // 2^-20) settle the others without the eight FP64 operations of each
+    // side.  famax = 0: every flux the ratio multiplies is 0.
+    long long qx[NOUT_IT], qn[NOUT_IT];
+    auto zalesak = [&](int a, int b, int e, long long &kqx, long long &kqn) {
+      const int nbr = NBR[e];
+      const int ew = nbr & 1 ? e - 1 : e, ee = nbr & 2 ? e + 1 : e, es = nbr & 4 ? e - RX : e, en = nbr & 8 ? e + RX : e;
+      kqx = max(max(max(max(kmx_at(e), kmx_at(ew)), kmx_at(ee)), kmx_at(es)), kmx_at(en));
+      kqn = min(min(min(min(kmn_at(e), kmn_at(ew)), kmn_at(ee)), kmn_at(es)), kmn_at(en));
       const double lo = FLO[e];
-      double rp = 0.0, rm = 0.0;
-      if (gt0(famax)) {
-        const double qp = (fqmax - lo) * FCN[e] * SCL[e] * qdt2;
-        rp = klt(qp, famax) ? div_rn(qp, famax) : 1.0;
+      const double dmx = from_dkey(kqx) - lo, dmn = lo - from_dkey(kqn);
+      // ib=ipip1, jb=ipjp1 (:873-875): land to the E/N -> own face twice
+      const float xa = FXF[e], xb = FXF[ee], ya = FYF[e], yb = FYF[en], qf = QF[e];
+      const float amax = (fmaxf(xa, 0.0f) - fminf(xb, 0.0f)) + (fmaxf(ya, 0.0f) - fminf(yb, 0.0f));
+      const float amin = (fmaxf(xb, 0.0f) - fminf(xa, 0.0f)) + (fmaxf(yb, 0.0f) - fminf(ya, 0.0f));
+      double rp = 1.0, rm = 1.0;
+      if (!(f32_below(dmx) * qf > amax * 1.000004f || amax == 0.0f)) {
+        const double famax = pos0(FX[e]) - neg0(FX[ee]) + pos0(FY[e]) - neg0(FY[en]);
+        const double qp = dmx * fcn_of(a, b) * scl_of(a, b) * qdt2;
+        rp = !gt0(famax) ? 0.0 : klt(qp, famax) ? div_rn(qp, famax) : 1.0;
       }
-      if (gt0(famin)) {
-        const double qm = (lo - fqmin) * FCN[e] * SCL[e] * qdt2;
-        rm = klt(qm, famin) ? div_rn(qm, famin) : 1.0;
+      if (!(f32_below(dmn) * qf > amin * 1.000004f || amin == 0.0f)) {
+        const double famin = pos0(FX[ee]) - neg0(FX[e]) + pos0(FY[en]) - neg0(FY[e]);
+        const double qm = dmn * fcn_of(a, b) * scl_of(a, b) * qdt2;
+        rm = !gt0(famin) ? 0.0 : klt(qm, famin) ? div_rn(qm, famin) : 1.0;
       }
       RP[e] = rp;
       RM[e] = rm;
     };
     rect<RX, 3, RW - 3, 3, RY - 3>([&](int a, int b, int e, int it) {
-      if (MSK[e] & kIP) zalesak(e, qx[it], qn[it]);
+      if (MSK[e] & kIP) zalesak(a, b, e, qx[it], qn[it]);
     });
     {  // the ring [2,RW-2) x [2,RY-2) minus the output cells: ratios only
       constexpr int NRING = 2 * (RW - 4) + 2 * (RY - 6);
@@ -321,8 +341,8 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
         else if (t < 2 * (RW - 4) + (RY - 6)) { a = 2; b = 3 + t - 2 * (RW - 4); }
         else { a = RW - 3; b = 3 + t - 2 * (RW - 4) - (RY - 6); }
         const int e = b * RX + a;
-        double dx, dn;
-        if (MSK[e] & kIP) zalesak(e, dx, dn);
+        long long dx, dn;
+        if (MSK[e] & kIP) zalesak(a, b, e, dx, dn);
       }
     }
     __syncthreads();
@@ -331,14 +351,16 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
     rect<RX, 3, RW - 2, 3, RY - 3>([&](int a, int b, int e, int) {
       if (!(MSK[e] & kIU)) return;
       const double f = FX[e];
-      const double fact = lt0(f) ? kmin(RP[e - 1], RM[e]) : kmin(RP[e], RM[e - 1]);
-      FX[e] = fact * f;
+      const int ep = lt0(f) ? e - 1 : e, em = e + e - 1 - ep;
+      const double fact = kmin(RP[ep], RM[em]);
+      if (__double_as_longlong(fact) != kOneBits) FX[e] = fact * f;
     });
     rect<RX, 3, RW - 3, 3, RY - 2>([&](int a, int b, int e, int) {
       if (!(MSK[e] & kIV)) return;
       const double f = FY[e];
-      const double fact = lt0(f) ? kmin(RP[e - RX], RM[e]) : kmin(RP[e], RM[e - RX]);
-      FY[e] = fact * f;
+      const int ep = lt0(f) ? e - RX : e, em = e + e - RX - ep;
+      const double fact = kmin(RP[ep], RM[em]);
+      if (__double_as_longlong(fact) != kOneBits) FY[e] = fact * f;
     });
     __syncthreads();
 
@@ -346,8 +368,8 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
     rect<RX, 3, RW - 3, 3, RY - 3>([&](int a, int b, int e, int it) {
       const int i = ib0 + a, j = jb0 + b;
       if (i > ii || j > jj || !(MSK[e] & kIP)) return;
-      const double fdv = ((FX[e + 1] - FX[e]) + (FY[e + RX] - FY[e])) * dt2 * SCI[e];
-      const double res = kmax(qn[it], kmin(qx[it], FLO[e] - div_rcp(fdv, HN[e], RH[e])));
+      const double fdv = mul_rn(mul_rn((FX[e + 1] - FX[e]) + (FY[e + RX] - FY[e]), dt2), SCI[e]);
+      const double res = from_dkey(max(qn[it], min(qx[it], dkey(FLO[e] - div_by(fdv, HN[e], RC[e])))));
       const long long o = (long long)(i + nb - 1) + (long long)(j + nb - 1) * ld1;
       out[o] = res;
       if (A.images) {  // periodic in x: the xctilr copy (mod_xc_sm.h:1415-1421) written here
