@@ -8,6 +8,7 @@
 #include "hyc_ens.h"
 #include "hyc_internal.h"
 #include "hyc_fct.cuh"
+#include "hyc_march.cuh"
 #include "hyc_tile.cuh"
 
 namespace hyc {
@@ -56,6 +57,47 @@ static cudaError_t launch_shape(int scheme, const TileArgs &a, int nlayers, cuda
   return cudaErrorInvalidValue;
 }
 
+// FCT2/FCT4 strip kernel.  Rows a CTA: the fewest row steps over the waves of
+// CTAs that the chip holds (each CTA takes nrow + 7 steps)
+template <int S, int NT, int NG>
+static cudaError_t launch_march_one(const TileArgs &a, int nlayers, cudaStream_t s) {
+  using G = MarchGeom<NT, NG>;
+  static unsigned long long attr_done = 0;
+  auto kern = march_kernel<S, NT, NG>;
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !(attr_done >> dev & 1ULL)) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::smem_bytes);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    if (dev < 64) attr_done |= 1ULL << dev;
+  }
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const long long strips = (a.ii + G::OUT - 1) / G::OUT, per = strips * nlayers * ((a.nfld + NG - 1) / NG);
+  const int resident = nsm * (int)(227 * 1024 / (G::smem_bytes + 1024) < 512 / (NT * NG) ? 227 * 1024 / (G::smem_bytes + 1024)
+                                                                                         : 512 / (NT * NG));
+  int nrow = 0;
+  long long best = LLONG_MAX;
+  for (int r = 4; r <= 256; r += r < 32 ? 1 : 4) {
+    const long long cost = ((per * ((a.jj + r - 1) / r) + resident - 1) / resident) * (r + 7);
+    if (cost < best) best = cost, nrow = r;
+  }
+  dim3 grid((unsigned)strips, (unsigned)((a.jj + nrow - 1) / nrow), (unsigned)(nlayers * ((a.nfld + NG - 1) / NG)));
+  kern<<<grid, NT * NG, G::smem_bytes, s>>>(a, nrow);
+  return cudaGetLastError();
+}
+
+bool march_takes(int scheme, const TileArgs &a, int nlayers) {
+  return (scheme == kFCT2 || scheme == kFCT4) && !a.ufco && nlayers * ((a.nfld + 1) / 2) <= 65535;
+}
+
+cudaError_t launch_march(int scheme, const TileArgs &a, int nlayers, cudaStream_t s) {
+  if (a.nfld == 1)
+    return scheme == kFCT2 ? launch_march_one<kFCT2, 128, 1>(a, nlayers, s) : launch_march_one<kFCT4, 128, 1>(a, nlayers, s);
+  return scheme == kFCT2 ? launch_march_one<kFCT2, 128, 2>(a, nlayers, s) : launch_march_one<kFCT4, 128, 2>(a, nlayers, s);
+}
+
 bool advect_tile_shape_ok(TileShape t) {
   return (t.tx == 32 && t.ty == 16) || (t.tx == 32 && t.ty == 32) ||
          (t.tx == 16 && t.ty == 16);
@@ -77,6 +119,7 @@ size_t advect_tiles_smem(TileShape t) {
 }
 
 cudaError_t launch_advect_tiles(int scheme, const TileArgs &a, int nlayers, TileShape t, cudaStream_t s) {
+  if (march_takes(scheme, a, nlayers)) return launch_march(scheme, a, nlayers, s);
   if (t.tx == 32 && t.ty == 16) return launch_shape<32, 16>(scheme, a, nlayers, s);
   if (t.tx == 32 && t.ty == 32) return launch_shape<32, 32>(scheme, a, nlayers, s);
   if (t.tx == 16 && t.ty == 16) return launch_shape<16, 16>(scheme, a, nlayers, s);

@@ -728,7 +728,7 @@ int hyc_advem(hyc_ctx *c, int32_t advtyp, double *fld, const double *fldc, const
   a.out = c->d_scratch;
   a.kdm = 1;
   a.err = c->d_err;
-  if (hyc::advect_tiles_tma(advtyp, c->shape)) {  // the tile kernel stages by TMA
+  if (hyc::advect_tiles_tma(advtyp, c->shape) && !hyc::march_takes(advtyp, a, 1)) {  // the tile kernel stages by TMA
     TileMaps tmv;
     const long m0 = tile_maps_add(c, a, 1, true, tmv);
     if (m0 >= 0) {
@@ -951,7 +951,7 @@ int hyc_tsadvc(hyc_ctx *c, int32_t m, int32_t n, const hyc_tsadvc_params *p, dou
       Launch L{a, nlay, -1};
       L.a.nfld = (int)(grp.size() - f0) < chunk ? (int)(grp.size() - f0) : chunk;
       for (int q = 0; q < L.a.nfld; q++) L.a.f[q] = grp[f0 + q];
-      if (fct) L.map0 = tile_maps_add(c, L.a, kk, flux1, tmv);
+      if (fct && !hyc::march_takes(at, L.a, nlay)) L.map0 = tile_maps_add(c, L.a, kk, flux1, tmv);
       launches.push_back(L);
     }
   };

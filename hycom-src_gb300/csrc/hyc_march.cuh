@@ -1,0 +1,343 @@
+// hyc_march.cuh -- FP64 FCT2/FCT4 strip kernel: a CTA marches up the rows of
+// a strip of columns, one barrier per row.
+//
+// Thread t owns column i0 - 3 + t of the strip (NT columns, the middle NT - 6
+// are updated) for one field; the NG groups of NT threads of a CTA carry NG
+// fields of the layer and share its thickness factors, which they form in
+// turn, one group a row.  At row J a thread runs every stage of the scheme,
+// each on an earlier row (map to mod_tsadvc.F90:645-997 for FCT2 and
+// :1370-1706 for FCT4):
+//   P  row J    fco+onemu, fcn+onemu, its reciprocal, fcn*scal/dt2  :1905-1942
+//   A  row J    upwind and antidiffusive fluxes                :686-720, :817-855
+//   B  row J-1  extrema, low-order fldlo, fmxlo/fmnlo               :778-797
+//   D  row J-2  Zalesak bounds and ratios                           :863-909
+//   E  row J-3  limited x-flux (y: row J-2)                         :922-946
+//   F  row J-4  corrected update, clip                              :962-982
+// North and south neighbours are the thread's own earlier rows, in registers;
+// a west or east neighbour's value was written to a ring of rows in shared
+// memory at an earlier row step, so one barrier a row orders everything.
+//
+// What bounds it: the FP64 pipe (a warp instruction per 16 clocks and SM) and
+// the integer pipes that stand in for it (hyc_div.cuh).  The stages of one
+// row step do not depend on one another but for B -> D -> E, so both pipes
+// have work at any time, where a tile kernel's stages between barriers use
+// one or the other (59 % / 36 % busy); and a strip recomputes 6 of NT columns
+// and 7 rows of a segment, where a 32x16 tile recomputes 20-60 % of a stage.
+#pragma once
+#include "hyc_args.h"
+#include "hyc_device.cuh"
+
+namespace hyc {
+
+template <int NT, int NG>
+struct MarchGeom {
+  static constexpr int OUT = NT - 6;   // columns a strip updates
+  static constexpr int P = NT + 4;     // a row: two columns of padding at each end
+  static constexpr int ROW = P * 8;    // bytes of a row of doubles
+  // rows shared by the fields, then rows of each field (ring length in [])
+  enum { U = 0, V = U + 4, DP = V + 4, SCL = DP + 4, X3 = SCL + 4, SCI = X3 + 4, HN = SCI + 8, RQ = HN + 8, HO = RQ + 8,
+         SHARED = HO + 2 };
+  enum { F = 0, C = F + 4, FX = C + 4, FA = FX + 2, KX = FA + 4, KN = KX + 2, RP = KN + 2, RM = RP + 2, FXL = RM + 2,
+         FAF = FXL + 2, FIELD = FAF + 2 };  // FAF: four rows of floats
+  static constexpr int MSK = (SHARED + NG * FIELD) * ROW;  // four rows of bytes
+  static constexpr size_t smem_bytes = MSK + 4 * P;
+};
+
+// x/2, exact (the FP64 pipe is left to operands near the ends of the range)
+__device__ __forceinline__ double half_of(double x) {
+  const int h = __double2hiint(x);
+  return idiv::mid_range((uint32_t)h) ? __hiloint2double(h - 0x100000, __double2loint(x)) : x * 0.5;
+}
+
+// 8 bytes from global to shared memory, or zeros
+__device__ __forceinline__ void copy8(void *dst, const double *src, bool in) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = in ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+// Rows [j0, j0 + nrow) of one strip of layer k (0-based), fields f0 .. f0+NG-1
+// of the launch (those past nfld or outside their layers idle).
+template <int SCHEME, int NT, int NG>
+__device__ __forceinline__ void march_body(const TileArgs &A, const int strip, const int j0, const int nrow, const int k,
+                                           const int f0, char *sm) {
+  using G = MarchGeom<NT, NG>;
+  constexpr int ROW = G::ROW;
+  constexpr uint8_t kW = 8, kE = 16, kS = 32, kN = 64;  // sea to the west, east, south, north
+  const int t = NG == 1 ? threadIdx.x : threadIdx.x % NT, g = NG == 1 ? 0 : threadIdx.x / NT;
+  const int i = 1 + strip * G::OUT - 3 + t;
+  const int nb = A.nbdy, ld1 = A.ld1, ii = A.ii, jj = A.jj;
+  const long long sl = A.slice;
+  const double dt2 = A.dt2;
+  char *sh = sm + (t + 2) * 8, *sf = sh + (G::SHARED + g * G::FIELD) * ROW;
+  uint8_t *sk = reinterpret_cast<uint8_t *>(sm) + G::MSK + t + 2;
+  auto S = [&](int arr, int slot, int dx = 0) -> double & {  // own column + dx of a shared row
+    return *reinterpret_cast<double *>(sh + arr * ROW + slot * ROW + dx * 8);
+  };
+  auto Q = [&](int arr, int slot, int dx = 0) -> double & {  // of a row of this group's field
+    return *reinterpret_cast<double *>(sf + arr * ROW + slot * ROW + dx * 8);
+  };
+  auto FAF = [&](int slot, int dx = 0) -> float & {
+    return *reinterpret_cast<float *>(sf - (t + 2) * 4 + G::FAF * ROW + slot * (ROW / 2) + dx * 4);
+  };
+  const int fi = f0 + g;
+  const bool on = fi < A.nfld && k + 1 <= A.f[fi < A.nfld ? fi : 0].kmax && k + 1 >= A.f[fi < A.nfld ? fi : 0].kmin;
+  const FieldDesc &fd = A.f[on ? fi : 0];
+  const bool incol = i >= 1 - nb && i <= ii + nb;
+  const int xc = incol ? i + nb - 1 : 0;
+  const double *fn = fd.nbase + (long long)(k + fd.k_off) * sl + xc;
+  const double *fm = fd.mbase + (long long)(k + fd.k_off) * sl + xc;
+  double *out = A.out + ((long long)fi * A.kdm + k) * sl + xc;
+  const long long lk = A.mode == 0 ? k * sl : 0;
+  const double *x3 = A.mode == 0 ? A.oneta_n : A.fco;  // onetamas(:,:,m) (null: 1) or fco
+  const double *dpk = (A.mode == 0 ? A.dpn : A.fcn) + lk;
+  const uint8_t *msk = A.msk;
+
+  // row r of every array into its ring slots (zeros outside the arrays)
+  auto fetch = [&](int r) -> uint8_t {
+    const bool in = incol && r >= 1 - nb && r <= jj + nb;
+    const long long o = in ? (long long)(r + nb - 1) * ld1 : 0;
+    const int s4 = r & 3;
+    if (on) {
+      copy8(&Q(G::F, s4), fn + o, in);
+      copy8(&Q(G::C, s4), fm + o, in);
+    }
+    if (g == 0) {
+      copy8(&S(G::U, s4), A.uflx + lk + xc + o, in);
+      copy8(&S(G::V, s4), A.vflx + lk + xc + o, in);
+      copy8(&S(G::DP, s4), dpk + xc + o, in);
+    }
+    uint8_t m = 0;
+    if (g == NG - 1) {
+      copy8(&S(G::SCI, r & 7), A.scali + xc + o, in);
+      copy8(&S(G::SCL, s4), A.scal + xc + o, in);
+      if (x3) copy8(&S(G::X3, s4), x3 + xc + o, in);
+      if (in) m = msk[xc + o];
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    return m;
+  };
+  auto arrive = [&](int r, uint8_t m) {  // the row fetched last is there for every thread
+    if (g == NG - 1) sk[(r & 3) * G::P] = m;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+  };
+
+  __syncthreads();  // the previous item's readers are done
+  if (t < 2) {      // the padding columns
+    for (int r = g; r < G::SHARED + NG * G::FIELD; r += NG) {
+      *reinterpret_cast<double *>(sm + r * ROW + t * 8) = 0.0;
+      *reinterpret_cast<double *>(sm + r * ROW + (NT + 2 + t) * 8) = 0.0;
+    }
+    for (int r = 0; r < 4; r++) sk[r * G::P - 2] = sk[r * G::P + NT] = 0;
+  }
+  const int jfirst = j0 - 3, jlast = j0 + nrow + 3;
+  {
+    const uint8_t m = fetch(jfirst);
+    arrive(jfirst, m);
+    const uint8_t m2 = fetch(jfirst + 1);
+    arrive(jfirst + 1, m2);
+  }
+  const float qdt2f = f32_below(A.qdt2);
+  // earlier rows of this column
+  uint32_t fl = 0;                      // flags of rows J-1 (lowest byte) .. J-4
+  uint8_t m1 = 0, m2 = 0;               // masks of rows J-1, J-2
+  double f1 = 0, f2 = 0, c1 = 0, c2 = 0;  // old and centre level of rows J-1, J-2
+  double fy1 = 0;                       // upwind y-flux of face J-1
+  double ay1 = 0, ay2 = 0;              // antidiffusive y-fluxes of faces J-1, J-2
+  float af1 = 0, af2 = 0;               // their FP32 bounds
+  long long kx3 = 0, kn3 = 0;           // fmxlo/fmnlo of row J-3
+  double lo2 = 0, lo3 = 0, lo4 = 0;     // fldlo of rows J-2 .. J-4
+  long long qx3 = 0, qn3 = 0, qx4 = 0, qn4 = 0;  // fqmax/fqmin of rows J-3, J-4
+  double yl3 = 0, yl4 = 0;              // limited y-fluxes of faces J-3, J-4
+
+#pragma unroll 1
+  for (int J = jfirst; J <= jlast; J++) {
+    const uint8_t mnext = fetch(J + 2);
+    const int s0 = J & 3, s1 = (J - 1) & 3, p0 = J & 1, p1 = p0 ^ 1;
+    const uint8_t m0 = sk[s0 * G::P];
+
+    // P: thickness factors of row J
+    if (NG == 1 || (J & (NG - 1)) == g) {
+      const double d = S(G::DP, s0);
+      double fco, fcn;
+      if (A.mode == 0) {  // :1931-1938
+        const double o = x3 ? S(G::X3, s0) * d : d;
+        const double fdv =
+            mul_rn(mul_rn((S(G::U, s0, 1) - S(G::U, s0)) + (S(G::V, (J + 1) & 3) - S(G::V, s0)), dt2), S(G::SCI, J & 7));
+        fco = kmax(o + fdv, 0.0);
+        fcn = kmax(o, 0.0);
+      } else {
+        fco = S(G::X3, s0);
+        fcn = d;
+      }
+      const double hn = fcn + kOnemu;
+      S(G::HO, p0) = fco + kOnemu;
+      S(G::HN, J & 7) = hn;
+      // fcn*scal/dt2 from below, 0 where FP32 could lose it
+      const float fs = f32_below(fcn) * f32_below(S(G::SCL, s0)), qf = fs * qdt2f;
+      *reinterpret_cast<uint2 *>(&S(G::RQ, J & 7)) =
+          make_uint2(recip_of(hn), __float_as_uint(fs > 1e-30f && fs < 1e30f && qf > 1e-30f && qf < 1e30f ? qf : 0.0f));
+    }
+
+    if (on) {
+      // A: fluxes through the west and south faces of row J (0 on faces that
+      // are not between two sea cells)
+      const double fc = Q(G::F, s0), cc = Q(G::C, s0);
+      double fx = 0.0, ax = 0.0, fy = 0.0, ay = 0.0;
+      if (m0 & kIU) {
+        const double u = S(G::U, s0), fw = Q(G::F, s0, -1), cw = Q(G::C, s0, -1);
+        fx = u * (ge0(u) ? fw : fc);
+        double fh;
+        if (SCHEME == kFCT4 && (sk[s0 * G::P - 1] & sk[s0 * G::P + 1] & kIU)) {
+          const double ft14 = 7.0 / 12.0, ft24 = -1.0 / 12.0;
+          fh = u * (ft14 * (cc + cw) + ft24 * (Q(G::C, s0, 1) + Q(G::C, s0, -2)));
+        } else {
+          fh = half_of(u) * (cc + cw);
+        }
+        ax = fh - fx;
+      }
+      Q(G::FX, p0) = fx;
+      Q(G::FA, s0) = ax;
+      FAF(s0) = f32_away(ax);
+      if (m0 & kIV) {
+        const double v = S(G::V, s0);
+        fy = v * (ge0(v) ? f1 : fc);
+        double fh;
+        if (SCHEME == kFCT4 && (m1 & sk[((J + 1) & 3) * G::P] & kIV)) {
+          const double ft14 = 7.0 / 12.0, ft24 = -1.0 / 12.0;
+          fh = v * (ft14 * (cc + c1) + ft24 * (Q(G::C, (J + 1) & 3) + c2));
+        } else {
+          fh = half_of(v) * (cc + c1);
+        }
+        ay = fh - fy;
+      }
+      const float af = f32_away(ay);
+
+      // B: low-order solution of row J-1
+      fl = fl << 8 | m1 | (sk[s1 * G::P - 1] & kIP ? kW : 0) | (sk[s1 * G::P + 1] & kIP ? kE : 0) |
+           (m2 & kIP ? kS : 0) | (m0 & kIP ? kN : 0);
+      long long kx1 = 0, kn1 = 0;
+      double lo1 = 0.0;
+      if (m1 & kIP) {
+        const long long kc = dkey(f1), kw = dkey(Q(G::F, s1, fl & kW ? -1 : 0)), ke = dkey(Q(G::F, s1, fl & kE ? 1 : 0)),
+                        ks = fl & kS ? dkey(f2) : kc, kn = fl & kN ? dkey(fc) : kc;
+        const long long fmx = max(max(max(max(kc, kw), ke), ks), kn);
+        const long long fmn = min(min(min(min(kc, kw), ke), ks), kn);
+        const double fdv =
+            mul_rn(mul_rn((Q(G::FX, p1, 1) - Q(G::FX, p1)) + (fy - fy1), dt2), S(G::SCI, (J - 1) & 7));
+        const double q = mul_rn(f1, S(G::HO, p1)) - fdv;
+        const uint32_t R = reinterpret_cast<const uint2 *>(&S(G::RQ, (J - 1) & 7))->x;
+        const long long klo = max(fmn, min(fmx, dkey(div_by(q, S(G::HN, (J - 1) & 7), R))));
+        lo1 = from_dkey(klo);
+        const long long kcc = dkey(c1);
+        kx1 = max(max(kc, kcc), klo);  // :792-793
+        kn1 = min(min(kc, kcc), klo);
+      }
+      Q(G::KX, p1) = __longlong_as_double(kx1);
+      Q(G::KN, p1) = __longlong_as_double(kn1);
+
+      // D: Zalesak bounds (keys) and ratios of row J-2.  A ratio is 1 unless
+      // qp < famax, which holds at a few cells only, those near an extremum of
+      // the field: FP32 bounds of the two sides (below qp, above famax, 2^-18
+      // apart where the roundings of either are below 2^-20) settle the others
+      // without the eight FP64 operations of each side.  famax = 0: every flux
+      // the ratio multiplies is 0.
+      const uint32_t w2 = fl >> 8;
+      const long long kx2 = __double_as_longlong(Q(G::KX, p0)), kn2 = __double_as_longlong(Q(G::KN, p0));
+      long long qx = 0, qn = 0;
+      double rp = 1.0, rm = 1.0;
+      if (w2 & kIP) {
+        const int dw = w2 & kW ? -1 : 0, de = w2 & kE ? 1 : 0;
+        qx = max(max(kx2, __double_as_longlong(Q(G::KX, p0, dw))), __double_as_longlong(Q(G::KX, p0, de)));
+        qn = min(min(kn2, __double_as_longlong(Q(G::KN, p0, dw))), __double_as_longlong(Q(G::KN, p0, de)));
+        if (w2 & kS) qx = max(qx, kx3), qn = min(qn, kn3);
+        if (w2 & kN) qx = max(qx, kx1), qn = min(qn, kn1);
+        const double dmx = from_dkey(qx) - lo2, dmn = lo2 - from_dkey(qn);
+        // ib=ipip1, jb=ipjp1 (:873-875): land to the E/N -> own face twice
+        const int s2 = (J - 2) & 3;
+        const float xa = FAF(s2), xb = FAF(s2, de), ya = af2, yb = w2 & kN ? af1 : af2;
+        const float qf = __uint_as_float(reinterpret_cast<const uint2 *>(&S(G::RQ, (J - 2) & 7))->y);
+        const float amax = (fmaxf(xa, 0.0f) - fminf(xb, 0.0f)) + (fmaxf(ya, 0.0f) - fminf(yb, 0.0f));
+        const float amin = (fmaxf(xb, 0.0f) - fminf(xa, 0.0f)) + (fmaxf(yb, 0.0f) - fminf(ya, 0.0f));
+        const bool ex = !(f32_below(dmx) * qf > amax * 1.000004f || amax == 0.0f);
+        const bool en = !(f32_below(dmn) * qf > amin * 1.000004f || amin == 0.0f);
+        if (ex || en) {
+          const long long o = xc + (long long)(J - 2 + nb - 1) * ld1;
+          const double d = dpk[o], scl = A.scal[o];
+          const double fcn = A.mode == 0 ? kmax(x3 ? x3[o] * d : d, 0.0) : d;
+          const double fxa = Q(G::FA, s2), fxb = Q(G::FA, s2, de), fya = ay2, fyb = w2 & kN ? ay1 : ay2;
+          if (ex) {
+            const double famax = pos0(fxa) - neg0(fxb) + pos0(fya) - neg0(fyb);
+            const double qp = dmx * fcn * scl * A.qdt2;
+            rp = !gt0(famax) ? 0.0 : klt(qp, famax) ? div_rn(qp, famax) : 1.0;
+          }
+          if (en) {
+            const double famin = pos0(fxb) - neg0(fxa) + pos0(fyb) - neg0(fya);
+            const double qm = dmn * fcn * scl * A.qdt2;
+            rm = !gt0(famin) ? 0.0 : klt(qm, famin) ? div_rn(qm, famin) : 1.0;
+          }
+        }
+      }
+      Q(G::RP, p0) = rp;
+      Q(G::RM, p0) = rm;
+
+      // E: limited fluxes, x of row J-3 and y of face J-2
+      const double rp3 = Q(G::RP, p1), rm3 = Q(G::RM, p1);
+      double xl = 0.0, yl = 0.0;
+      if (fl >> 16 & kIU) {
+        const double f = Q(G::FA, (J - 3) & 3);
+        const bool neg = lt0(f);
+        const double fact = kmin(neg ? Q(G::RP, p1, -1) : rp3, neg ? rm3 : Q(G::RM, p1, -1));
+        xl = __double_as_longlong(fact) == kOneBits ? f : fact * f;
+      }
+      Q(G::FXL, p1) = xl;
+      if (w2 & kIV) {
+        const double f = ay2;
+        const bool neg = lt0(f);
+        const double fact = kmin(neg ? rp3 : rp, neg ? rm : rm3);
+        yl = __double_as_longlong(fact) == kOneBits ? f : fact * f;
+      }
+
+      // F: corrected update of row J-4
+      const int j = J - 4;
+      if ((fl >> 24 & kIP) && j >= j0 && j <= jj && t >= 3 && t < NT - 3 && i <= ii) {
+        const double fdv =
+            mul_rn(mul_rn((Q(G::FXL, p0, 1) - Q(G::FXL, p0)) + (yl3 - yl4), dt2), S(G::SCI, j & 7));
+        const uint32_t R = reinterpret_cast<const uint2 *>(&S(G::RQ, j & 7))->x;
+        const double res = from_dkey(max(qn4, min(qx4, dkey(lo4 - div_by(fdv, S(G::HN, j & 7), R)))));
+        const long long o = (long long)(j + nb - 1) * ld1;
+        out[o] = res;
+        if (A.images) {  // periodic in x: the xctilr copy (mod_xc_sm.h:1415-1421) written here
+          if (i <= A.images) out[o + ii] = res;
+          if (i > ii - A.images) out[o - ii] = res;
+        }
+      }
+
+      f2 = f1, f1 = fc;
+      if (SCHEME == kFCT4) c2 = c1;
+      c1 = cc;
+      fy1 = fy;
+      ay2 = ay1, ay1 = ay, af2 = af1, af1 = af;
+      kx3 = kx2, kn3 = kn2;
+      lo4 = lo3, lo3 = lo2, lo2 = lo1;
+      qx4 = qx3, qn4 = qn3, qx3 = qx, qn3 = qn;
+      yl4 = yl3, yl3 = yl;
+    }
+    m2 = m1, m1 = m0;
+    arrive(J + 2, mnext);
+  }
+}
+
+// grid: (strips, segments, layers * field groups), the groups of a layer
+// next to each other
+template <int SCHEME, int NT, int NG>
+__global__ void __launch_bounds__(NT *NG, 512 / (NT * NG)) march_kernel(const TileArgs A, int nrow) {
+  extern __shared__ __align__(16) char smc[];
+  const int ngrp = (A.nfld + NG - 1) / NG;
+  const int k = blockIdx.z / ngrp, q = blockIdx.z - k * ngrp;
+  const int j0 = 1 + blockIdx.y * nrow;
+  march_body<SCHEME, NT, NG>(A, blockIdx.x, j0, min(nrow, A.jj + 1 - j0), k, q * NG, smc);
+}
+
+}  // namespace hyc
