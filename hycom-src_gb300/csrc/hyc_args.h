@@ -9,6 +9,9 @@ namespace hyc {
 constexpr uint8_t kIP = 1, kIU = 2, kIV = 4;  // mask bits: ip, iu, iv
 
 constexpr int kMaxFields = 16;
+// FCT strip kernel (hyc_march.cuh): columns a CTA marches over (6 fewer are
+// updated), fields it carries, and so the most groups of fields
+constexpr int kMarchCols = 64, kMarchFields = 2, kMaxMarchGroups = kMaxFields / kMarchFields;
 enum Scheme { kPCM = 0, kMPDATA = 1, kFCT2 = 2, kFCT4 = 4 };
 
 struct FieldDesc {
@@ -51,13 +54,14 @@ struct TileArgs {
   double dt2;
   double qdt2;  // 1/dt2, divided once on the host (the same IEEE quotient)
   int nfld;
-  FieldDesc f[kMaxFields];
+  int seg;  // rows per segment of the strip kernel's queue
   // output: out + (fi*kdm + k)*slice; sea cells of the interior are written
   double *out;
   int kdm;
   // >0: also write the periodic-x halo images of output cells with
   // i <= images or i > ii-images (an ensemble level is its own halo source)
   int images;
+  FieldDesc f[kMaxFields];  // last: the strip kernel's queue stages what is before it
 };
 
 // advem_fct2c (mod_tsadvc.F90:999-1368) over up to kMaxFields (field, layer)

@@ -47,9 +47,10 @@ cudaError_t launch_cell_words(const double *scp2i, const uint8_t *msk, double dt
                               cudaStream_t s);
 cudaError_t launch_wait_probe(int arrive, int *err, cudaStream_t s);
 
-// FP64 ensemble: the FCT tile body over a queue of (basin, tile, layer)
-cudaError_t launch_fct_queue(int scheme, TileShape t, const TileArgs *basins, const int4 *items, int nitems,
-                             int *head, int nsm, cudaStream_t s);
+// FP64 ensemble: the FCT strip kernel over a queue of (basin, strip and
+// field group, first row, layer)
+cudaError_t launch_march_queue(int scheme, const TileArgs *basins, const int4 *items, int nitems, int *head, int nsm,
+                               cudaStream_t s);
 
 cudaError_t launch_repitch(const void *src, int src_fp32, long long spitch, long long sslice, void *dst, int dst_fp32,
                            long long dpitch, long long dslice, int w, int h, int nslices, cudaStream_t s);

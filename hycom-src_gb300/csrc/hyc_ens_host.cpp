@@ -223,6 +223,19 @@ int col2_kchunk(const hyc_ens *e, const EBasin &) {
   return (int)std::max(1LL, std::min(8LL, kc));
 }
 
+// FP64 FCT strip kernel: strips of a basin and rows per segment.  About 12
+// work items per resident CTA over the ensemble, so that the queue's last wave
+// is short, in segments of 24 rows (7 more are recomputed) to 192.
+int march_strips(const EBasin &b) { return (b.idm + hyc::kMarchCols - 7) / (hyc::kMarchCols - 6); }
+int march_seg(const hyc_ens *e, const EBasin &b) {
+  long long rows = 0;
+  for (const auto &x : e->b)
+    rows += (long long)march_strips(x) * x.jdm * x.kdm * ((x.ntr + hyc::kMarchFields - 1) / hyc::kMarchFields);
+  const long long want = std::max(24LL, std::min(192LL, rows / (12LL * e->nsm * 4)));
+  const int nseg = (int)((b.jdm + want - 1) / want);
+  return (b.jdm + nseg - 1) / nseg;
+}
+
 // device tables for the three rotations (rebuilt when delt1 changes)
 int build_tables(hyc_ens *e, double dt2) {
   if (e->tbl_dt2 == dt2) return HYC_OK;
@@ -293,6 +306,7 @@ int build_tables(hyc_ens *e, double dt2) {
         a.dt2 = dt2;
         a.qdt2 = 1.0 / dt2;
         a.nfld = b.ntr;
+        a.seg = march_seg(e, b);
         for (int q = 0; q < b.ntr; q++) {
           a.f[q].nbase = (double *)b.lev[lo] + (long long)q * b.kdm * b.slice;
           a.f[q].mbase = (const double *)b.lev[lc] + (long long)q * b.kdm * b.slice;
@@ -366,7 +380,6 @@ int build_tables(hyc_ens *e, double dt2) {
 int strip_pass(const hyc_ens *e) { return std::min(e->strip_nq, e->maxntr); }
 
 int build_items(hyc_ens *e) {
-  const bool per_layer = e->prec != HYC_PREC_MIXED;
   const int nqm = strip_pass(e);
   if (e->d_items && e->items_tx == e->shape.tx && e->items_ty == e->shape.ty && e->items_nq == nqm) return HYC_OK;
   struct W {
@@ -376,7 +389,6 @@ int build_items(hyc_ens *e) {
   std::vector<W> w, wt;  // main launch, one-tracer launch
   for (int i = 0; i < (int)e->b.size(); i++) {
     const EBasin &b = e->b[i];
-    const int ntx = (b.idm + e->shape.tx - 1) / e->shape.tx, nty = (b.jdm + e->shape.ty - 1) / e->shape.ty;
     if (is_col2(e->shape)) {  // (basin, 56-column strip, segment, chunk of layers), all tracers
       // the layer chunks of a segment are queued together: the per-cell
       // words of the segment's rows are then read from DRAM about once
@@ -384,6 +396,7 @@ int build_items(hyc_ens *e) {
       // with pairs of tracers per pass, an odd count's last tracer goes to the
       // one-tracer launch instead of a pass that advances it twice
       const int nstrip = (b.nbdy + b.idm - 4 + hyc::kCol2Strip - 1) / hyc::kCol2Strip;
+      const int nty = (b.jdm + e->shape.ty - 1) / e->shape.ty;
       const int kc = col2_kchunk(e, b), nkc = (b.kdm + kc - 1) / kc;
       const int trm = nqm == 2 ? (b.ntr & ~1) : b.ntr;
       const bool tail = nqm == 2 && (b.ntr & 1);
@@ -396,13 +409,14 @@ int build_items(hyc_ens *e) {
           }
       continue;
     }
-    for (int t = 0; t < ntx * nty; t++) {
-      if (per_layer) {
-        for (int k = 0; k < b.kdm; k++) w.push_back({(long long)b.ntr, make_int4(i, t, k, 0)});
-      } else {
-        w.push_back({(long long)b.kdm * b.ntr, make_int4(i, t, 0, 0)});
-      }
-    }
+    // FP64 form: (basin, strip, segment, layer, group of fields)
+    constexpr int kMaxGroups = hyc::kMaxMarchGroups;
+    const int seg = march_seg(e, b), nstrip = march_strips(b), ngrp = (b.ntr + hyc::kMarchFields - 1) / hyc::kMarchFields;
+    for (int j0 = 1; j0 <= b.jdm; j0 += seg)
+      for (int k = 0; k < b.kdm; k++)
+        for (int st = 0; st < nstrip; st++)
+          for (int q = 0; q < ngrp; q++)
+            w.push_back({(long long)std::min(seg, b.jdm + 1 - j0) + 7, make_int4(i, st * kMaxGroups + q, j0, k)});
   }
   std::stable_sort(w.begin(), w.end(), [](const W &a, const W &c) { return a.work > c.work; });
   std::stable_sort(wt.begin(), wt.end(), [](const W &a, const W &c) { return a.work > c.work; });
@@ -471,8 +485,7 @@ int enqueue_step(hyc_ens *e, int advtyp, int r, int h, cudaStream_t st) {
     }
   }
   else
-    c = hyc::launch_fct_queue(advtyp, e->shape, e->d_targs[r], e->d_items, e->nitems, e->d_head + 2 * h, e->nsm,
-                              st);
+    c = hyc::launch_march_queue(advtyp, e->d_targs[r], e->d_items, e->nitems, e->d_head + 2 * h, e->nsm, st);
   if (c != cudaSuccess) return efail(e, HYC_ERR_CUDA, "step kernel: %s", cudaGetErrorString(c));
   e->stats.launches += launches;
   return HYC_OK;

@@ -4,9 +4,13 @@
 // mod_tsadvc.F90:645-997 for FCT2 and :1370-1706 for FCT4), reorganised so
 // that two CTAs fit on an SM (the FP64 pipe needs more resident warps to
 // hide its latency than one 256-thread CTA gives):
-//   * 15 shared arrays instead of 19: fmxlo/fmnlo overwrite fld/fldc in
-//     place once fld and fldc are dead, and fqmax/fqmin live in registers of
-//     the thread that later updates the same output cell;
+//   * 12 shared arrays of doubles instead of 19: fmxlo/fmnlo overwrite
+//     fld/fldc in place once fld and fldc are dead, fcn and scal are staged
+//     where the limiter ratios go later, and fqmax/fqmin live in registers of
+//     the thread that updates the same output cell;
+//   * divisions and the products of the flux divergence run on the integer
+//     pipes (hyc_div.cuh), and FP32 bounds settle most limiter ratios: FCT2,
+//     T and S, 1500x1100x10 3.80 -> 3.27 ms (FP64 pipe 72 -> 59 % busy);
 //   * fco+onemu is formed once per cell (the reference forms it per field);
 //   * the stage loops have compile-time bounds and are unrolled, so a
 //     thread's cells interleave (more independent FP64 work in flight).
@@ -14,6 +18,7 @@
 // one mbarrier, every wait bounded) when the launch carries tensor maps,
 // else by plain loads.  Only sea cells of the interior are written to the
 // output slice.
+// It serves launches too small for the strip kernel (hyc_march.cuh).
 #pragma once
 #include <cuda.h>
 
@@ -296,8 +301,8 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
 
     // S4: Zalesak bounds and ratios, :863-909.  Output cells keep
     // fqmax/fqmin (as keys) in registers for S6 (same thread-to-cell map).
-    // A ratio is 1 unless qp < famax, which holds at a few cells only, those
-    // near an extremum of the field: FP32 bounds of the two sides (below qp,
+    // A ratio is 1 unless qp < famax, mostly on one side of a cell (the side
+    // t and t-1 do not differ towards): FP32 bounds of the two sides (below qp,
     // above famax, 2^-18 apart where the roundings of either are below
     // 2^-20) settle the others without the eight FP64 operations of each
     // side.  famax = 0: every flux the ratio multiplies is 0.
@@ -393,41 +398,6 @@ __global__ void __launch_bounds__(256, 2) fct_tile_kernel(const TileArgs A) {
   __syncthreads();
   uint32_t ph = 0;
   fct_tile_body<SCHEME, TX, TY>(A, blockIdx.x, blockIdx.y, sm, &bar, ph);
-}
-
-// Persistent form for an ensemble of basins: CTAs take work items
-// (basin, tile, layer) from a queue until it is empty.
-template <int SCHEME, int TX, int TY>
-__global__ void __launch_bounds__(256, 2)
-    fct_queue_kernel(const TileArgs *__restrict__ basins, const int4 *__restrict__ items, int nitems, int *head) {
-  extern __shared__ __align__(16) double sm[];
-  __shared__ int cur;
-  __shared__ int cur_basin;
-  __shared__ __align__(16) TileArgs sa;  // the item's basin, staged once (read many times below)
-  __shared__ uint64_t bar;
-  uint32_t ph = 0;
-  if (threadIdx.x == 0) {
-    cur_basin = -1;
-    tma::bar_init(&bar, 1);
-    tma::fence_bar_init();
-  }
-  for (;;) {
-    if (threadIdx.x == 0) cur = atomicAdd(head, 1);
-    __syncthreads();
-    const int it = cur;
-    if (it >= nitems) break;
-    const int4 w = items[it];
-    if (w.x != cur_basin) {  // uniform: every thread read the same item
-      __syncthreads();
-      const int *src = reinterpret_cast<const int *>(basins + w.x);
-      int *dst = reinterpret_cast<int *>(&sa);
-      for (int q = threadIdx.x; q < (int)(sizeof(TileArgs) / 4); q += blockDim.x) dst[q] = src[q];
-      __syncthreads();
-      if (threadIdx.x == 0) cur_basin = w.x;
-    }
-    __syncthreads();
-    if (!fct_tile_body<SCHEME, TX, TY>(sa, w.y, w.z, sm, &bar, ph)) break;
-  }
 }
 
 }  // namespace hyc

@@ -1,6 +1,7 @@
 // hyc_fp64.cu -- FP64 kernels of the tracer-advection path and their launchers.
 // Compiled with -fmad=false so that every product and sum rounds separately,
 // as in the reference's REAL*8 build with no FMA contraction.
+#include <algorithm>
 #include <climits>
 #include <cstdio>
 #include <cstring>
@@ -75,11 +76,11 @@ static cudaError_t launch_march_one(const TileArgs &a, int nlayers, cudaStream_t
   }
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const long long strips = (a.ii + G::OUT - 1) / G::OUT, per = strips * nlayers * ((a.nfld + NG - 1) / NG);
-  const int resident = nsm * (int)(227 * 1024 / (G::smem_bytes + 1024) < 512 / (NT * NG) ? 227 * 1024 / (G::smem_bytes + 1024)
-                                                                                         : 512 / (NT * NG));
+  const int resident = nsm * std::min<int>(228 * 1024 / (G::smem_bytes + 1024), 512 / (NT * NG));
   int nrow = 0;
   long long best = LLONG_MAX;
   for (int r = 4; r <= 256; r += r < 32 ? 1 : 4) {
+    if ((a.jj + r - 1) / r > 65535) continue;
     const long long cost = ((per * ((a.jj + r - 1) / r) + resident - 1) / resident) * (r + 7);
     if (cost < best) best = cost, nrow = r;
   }
@@ -88,14 +89,29 @@ static cudaError_t launch_march_one(const TileArgs &a, int nlayers, cudaStream_t
   return cudaGetLastError();
 }
 
+// The strip kernel from the size on where its CTAs fill the chip: more 32x16
+// tiles than one wave of the tile kernel (two CTAs an SM), four waves where
+// the launch has one field.  A whole call (FCT2, T and S; tile / strip): 240
+// tiles 65 / 82 us, 351 tiles 88 / 83, 1170 tiles 188 / 150, the 4500x3298x41
+// basin 125 / 78 ms; one field: 551 tiles 71 / 84 us, 1276 tiles 119 / 120,
+// 3243 tiles 245 / 245.  The layer-1 fields of isopycnic mode that need a
+// second pair of fluxes (ufco) stay with the tile kernel.
 bool march_takes(int scheme, const TileArgs &a, int nlayers) {
-  return (scheme == kFCT2 || scheme == kFCT4) && !a.ufco && nlayers * ((a.nfld + 1) / 2) <= 65535;
+  if ((scheme != kFCT2 && scheme != kFCT4) || a.ufco) return false;
+  if ((long long)nlayers * ((a.nfld + kMarchFields - 1) / kMarchFields) > 65535) return false;  // grid limit
+  int dev = 0, nsm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const long long tiles = (long long)((a.ii + 31) / 32) * ((a.jj + 15) / 16) * nlayers;
+  return tiles > (a.nfld > 1 ? 1 : 4) * 2LL * nsm;
 }
 
 cudaError_t launch_march(int scheme, const TileArgs &a, int nlayers, cudaStream_t s) {
   if (a.nfld == 1)
-    return scheme == kFCT2 ? launch_march_one<kFCT2, 128, 1>(a, nlayers, s) : launch_march_one<kFCT4, 128, 1>(a, nlayers, s);
-  return scheme == kFCT2 ? launch_march_one<kFCT2, 128, 2>(a, nlayers, s) : launch_march_one<kFCT4, 128, 2>(a, nlayers, s);
+    return scheme == kFCT2 ? launch_march_one<kFCT2, kMarchCols, 1>(a, nlayers, s)
+                           : launch_march_one<kFCT4, kMarchCols, 1>(a, nlayers, s);
+  return scheme == kFCT2 ? launch_march_one<kFCT2, kMarchCols, kMarchFields>(a, nlayers, s)
+                         : launch_march_one<kFCT4, kMarchCols, kMarchFields>(a, nlayers, s);
 }
 
 bool advect_tile_shape_ok(TileShape t) {
@@ -126,34 +142,29 @@ cudaError_t launch_advect_tiles(int scheme, const TileArgs &a, int nlayers, Tile
   return cudaErrorInvalidValue;
 }
 
-// persistent FCT kernels for the FP64 ensemble
-template <int S, int TX, int TY>
-static cudaError_t launch_queue_one(const TileArgs *basins, const int4 *items, int nitems, int *head, int nsm,
-                                    cudaStream_t s) {
-  constexpr size_t smem = FctGeom<TX, TY>::smem_bytes;
-  auto kern = fct_queue_kernel<S, TX, TY>;
+// persistent FCT strip kernel for the FP64 ensemble
+template <int S>
+static cudaError_t launch_march_queue_one(const TileArgs *basins, const int4 *items, int nitems, int *head, int nsm,
+                                          cudaStream_t s) {
+  constexpr int NT = kMarchCols, NG = kMarchFields;
+  constexpr size_t smem = MarchGeom<NT, NG>::smem_bytes;
+  auto kern = march_queue_kernel<S, NT, NG>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT * NG, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
-  kern<<<nsm * per_sm, 256, smem, s>>>(basins, items, nitems, head);
+  kern<<<nsm * per_sm, NT * NG, smem, s>>>(basins, items, nitems, head);
   return cudaGetLastError();
 }
 
-cudaError_t launch_fct_queue(int scheme, TileShape t, const TileArgs *basins, const int4 *items, int nitems,
-                             int *head, int nsm, cudaStream_t s) {
-  if (t.tx == 32 && t.ty == 16) {
-    if (scheme == kFCT2) return launch_queue_one<kFCT2, 32, 16>(basins, items, nitems, head, nsm, s);
-    if (scheme == kFCT4) return launch_queue_one<kFCT4, 32, 16>(basins, items, nitems, head, nsm, s);
-  }
-  if (t.tx == 16 && t.ty == 16) {
-    if (scheme == kFCT2) return launch_queue_one<kFCT2, 16, 16>(basins, items, nitems, head, nsm, s);
-    if (scheme == kFCT4) return launch_queue_one<kFCT4, 16, 16>(basins, items, nitems, head, nsm, s);
-  }
+cudaError_t launch_march_queue(int scheme, const TileArgs *basins, const int4 *items, int nitems, int *head, int nsm,
+                               cudaStream_t s) {
+  if (scheme == kFCT2) return launch_march_queue_one<kFCT2>(basins, items, nitems, head, nsm, s);
+  if (scheme == kFCT4) return launch_march_queue_one<kFCT4>(basins, items, nitems, head, nsm, s);
   return cudaErrorInvalidValue;
 }
 

@@ -17,13 +17,21 @@
 // a west or east neighbour's value was written to a ring of rows in shared
 // memory at an earlier row step, so one barrier a row orders everything.
 //
-// What bounds it: the FP64 pipe (a warp instruction per 16 clocks and SM) and
-// the integer pipes that stand in for it (hyc_div.cuh).  The stages of one
-// row step do not depend on one another but for B -> D -> E, so both pipes
-// have work at any time, where a tile kernel's stages between barriers use
-// one or the other (59 % / 36 % busy); and a strip recomputes 6 of NT columns
-// and 7 rows of a segment, where a 32x16 tile recomputes 20-60 % of a stage.
+// What bounds it: the FP64 pipe (a warp instruction per 16 clocks and SM; 72 %
+// busy, about 85 % is reached in practice) and latency at 16 warps per SM
+// (registers and shared memory both stop there); issue slots are 43 % used.
+// FCT2, T and S, 1500x1100x10: 2.40 ms; the 32x16 tile kernel 3.80 ms with
+// every operation on the FP64 pipe, 3.27 ms with the same integer operations
+// as here.  A strip recomputes 6 of NT columns and 7 rows of a segment, where
+// a tile recomputes 20-60 % of a stage, and the stages of one row step do not
+// depend on one another but for B -> D -> E, so both pipes have work at any
+// time.  NT = 64: four CTAs of four warps wait less at their barriers than
+// two of eight (NT = 128: 2.54 ms), though 10 % of the columns are recomputed.
+// Divisions and the products of P and B run on the integer pipes: with all of
+// them on the FP64 pipe 2.53 ms, with A's too on the integer pipes 2.56 ms.
 #pragma once
+#include <cstddef>
+
 #include "hyc_args.h"
 #include "hyc_device.cuh"
 
@@ -32,10 +40,10 @@ namespace hyc {
 template <int NT, int NG>
 struct MarchGeom {
   static constexpr int OUT = NT - 6;   // columns a strip updates
-  static constexpr int P = NT + 4;     // a row: two columns of padding at each end
+  static constexpr int P = NT + 3;     // a row: two columns of padding to the west, one to the east
   static constexpr int ROW = P * 8;    // bytes of a row of doubles
   // rows shared by the fields, then rows of each field (ring length in [])
-  enum { U = 0, V = U + 4, DP = V + 4, SCL = DP + 4, X3 = SCL + 4, SCI = X3 + 4, HN = SCI + 8, RQ = HN + 8, HO = RQ + 8,
+  enum { U = 0, V = U + 4, DP = V + 4, SCL = DP + 4, SCI = SCL + 8, HN = SCI + 8, RQ = HN + 8, FCN = RQ + 8, HO = FCN + 4,
          SHARED = HO + 2 };
   enum { F = 0, C = F + 4, FX = C + 4, FA = FX + 2, KX = FA + 4, KN = KX + 2, RP = KN + 2, RM = RP + 2, FXL = RM + 2,
          FAF = FXL + 2, FIELD = FAF + 2 };  // FAF: four rows of floats
@@ -46,7 +54,7 @@ struct MarchGeom {
 // x/2, exact (the FP64 pipe is left to operands near the ends of the range)
 __device__ __forceinline__ double half_of(double x) {
   const int h = __double2hiint(x);
-  return idiv::mid_range((uint32_t)h) ? __hiloint2double(h - 0x100000, __double2loint(x)) : x * 0.5;
+  return idiv::mid_range((uint32_t)h) ? __hiloint2double(h - 0x100000, __double2loint(x)) : idiv::fp64_mul(x, 0.5);
 }
 
 // 8 bytes from global to shared memory, or zeros
@@ -57,10 +65,11 @@ __device__ __forceinline__ void copy8(void *dst, const double *src, bool in) {
 }
 
 // Rows [j0, j0 + nrow) of one strip of layer k (0-based), fields f0 .. f0+NG-1
-// of the launch (those past nfld or outside their layers idle).
+// of the launch (those past nfld or outside their layers idle), described in
+// fds (A.f is not read).
 template <int SCHEME, int NT, int NG>
-__device__ __forceinline__ void march_body(const TileArgs &A, const int strip, const int j0, const int nrow, const int k,
-                                           const int f0, char *sm) {
+__device__ __forceinline__ void march_body(const TileArgs &A, const FieldDesc *fds, const int strip, const int j0,
+                                           const int nrow, const int k, const int f0, char *sm) {
   using G = MarchGeom<NT, NG>;
   constexpr int ROW = G::ROW;
   constexpr uint8_t kW = 8, kE = 16, kS = 32, kN = 64;  // sea to the west, east, south, north
@@ -81,8 +90,8 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
     return *reinterpret_cast<float *>(sf - (t + 2) * 4 + G::FAF * ROW + slot * (ROW / 2) + dx * 4);
   };
   const int fi = f0 + g;
-  const bool on = fi < A.nfld && k + 1 <= A.f[fi < A.nfld ? fi : 0].kmax && k + 1 >= A.f[fi < A.nfld ? fi : 0].kmin;
-  const FieldDesc &fd = A.f[on ? fi : 0];
+  const FieldDesc &fd = fds[fi < A.nfld ? fi : 0];
+  const bool on = fi < A.nfld && k + 1 <= fd.kmax && k + 1 >= fd.kmin;
   const bool incol = i >= 1 - nb && i <= ii + nb;
   const int xc = incol ? i + nb - 1 : 0;
   const double *fn = fd.nbase + (long long)(k + fd.k_off) * sl + xc;
@@ -110,8 +119,7 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
     uint8_t m = 0;
     if (g == NG - 1) {
       copy8(&S(G::SCI, r & 7), A.scali + xc + o, in);
-      copy8(&S(G::SCL, s4), A.scal + xc + o, in);
-      if (x3) copy8(&S(G::X3, s4), x3 + xc + o, in);
+      copy8(&S(G::SCL, r & 7), A.scal + xc + o, in);
       if (in) m = msk[xc + o];
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -127,9 +135,12 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
   if (t < 2) {      // the padding columns
     for (int r = g; r < G::SHARED + NG * G::FIELD; r += NG) {
       *reinterpret_cast<double *>(sm + r * ROW + t * 8) = 0.0;
-      *reinterpret_cast<double *>(sm + r * ROW + (NT + 2 + t) * 8) = 0.0;
+      if (t == 0) *reinterpret_cast<double *>(sm + r * ROW + (NT + 2) * 8) = 0.0;
     }
-    for (int r = 0; r < 4; r++) sk[r * G::P - 2] = sk[r * G::P + NT] = 0;
+    for (int r = 0; r < 4; r++) {
+      sk[r * G::P - 2] = 0;
+      if (t == 0) sk[r * G::P + NT] = 0;
+    }
   }
   const int jfirst = j0 - 3, jlast = j0 + nrow + 3;
   {
@@ -158,24 +169,28 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
     const uint8_t m0 = sk[s0 * G::P];
 
     // P: thickness factors of row J
-    if (NG == 1 || (J & (NG - 1)) == g) {
+    if ((NG == 1 || (J & (NG - 1)) == g) && __any_sync(0xffffffffu, m0 & kIP)) {
       const double d = S(G::DP, s0);
+      double t3 = 0.0;  // onetamas(:,:,m) or fco
+      if (x3 && (m0 & kIP)) t3 = x3[xc + (long long)(J + nb - 1) * ld1];
       double fco, fcn;
       if (A.mode == 0) {  // :1931-1938
-        const double o = x3 ? S(G::X3, s0) * d : d;
+        double o = d;
+        if (x3) o = mul_rn(t3, d);
         const double fdv =
             mul_rn(mul_rn((S(G::U, s0, 1) - S(G::U, s0)) + (S(G::V, (J + 1) & 3) - S(G::V, s0)), dt2), S(G::SCI, J & 7));
         fco = kmax(o + fdv, 0.0);
         fcn = kmax(o, 0.0);
       } else {
-        fco = S(G::X3, s0);
+        fco = t3;
         fcn = d;
       }
       const double hn = fcn + kOnemu;
       S(G::HO, p0) = fco + kOnemu;
       S(G::HN, J & 7) = hn;
+      S(G::FCN, s0) = fcn;
       // fcn*scal/dt2 from below, 0 where FP32 could lose it
-      const float fs = f32_below(fcn) * f32_below(S(G::SCL, s0)), qf = fs * qdt2f;
+      const float fs = f32_below(fcn) * f32_below(S(G::SCL, J & 7)), qf = fs * qdt2f;
       *reinterpret_cast<uint2 *>(&S(G::RQ, J & 7)) =
           make_uint2(recip_of(hn), __float_as_uint(fs > 1e-30f && fs < 1e30f && qf > 1e-30f && qf < 1e30f ? qf : 0.0f));
     }
@@ -185,17 +200,28 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
       // are not between two sea cells)
       const double fc = Q(G::F, s0), cc = Q(G::C, s0);
       double fx = 0.0, ax = 0.0, fy = 0.0, ay = 0.0;
+      long long kx1 = 0, kn1 = 0, kx2 = 0, kn2 = 0, qx = 0, qn = 0;
+      double lo1 = 0.0, yl = 0.0;
+      float af = 0.0f;
+      const double ft14 = 7.0 / 12.0, ft24 = -1.0 / 12.0;
+      fl <<= 8;
+      // a warp whose columns are land on every row in flight only keeps its
+      // faces' zeros
+      if (!__any_sync(0xffffffffu, (fl | m0 | m1) != 0)) {
+        Q(G::FX, p0) = 0.0;
+        Q(G::FA, s0) = 0.0;
+        FAF(s0) = 0.0f;
+        Q(G::FXL, p1) = 0.0;
+      } else {
       if (m0 & kIU) {
         const double u = S(G::U, s0), fw = Q(G::F, s0, -1), cw = Q(G::C, s0, -1);
         fx = u * (ge0(u) ? fw : fc);
-        double fh;
-        if (SCHEME == kFCT4 && (sk[s0 * G::P - 1] & sk[s0 * G::P + 1] & kIU)) {
-          const double ft14 = 7.0 / 12.0, ft24 = -1.0 / 12.0;
-          fh = u * (ft14 * (cc + cw) + ft24 * (Q(G::C, s0, 1) + Q(G::C, s0, -2)));
-        } else {
-          fh = half_of(u) * (cc + cw);
-        }
-        ax = fh - fx;
+        double c = cc + cw, uh = u;
+        if (SCHEME == kFCT4 && (sk[s0 * G::P - 1] & sk[s0 * G::P + 1] & kIU))
+          c = ft14 * c + ft24 * (Q(G::C, s0, 1) + Q(G::C, s0, -2));
+        else
+          uh = half_of(u);
+        ax = uh * c - fx;
       }
       Q(G::FX, p0) = fx;
       Q(G::FA, s0) = ax;
@@ -203,22 +229,18 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
       if (m0 & kIV) {
         const double v = S(G::V, s0);
         fy = v * (ge0(v) ? f1 : fc);
-        double fh;
-        if (SCHEME == kFCT4 && (m1 & sk[((J + 1) & 3) * G::P] & kIV)) {
-          const double ft14 = 7.0 / 12.0, ft24 = -1.0 / 12.0;
-          fh = v * (ft14 * (cc + c1) + ft24 * (Q(G::C, (J + 1) & 3) + c2));
-        } else {
-          fh = half_of(v) * (cc + c1);
-        }
-        ay = fh - fy;
+        double c = cc + c1, vh = v;
+        if (SCHEME == kFCT4 && (m1 & sk[((J + 1) & 3) * G::P] & kIV))
+          c = ft14 * c + ft24 * (Q(G::C, (J + 1) & 3) + c2);
+        else
+          vh = half_of(v);
+        ay = vh * c - fy;
       }
-      const float af = f32_away(ay);
+      af = f32_away(ay);
 
       // B: low-order solution of row J-1
-      fl = fl << 8 | m1 | (sk[s1 * G::P - 1] & kIP ? kW : 0) | (sk[s1 * G::P + 1] & kIP ? kE : 0) |
+      fl |= m1 | (sk[s1 * G::P - 1] & kIP ? kW : 0) | (sk[s1 * G::P + 1] & kIP ? kE : 0) |
            (m2 & kIP ? kS : 0) | (m0 & kIP ? kN : 0);
-      long long kx1 = 0, kn1 = 0;
-      double lo1 = 0.0;
       if (m1 & kIP) {
         const long long kc = dkey(f1), kw = dkey(Q(G::F, s1, fl & kW ? -1 : 0)), ke = dkey(Q(G::F, s1, fl & kE ? 1 : 0)),
                         ks = fl & kS ? dkey(f2) : kc, kn = fl & kN ? dkey(fc) : kc;
@@ -238,14 +260,13 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
       Q(G::KN, p1) = __longlong_as_double(kn1);
 
       // D: Zalesak bounds (keys) and ratios of row J-2.  A ratio is 1 unless
-      // qp < famax, which holds at a few cells only, those near an extremum of
-      // the field: FP32 bounds of the two sides (below qp, above famax, 2^-18
+      // qp < famax, mostly on one side of a cell (the side t and t-1 do not
+      // differ towards): FP32 bounds of the two sides (below qp, above famax, 2^-18
       // apart where the roundings of either are below 2^-20) settle the others
       // without the eight FP64 operations of each side.  famax = 0: every flux
       // the ratio multiplies is 0.
       const uint32_t w2 = fl >> 8;
-      const long long kx2 = __double_as_longlong(Q(G::KX, p0)), kn2 = __double_as_longlong(Q(G::KN, p0));
-      long long qx = 0, qn = 0;
+      kx2 = __double_as_longlong(Q(G::KX, p0)), kn2 = __double_as_longlong(Q(G::KN, p0));
       double rp = 1.0, rm = 1.0;
       if (w2 & kIP) {
         const int dw = w2 & kW ? -1 : 0, de = w2 & kE ? 1 : 0;
@@ -260,12 +281,14 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
         const float qf = __uint_as_float(reinterpret_cast<const uint2 *>(&S(G::RQ, (J - 2) & 7))->y);
         const float amax = (fmaxf(xa, 0.0f) - fminf(xb, 0.0f)) + (fmaxf(ya, 0.0f) - fminf(yb, 0.0f));
         const float amin = (fmaxf(xb, 0.0f) - fminf(xa, 0.0f)) + (fmaxf(yb, 0.0f) - fminf(ya, 0.0f));
-        const bool ex = !(f32_below(dmx) * qf > amax * 1.000004f || amax == 0.0f);
-        const bool en = !(f32_below(dmn) * qf > amin * 1.000004f || amin == 0.0f);
+        bool ex = !(f32_below(dmx) * qf > amax * 1.000004f || amax == 0.0f);
+        bool en = !(f32_below(dmn) * qf > amin * 1.000004f || amin == 0.0f);
+        // at an extremum the distance is 0, and so is the ratio
+        const float inf = __int_as_float(0x7F800000);
+        if (ex && __double_as_longlong(dmx) == 0 && qf > 0.0f && amax < inf) ex = false, rp = 0.0;
+        if (en && __double_as_longlong(dmn) == 0 && qf > 0.0f && amin < inf) en = false, rm = 0.0;
         if (ex || en) {
-          const long long o = xc + (long long)(J - 2 + nb - 1) * ld1;
-          const double d = dpk[o], scl = A.scal[o];
-          const double fcn = A.mode == 0 ? kmax(x3 ? x3[o] * d : d, 0.0) : d;
+          const double fcn = S(G::FCN, s2), scl = S(G::SCL, (J - 2) & 7);
           const double fxa = Q(G::FA, s2), fxb = Q(G::FA, s2, de), fya = ay2, fyb = w2 & kN ? ay1 : ay2;
           if (ex) {
             const double famax = pos0(fxa) - neg0(fxb) + pos0(fya) - neg0(fyb);
@@ -284,7 +307,7 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
 
       // E: limited fluxes, x of row J-3 and y of face J-2
       const double rp3 = Q(G::RP, p1), rm3 = Q(G::RM, p1);
-      double xl = 0.0, yl = 0.0;
+      double xl = 0.0;
       if (fl >> 16 & kIU) {
         const double f = Q(G::FA, (J - 3) & 3);
         const bool neg = lt0(f);
@@ -303,7 +326,7 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
       const int j = J - 4;
       if ((fl >> 24 & kIP) && j >= j0 && j <= jj && t >= 3 && t < NT - 3 && i <= ii) {
         const double fdv =
-            mul_rn(mul_rn((Q(G::FXL, p0, 1) - Q(G::FXL, p0)) + (yl3 - yl4), dt2), S(G::SCI, j & 7));
+            ((Q(G::FXL, p0, 1) - Q(G::FXL, p0)) + (yl3 - yl4)) * dt2 * S(G::SCI, j & 7);
         const uint32_t R = reinterpret_cast<const uint2 *>(&S(G::RQ, j & 7))->x;
         const double res = from_dkey(max(qn4, min(qx4, dkey(lo4 - div_by(fdv, S(G::HN, j & 7), R)))));
         const long long o = (long long)(j + nb - 1) * ld1;
@@ -312,6 +335,7 @@ __device__ __forceinline__ void march_body(const TileArgs &A, const int strip, c
           if (i <= A.images) out[o + ii] = res;
           if (i > ii - A.images) out[o - ii] = res;
         }
+      }
       }
 
       f2 = f1, f1 = fc;
@@ -337,7 +361,37 @@ __global__ void __launch_bounds__(NT *NG, 512 / (NT * NG)) march_kernel(const Ti
   const int ngrp = (A.nfld + NG - 1) / NG;
   const int k = blockIdx.z / ngrp, q = blockIdx.z - k * ngrp;
   const int j0 = 1 + blockIdx.y * nrow;
-  march_body<SCHEME, NT, NG>(A, blockIdx.x, j0, min(nrow, A.jj + 1 - j0), k, q * NG, smc);
+  march_body<SCHEME, NT, NG>(A, A.f, blockIdx.x, j0, min(nrow, A.jj + 1 - j0), k, q * NG, smc);
+}
+
+// Persistent form for an ensemble of basins: CTAs take work items (basin,
+// strip * kMaxMarchGroups + field group, first row, layer) from a queue until
+// it is empty.  The item's basin is staged in shared memory but for its fields: the
+// full TileArgs would leave room for three CTAs on an SM instead of four.
+template <int SCHEME, int NT, int NG>
+__global__ void __launch_bounds__(NT *NG, 512 / (NT * NG))
+    march_queue_kernel(const TileArgs *__restrict__ basins, const int4 *__restrict__ items, int nitems, int *head) {
+  extern __shared__ __align__(16) char smc[];
+  __shared__ int cur;
+  __shared__ __align__(8) int sa[offsetof(TileArgs, f) / 4];
+  int basin = -1;
+  for (;;) {
+    __syncthreads();  // every thread has read cur
+    if (threadIdx.x == 0) cur = atomicAdd(head, 1);
+    __syncthreads();
+    const int it = cur;
+    if (it >= nitems) break;
+    const int4 w = items[it];
+    if (w.x != basin) {  // the previous item's readers of sa passed the barriers above
+      basin = w.x;
+      const int *src = reinterpret_cast<const int *>(basins + basin);
+      for (int q = threadIdx.x; q < (int)(offsetof(TileArgs, f) / 4); q += NT * NG) sa[q] = src[q];
+      __syncthreads();
+    }
+    const TileArgs &A = *reinterpret_cast<const TileArgs *>(sa);
+    const int strip = w.y / kMaxMarchGroups, q = w.y - strip * kMaxMarchGroups;
+    march_body<SCHEME, NT, NG>(A, basins[basin].f, strip, w.z, min(A.seg, A.jj + 1 - w.z), w.w, q * NG, smc);
+  }
 }
 
 }  // namespace hyc
