@@ -7,8 +7,12 @@
 // of oneta(m) that turns the filtered thickness back into dp) are computed
 // once per cell and reused by every layer.  FP64, built without FMA
 // contraction, in the reference's operation order: the filtered values equal
-// the oracle's bit for bit (the division by oneta(m) is the correctly
-// rounded div_rcp of hyc_device.cuh).  Only temperature-advecting hybrid
+// the oracle's bit for bit.  The filter is bound by the FP64 pipe: divisions,
+// square root and the products of the equation of state and of the scalars'
+// weights run on the integer pipes, the remaining products on the FP64 pipe
+// (all of them on the integer pipes overflow the instruction cache: 1.37 ms):
+// T and S, 1500x1100x10, 1.98 -> 1.23 ms (FP64 pipe 84 -> 75 %, issue slots
+// 12 -> 48 %).  Only temperature-advecting hybrid
 // layers are supported: the 17-term equation of state has no tofsig.
 #include <cuda_runtime.h>
 
@@ -49,11 +53,24 @@ __global__ void asselin_save_kernel(const AsselinArgs A) {
       A.onetao[nn * sl + c] = on;
       A.onetao[mm * sl + c] = om;
     }
-    for (int k = 0; k < kk; k++) {
+    int k = 0;
+    // four layers' loads in flight at a time (one layer's at a time: 36 % of HBM)
+    for (; k + 4 <= kk; k += 4) {
+      const long long lk = k * sl + c, ln = ((long long)k + (long long)nn * kk) * sl + c;
+      double tv[4], sv[4], dv[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) tv[r] = A.temp[ln + r * sl], sv[r] = A.saln[ln + r * sl], dv[r] = A.th3d[ln + r * sl];
+#pragma unroll
+      for (int r = 0; r < 4; r++) A.otemp[lk + r * sl] = tv[r], A.osaln[lk + r * sl] = sv[r], A.oth3d[lk + r * sl] = dv[r];
+    }
+    for (; k < kk; k++) {
       const long long lk = k * sl + c, ln = ((long long)k + (long long)nn * kk) * sl + c;
       A.otemp[lk] = A.temp[ln];
       A.osaln[lk] = A.saln[ln];
       A.oth3d[lk] = A.th3d[ln];
+    }
+    for (k = 0; (A.ntracr > 0 || A.mxlmy) && k < kk; k++) {
+      const long long lk = k * sl + c, ln = ((long long)k + (long long)nn * kk) * sl + c;
       for (int q = 0; q < A.ntracr; q++)
         A.otracer[(long long)q * kk * sl + lk] = A.tracer[(long long)q * 2 * kk * sl + ln];
       if (A.mxlmy) {  // q2(…,k,n) with k 1-based in 0:kk+1
@@ -69,9 +86,9 @@ __global__ void asselin_save_kernel(const AsselinArgs A) {
 __device__ __forceinline__ double ra_scalar(double fo, double fm, double fn, double dpold, double dpmid, double dpnew,
                                             double hra, double qdpmidn) {
   const double smin = kmin(kmin(fo, fm), fn);
-  const double dpsold = dpold * (fo - smin), dpsmid = dpmid * (fm - smin), dpsnew = dpnew * (fn - smin);
-  const double q = hra * (dpsold + dpsnew - 2.0 * dpsmid);
-  return smin + (dpsmid + q) * qdpmidn;
+  const double dpsold = mul_rn(dpold, fo - smin), dpsmid = mul_rn(dpmid, fm - smin), dpsnew = mul_rn(dpnew, fn - smin);
+  const double q = hra * (dpsold + dpsnew - twice_of(dpsmid));
+  return smin + mul_rn(dpsmid + q, qdpmidn);
 }
 
 // asselin_filter for advflg = 0 hybrid layers (:106-236)
@@ -85,15 +102,15 @@ __global__ void asselin_filter_kernel(const AsselinArgs A) {
     const double on = oneta_of(A, c, nn), om = oneta_of(A, c, mm);
     A.oneta[nn * sl + c] = on;
     A.oneta[mm * sl + c] = om;
-    const double ron = rcp_rn(om);
+    const uint32_t rom = recip_of(om);
     const double oon = A.onetao[nn * sl + c], oom = A.onetao[mm * sl + c];
     for (int k = 0; k < kk; k++) {
       const long long lk = k * sl + c, lm = ((long long)k + (long long)mm * kk) * sl + c,
                       ln = ((long long)k + (long long)nn * kk) * sl + c;
       const double dpold = A.dpo[ln] * oon, dpmid = A.dpo[lm] * oom, dpnew = A.dp[ln] * on;
-      const double q = hra * (dpold + dpnew - 2.0 * dpmid);
+      const double q = mul_rn(hra, dpold + dpnew - twice_of(dpmid));
       const double dpmidn = dpmid + q;
-      A.dp[lm] = div_rcp(dpmidn, om, ron);
+      A.dp[lm] = div_by(dpmidn, om, rom);
       if (!(dpmidn > kOnezm)) continue;
       const double qdpmidn = rcp_rn(dpmidn);
       const double s = ra_scalar(A.osaln[lk], A.saln[lm], A.saln[ln], dpold, dpmid, dpnew, hra, qdpmidn);

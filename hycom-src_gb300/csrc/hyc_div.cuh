@@ -36,6 +36,7 @@
 #pragma once
 #include <cstdint>
 #include <cstring>
+#include <cmath>
 
 #ifdef __CUDACC__
 #define HYC_HD __host__ __device__ __forceinline__
@@ -116,6 +117,7 @@ HYC_HD float seed(float x) {
 #ifdef __CUDACC__
 static __device__ __noinline__ double slow_mul(double a, double b) { return a * b; }
 static __device__ __noinline__ double slow_div(double a, double b) { return a / b; }
+static __device__ __noinline__ double slow_sqrt(double a) { return sqrt(a); }
 #endif
 HYC_HD double fp64_mul(double a, double b) {
 #ifdef __CUDA_ARCH__
@@ -129,6 +131,24 @@ HYC_HD double fp64_div(double a, double b) {
   return slow_div(a, b);
 #else
   return a / b;
+#endif
+}
+HYC_HD double fp64_sqrt(double a) {
+#ifdef __CUDA_ARCH__
+  return slow_sqrt(a);
+#else
+  return sqrt(a);
+#endif
+}
+// FP32 reciprocal square root of x in [1,4), relative error below 2^-21.7
+// (the hardware's approximation is within 2 ulp)
+HYC_HD float rseed(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return (float)(1.0 / sqrt((double)x));
 #endif
 }
 HYC_HD uint64_t significand(uint64_t b) { return (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull; }
@@ -219,6 +239,50 @@ HYC_HD double mul_rn(double a, double b) {
   // exponents and signs add; -1 for the significand's own bit 52
   const uint32_t ex = (ha & 0xFFF00000u) + (hb & 0xFFF00000u) - 0x3FF00000u - (sh << 20);
   return from_bits(q + ((uint64_t)ex << 32));
+}
+
+// x/2 and 2x, exact
+HYC_HD double half_of(double x) {
+  const uint64_t b = idiv::bits(x);
+  return idiv::mid_range((uint32_t)(b >> 32)) ? idiv::from_bits(b - (1ull << 52)) : idiv::fp64_mul(x, 0.5);
+}
+HYC_HD double twice_of(double x) {
+  const uint64_t b = idiv::bits(x);
+  return idiv::mid_range((uint32_t)(b >> 32)) ? idiv::from_bits(b + (1ull << 52)) : idiv::fp64_mul(x, 2.0);
+}
+
+// sqrt(x), correctly rounded, on the integer pipes.  x = M*2^2k, M in
+// [2^52, 2^54); q = floor(sqrt(M*2^54)) has 54 bits and its last one rounds
+// (no square root of 53 bits lies halfway).  q = a*2^26 + b: a, 28 bits, from
+// the FP32 seed y = 1/sqrt and one Newton step (within 2), b from the
+// remainder r = 4M - a^2 times y (within 70), then from the exact remainder
+// again (within 1), which also settles the last unit.  The remainders are
+// below 2^62, so arithmetic modulo 2^64 holds them.
+HYC_HD double sqrt_rn(double x) {
+  using namespace idiv;
+  const uint64_t ib = bits(x);
+  const uint32_t h = (uint32_t)(ib >> 32);
+  if (!(mid_range(h) && (int32_t)h > 0)) return fp64_sqrt(x);
+  const uint32_t odd = ~(h >> 20) & 1u;  // of the unbiased exponent
+  const uint64_t M = significand(ib) << odd;
+  const float xf = u2f(((127u + odd) << 23) | ((uint32_t)(ib >> 29) & 0x7FFFFFu));
+  const float y = fminf(fmaxf(rseed(xf), 0.5f), 0.99999994f);        // in [0.5, 1)
+  const float af = fminf(fmaxf(xf * y, 1.0f), 1.9999999f);          // sqrt, in [1, 2)
+  const int32_t yi = (int32_t)((f2u(y) & 0x7FFFFFu) | 0x800000u);   // y*2^24
+  const uint32_t a0 = ((f2u(af) & 0x7FFFFFu) | 0x800000u) << 4;     // sqrt*2^27
+  const uint64_t H = M << 2;
+  const int64_t d = (int64_t)(H - (uint64_t)a0 * a0);
+  const uint32_t a = a0 + (uint32_t)(mulhi_s((int32_t)(d >> 6), yi) >> 14);
+  const int32_t r = (int32_t)(uint32_t)(H - (uint64_t)a * a);
+  const int32_t b = mulhi_s(r, yi << 6);
+  const uint64_t Q = ((uint64_t)a << 26) + (uint64_t)(int64_t)b;
+  const uint64_t rem = ((uint64_t)(uint32_t)r << 52) - (uint64_t)(int64_t)b * (Q + ((uint64_t)a << 26));
+  const int32_t db = mulhi_s((int32_t)((int64_t)rem >> 34), yi << 6) >> 18;
+  uint64_t q = Q + (uint64_t)(int64_t)db;
+  const int64_t rem1 = (int64_t)(rem - (uint64_t)(int64_t)db * (Q + q));
+  q = rem1 < 0 ? q - 1 : rem1 > (int64_t)(q << 1) ? q + 1 : q;
+  const uint32_t ex = (((h >> 20) + 1u) >> 1) + 510u;  // the result's exponent field, less one for bit 52
+  return from_bits(((q + 1) >> 1) + ((uint64_t)ex << 52));
 }
 
 }  // namespace hyc

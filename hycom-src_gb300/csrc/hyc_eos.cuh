@@ -3,7 +3,8 @@
 // coefficients, :496-505 sig; EOS_17T with EOS_SIG2), in the reference's
 // operation order.  Built without FMA contraction by its users, sig17 equals
 // the reference's sig() bit for bit (one correctly rounded reciprocal and
-// square root).  The 17-term form has no inverse (tofsig is "not available",
+// square root).  Products, reciprocal and square root run on the integer
+// pipes: its callers are bound by the FP64 pipe, which keeps the 15 sums.  The 17-term form has no inverse (tofsig is "not available",
 // stmt_fns.h:530-532), so only temperature-advecting layers can use it.
 #pragma once
 #include "hyc_device.cuh"
@@ -31,11 +32,12 @@ constexpr double c101 = c001 + (c018 - c021 * kRpdb) * kRpdb, c103 = c003 + (c01
 // sig(t,s) = sig_n*sig_q - 1000, sig_q = 1/sig_d (stmt_fns.h:497-505)
 __device__ __forceinline__ double sig17(double t, double s) {
   using namespace eos17;
-  const double sn = c101 + t * (c002 + t * (c103 + t * c004)) + s * (c105 - t * c006 + s * c007);
-  const double sd = c108 + t * (c109 + t * (c010 + t * (c111 + t * c012))) +
-                    s * (c013 - t * (c014 + t * t * c015) + sqrt(pos0(s)) * (c016 + t * t * c017));
-  const double sq = rcp_rn(sd);  // aone/sig_d, correctly rounded
-  return sn * sq - 1000.0;
+  const double tt = mul_rn(t, t);
+  const double sn = c101 + mul_rn(t, c002 + mul_rn(t, c103 + mul_rn(t, c004))) +
+                    mul_rn(s, c105 - mul_rn(t, c006) + mul_rn(s, c007));
+  const double sd = c108 + mul_rn(t, c109 + mul_rn(t, c010 + mul_rn(t, c111 + mul_rn(t, c012)))) +
+                    mul_rn(s, c013 - mul_rn(t, c014 + mul_rn(tt, c015)) + mul_rn(sqrt_rn(pos0(s)), c016 + mul_rn(tt, c017)));
+  return mul_rn(sn, rcp_rn(sd)) - 1000.0;  // aone/sig_d, correctly rounded
 }
 
 }  // namespace hyc

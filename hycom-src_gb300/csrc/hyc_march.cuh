@@ -51,12 +51,6 @@ struct MarchGeom {
   static constexpr size_t smem_bytes = MSK + 4 * P;
 };
 
-// x/2, exact (the FP64 pipe is left to operands near the ends of the range)
-__device__ __forceinline__ double half_of(double x) {
-  const int h = __double2hiint(x);
-  return idiv::mid_range((uint32_t)h) ? __hiloint2double(h - 0x100000, __double2loint(x)) : idiv::fp64_mul(x, 0.5);
-}
-
 // 8 bytes from global to shared memory, or zeros
 __device__ __forceinline__ void copy8(void *dst, const double *src, bool in) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
