@@ -10,10 +10,16 @@
 // first GPU form keeps that structure: one kernel per sweep over the same
 // margin, layer after layer, so every value the reference computes (halo
 // cells included) is computed here, in the same operation order, FP64
-// without FMA contraction: the results equal the oracle's bit for bit.  The
-// sweeps are memory-bound (about 55 slice reads/writes per cell and layer
-// against 11 for a fused form); a tile kernel that walks the layers with a
-// six-cell halo is the next form.
+// without FMA contraction: the results equal the oracle's bit for bit.
+//
+// What bounds them: at the start the FP64 pipe (71-82 % busy in every sweep);
+// with products and divisions on the integer pipes (hyc_div.cuh) the pipe, the
+// integer pipes and the memory system are each half to two thirds busy, so the
+// operands of a sweep are loaded before the first is used.  1500x1100, one
+// layer, before / after: cn_flux 45 / 41 us, cn_low 27 / 24, cn_ratio 55 / 32,
+// cn_clip 40 / 26, cn_update 27 / 25, cn_btflux 37 / 28, cn_thk_util 34 / 27,
+// cn_thk_flux 112 / 82, cn_thk_p 21 / 19.  The sweeps move about 55 slices per
+// cell and layer against 11 for a fused form.
 //
 // Work slices (CnuityArgs::w): uflux, vflux, uflux2, vflux2, utotn, vtotn,
 // util1, util2, util3, pold, oneta_u, oneta_v, onetamas(:,:,1:2).
@@ -58,6 +64,15 @@ __device__ __forceinline__ double *W(const CnuityArgs &A, int s) { return A.w + 
 // never reach a result of this path)
 __device__ __forceinline__ double mx(double a, double b) { return kmax(a, b); }
 __device__ __forceinline__ double mn(double a, double b) { return kmin(a, b); }
+
+__device__ __forceinline__ bool is0(double x) { return (unsigned long long)__double_as_longlong(x) << 1 == 0; }
+// q*x, q finite: x = 0 (thin layers) does not go to the FP64 pipe
+__device__ __forceinline__ double scaled(double q, double x) { return is0(x) ? 0.0 : mul_rn(q, x); }
+// -x without the FP64 pipe
+__device__ __forceinline__ double minus(double x) {
+  return __longlong_as_double(__double_as_longlong(x) ^ (long long)0x8000000000000000ULL);
+}
+__device__ __forceinline__ bool finite(double x) { return (__double2hiint(x) & 0x7FF00000) != 0x7FF00000; }
 
 // :112-157 at margin 6
 __global__ void cn_init(const CnuityArgs A) {
@@ -110,24 +125,30 @@ __global__ void cn_flux(const CnuityArgs A, int k) {
   const double *dk = A.dp + ((long long)k + (long long)nn * A.kdm) * sl;
   const double *u3 = W(A, W_U3), *omn = W(A, W_OM) + nn * sl;
   const long long lm = ((long long)k + (long long)mm * A.kdm) * sl;
+  if (!(mk & (kIU | kIV))) return;
+  // every operand is loaded before the first is used: the upwind cell is
+  // known only after the velocity is
+  const double d0 = dk[c], dw = dk[c - 1], ds = dk[c - ld], t0 = u3[c], tw = u3[c - 1], ts = u3[c - ld];
+  const double uu = A.u[lm + c], ub = A.ubavg[mm * sl + c], su = A.scuy[c], du = A.depthu[c], hu = A.dpu[lm + c];
+  const double vv = A.v[lm + c], vb = A.vbavg[mm * sl + c], sv = A.scvx[c], dv = A.depthv[c], hv = A.dpv[lm + c];
   if (mk & kIU) {
-    const double utotm = (A.u[lm + c] + A.ubavg[mm * sl + c]) * A.scuy[c];
-    const long long cq = ge0(utotm) ? c - 1 : c;
-    const double q0 = mn(dk[cq], mx(0., A.depthu[c] - u3[cq]));
-    const double uf = utotm * (BT ? q0 * omn[cq] : q0);
+    const double utotm = mul_rn(uu + ub, su);
+    const bool up = ge0(utotm);
+    const double q0 = mn(up ? dw : d0, mx(0., du - (up ? tw : t0)));
+    const double uf = mul_rn(utotm, BT ? mul_rn(q0, omn[up ? c - 1 : c]) : q0);
     W(A, W_UF)[c] = uf;
-    const double ud = utotm * A.dpu[lm + c];
-    W(A, W_UF2)[c] = (BT ? ud * W(A, W_OU)[c] : ud) - uf;
+    const double ud = mul_rn(utotm, hu);
+    W(A, W_UF2)[c] = (BT ? mul_rn(ud, W(A, W_OU)[c]) : ud) - uf;
     A.uflx[(long long)k * sl + c] = uf;
   }
   if (mk & kIV) {
-    const double vtotm = (A.v[lm + c] + A.vbavg[mm * sl + c]) * A.scvx[c];
-    const long long cq = ge0(vtotm) ? c - ld : c;
-    const double q0 = mn(dk[cq], mx(0., A.depthv[c] - u3[cq]));
-    const double vf = vtotm * (BT ? q0 * omn[cq] : q0);
+    const double vtotm = mul_rn(vv + vb, sv);
+    const bool up = ge0(vtotm);
+    const double q0 = mn(up ? ds : d0, mx(0., dv - (up ? ts : t0)));
+    const double vf = mul_rn(vtotm, BT ? mul_rn(q0, omn[up ? c - ld : c]) : q0);
     W(A, W_VF)[c] = vf;
-    const double vd = vtotm * A.dpv[lm + c];
-    W(A, W_VF2)[c] = (BT ? vd * W(A, W_OV)[c] : vd) - vf;
+    const double vd = mul_rn(vtotm, hv);
+    W(A, W_VF2)[c] = (BT ? mul_rn(vd, W(A, W_OV)[c]) : vd) - vf;
     A.vflx[(long long)k * sl + c] = vf;
   }
 }
@@ -155,8 +176,8 @@ __global__ void cn_low(const CnuityArgs A, int k) {
     double *dk = A.dp + ((long long)k + (long long)nn * A.kdm) * sl;
     const double *uf = W(A, W_UF), *vf = W(A, W_VF);
     W(A, W_U3)[c] = W(A, W_U3)[c] + dk[c];
-    d = (BT ? dk[c] * W(A, W_OM)[nn * sl + c] : dk[c]) -
-        ((uf[c + 1] - uf[c]) + (vf[c + ld] - vf[c])) * A.delt1 * A.scp2i[c];
+    d = (BT ? mul_rn(dk[c], W(A, W_OM)[nn * sl + c]) : dk[c]) -
+        mul_rn(mul_rn((uf[c + 1] - uf[c]) + (vf[c + ld] - vf[c]), A.delt1), A.scp2i[c]);
     dk[c] = d;
     A.dpo[((long long)k + (long long)mm * A.kdm) * sl + c] = d;
     sea = true;
@@ -180,10 +201,37 @@ __global__ void cn_ratio(const CnuityArgs A, int k) {
   const double u1 = mx(mx(mx(mx(d, dk[ca]), dk[cb]), dk[cja]), dk[cjb]);
   const double u2 = mx(0., mn(mn(mn(mn(d, dk[ca]), dk[cb]), dk[cja]), dk[cjb]));
   const double *f2u = W(A, W_UF2), *f2v = W(A, W_VF2);
-  W(A, W_U1)[c] = div_rn(u1 - d, (((pos0(f2u[c]) - neg0(f2u[c + 1])) + (pos0(f2v[c]) - neg0(f2v[c + ld]))) + kEpsilCb) *
-                                     A.delt1 * A.scp2i[c]);
-  W(A, W_U2)[c] = div_rn(u2 - d, (((neg0(f2u[c]) - pos0(f2u[c + 1])) + (neg0(f2v[c]) - pos0(f2v[c + ld]))) - kEpsilCb) *
-                                     A.delt1 * A.scp2i[c]);
+  const double fu0 = f2u[c], fu1 = f2u[c + 1], fv0 = f2v[c], fv1 = f2v[c + ld];
+  // The ratios are used as min(1, ratio) only.  FP32 bounds (below the
+  // numerator, above the denominator) show most of them to be at least 1, and
+  // a numerator of 0 gives 0; the rest take the division.
+  const float a0 = f32_away(fu0), a1 = f32_away(fu1), b0 = f32_away(fv0), b1 = f32_away(fv1);
+  const float ds = f32_away(A.delt1) * f32_away(A.scp2i[c]);
+  const float in = ((fmaxf(a0, 0.0f) - fminf(a1, 0.0f)) + (fmaxf(b0, 0.0f) - fminf(b1, 0.0f))) + 1.0001e-11f;
+  const float out = ((fmaxf(a1, 0.0f) - fminf(a0, 0.0f)) + (fmaxf(b1, 0.0f) - fminf(b0, 0.0f))) + 1.0001e-11f;
+  const float din = in * ds * 1.000004f, dout = out * ds * 1.000004f;
+  const bool fine = ds > 1e-30f && din > 1e-30f && dout > 1e-30f && din < 1e37f && dout < 1e37f;
+  const double n1 = u1 - d, n2 = d - u2;  // the second ratio with both signs turned
+  double r1 = 1.0, r2 = 1.0;
+  if (!(fine && f32_below(n1) > din)) {
+    r1 = 0.0;
+    if (!(fine && is0(n1)))
+      r1 = div_rn(n1, mul_rn(mul_rn(((pos0(fu0) - neg0(fu1)) + (pos0(fv0) - neg0(fv1))) + kEpsilCb, A.delt1), A.scp2i[c]));
+  }
+  if (!(fine && f32_below(n2) > dout)) {
+    r2 = 0.0;
+    if (!(fine && is0(n2)))
+      r2 = div_rn(n2, mul_rn(mul_rn(((pos0(fu1) - neg0(fu0)) + (pos0(fv1) - neg0(fv0))) + kEpsilCb, A.delt1), A.scp2i[c]));
+  }
+  W(A, W_U1)[c] = r1;
+  W(A, W_U2)[c] = r2;
+}
+
+// f2*clip; the part clipped off is added to rest (nothing where clip = 1)
+__device__ __forceinline__ double clipped(double f2, double clip, double *rest) {
+  if (__double_as_longlong(clip) == kOneBits && finite(f2)) return f2;
+  *rest = *rest + mul_rn(f2, 1. - clip);
+  return mul_rn(f2, clip);
 }
 
 // :442-472 at margin 3: clip the antidiffusive fluxes
@@ -192,22 +240,24 @@ __global__ void cn_clip(const CnuityArgs A, int k) {
   if (!cell_of(A, 3, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
   const uint8_t mk = A.msk[c];
+  if (!(mk & (kIU | kIV))) return;
   const double *u1 = W(A, W_U1), *u2 = W(A, W_U2);
+  double *ul = A.uflx + (long long)k * sl + c, *vl = A.vflx + (long long)k * sl + c;
+  const double a1 = u1[c], a2 = u2[c], w1 = u1[c - 1], w2 = u2[c - 1], s1 = u1[c - ld], s2 = u2[c - ld];
+  const double f2 = W(A, W_UF2)[c], g2 = W(A, W_VF2)[c], ul0 = *ul, vl0 = *vl;
   if (mk & kIU) {
-    const double f2 = W(A, W_UF2)[c];
-    const double clip = ge0(f2) ? mn(mn(1., u1[c]), u2[c - 1]) : mn(mn(1., u2[c]), u1[c - 1]);
-    W(A, W_UTN)[c] = W(A, W_UTN)[c] + f2 * (1. - clip);
-    const double uf = f2 * clip;
+    const bool up = ge0(f2);
+    const double clip = mn(mn(1., up ? a1 : a2), up ? w2 : w1);
+    const double uf = clipped(f2, clip, W(A, W_UTN) + c);
     W(A, W_UF)[c] = uf;
-    A.uflx[(long long)k * sl + c] = A.uflx[(long long)k * sl + c] + uf;
+    *ul = ul0 + uf;
   }
   if (mk & kIV) {
-    const double f2 = W(A, W_VF2)[c];
-    const double clip = ge0(f2) ? mn(mn(1., u1[c]), u2[c - ld]) : mn(mn(1., u2[c]), u1[c - ld]);
-    W(A, W_VTN)[c] = W(A, W_VTN)[c] + f2 * (1. - clip);
-    const double vf = f2 * clip;
+    const bool up = ge0(g2);
+    const double clip = mn(mn(1., up ? a1 : a2), up ? s2 : s1);
+    const double vf = clipped(g2, clip, W(A, W_VTN) + c);
     W(A, W_VF)[c] = vf;
-    A.vflx[(long long)k * sl + c] = A.vflx[(long long)k * sl + c] + vf;
+    *vl = vl0 + vf;
   }
 }
 
@@ -223,7 +273,7 @@ __global__ void cn_update(const CnuityArgs A, int k, int M, int slot) {
     const int nn = A.n - 1;
     double *dk = A.dp + ((long long)k + (long long)nn * A.kdm) * sl;
     const double *uf = W(A, W_UF), *vf = W(A, W_VF);
-    d = dk[c] - ((uf[c + 1] - uf[c]) + (vf[c + ld] - vf[c])) * A.delt1 * A.scp2i[c];
+    d = dk[c] - mul_rn(mul_rn((uf[c + 1] - uf[c]) + (vf[c + ld] - vf[c]), A.delt1), A.scp2i[c]);
     dk[c] = d;
     A.p[(long long)(k + 1) * sl + c] = A.p[(long long)k * sl + c] + d;
     sea = true;
@@ -231,21 +281,21 @@ __global__ void cn_update(const CnuityArgs A, int k, int M, int slot) {
   if (A.keys && slot >= 0) row_min(A, x, in && sea, d, slot);
 }
 
-// loop 77: RN(1/p(kk+1)) of every sea cell at margin 2, into util1 (free
-// until the interface diffusion).  p(kk+1) does not change during loop 77
-// before its last layer's fluxes are formed, so one reciprocal per cell
-// serves every layer's division dp/p(kk+1).
+// loop 77: the 32-bit reciprocal (recip_of) of p(kk+1) of every sea cell at
+// margin 2, into util1 (free until the interface diffusion).  p(kk+1) does
+// not change during loop 77 before its last layer's fluxes are formed, so one
+// reciprocal per cell serves every layer's division dp/p(kk+1).
 __global__ void cn_rpb(const CnuityArgs A) {
   Cell x;
   if (!cell_of(A, 2, x)) return;
   const long long c = x.c;
   if (!(A.msk[c] & kIP)) return;
-  W(A, W_U1)[c] = rcp_rn(A.p[(long long)A.kdm * A.slice + c]);
+  W(A, W_U1)[c] = __longlong_as_double(recip_of(A.p[(long long)A.kdm * A.slice + c]));
 }
 
 // loop 77, :595-645 at margin 1: the barotropic correction fluxes of layer k.
-// q = dp/p(kk+1) by div_rcp with the cell's reciprocal: the IEEE quotient
-// bit for bit, for 5 FP64 operations instead of a division.
+// q = dp/p(kk+1) by div_by with the cell's reciprocal.  A face that clipped
+// nothing (most) has no correction flux: uf = 0*q = 0 for its finite q.
 __global__ void cn_btflux(const CnuityArgs A, int k) {
   Cell x;
   if (!cell_of(A, 1, x)) return;
@@ -254,19 +304,26 @@ __global__ void cn_btflux(const CnuityArgs A, int k) {
   const int nn = A.n - 1;
   const double *dk = A.dp + ((long long)k + (long long)nn * A.kdm) * sl, *pb = A.p + (long long)A.kdm * sl;
   const double *rpb = W(A, W_U1);
+  if (!(mk & (kIU | kIV))) return;
+  double *ul = A.uflx + (long long)k * sl + c, *vl = A.vflx + (long long)k * sl + c;
+  const double ut = W(A, W_UTN)[c], vt = W(A, W_VTN)[c], d0 = dk[c], dw = dk[c - 1], ds = dk[c - ld], p0 = pb[c],
+               pw = pb[c - 1], ps = pb[c - ld], r0 = rpb[c], rw = rpb[c - 1], rs = rpb[c - ld], ul0 = *ul, vl0 = *vl;
+  // the correction flux of a face with transport t from a cell of thickness
+  // d and total depth p, added onto *fl
+  auto flux = [](double t, double d, double p, double r, double l0, double *fl) {
+    const uint32_t R = (uint32_t)__double_as_longlong(r);
+    if (is0(t) && R != 0 && finite(d)) return 0.0;
+    const double f = mul_rn(t, div_by(d, p, R));
+    *fl = l0 + f;
+    return f;
+  };
   if (mk & kIU) {
-    const double ut = W(A, W_UTN)[c];
-    const long long cu = ge0(ut) ? c - 1 : c;
-    const double uf = ut * div_rcp(dk[cu], pb[cu], rpb[cu]);
-    W(A, W_UF)[c] = uf;
-    A.uflx[(long long)k * sl + c] = A.uflx[(long long)k * sl + c] + uf;
+    const bool up = ge0(ut);
+    W(A, W_UF)[c] = flux(ut, up ? dw : d0, up ? pw : p0, up ? rw : r0, ul0, ul);
   }
   if (mk & kIV) {
-    const double vt = W(A, W_VTN)[c];
-    const long long cv = ge0(vt) ? c - ld : c;
-    const double vf = vt * div_rcp(dk[cv], pb[cv], rpb[cv]);
-    W(A, W_VF)[c] = vf;
-    A.vflx[(long long)k * sl + c] = A.vflx[(long long)k * sl + c] + vf;
+    const bool up = ge0(vt);
+    W(A, W_VF)[c] = flux(vt, up ? ds : d0, up ? ps : p0, up ? rs : r0, vl0, vl);
   }
 }
 
@@ -280,7 +337,7 @@ __global__ void cn_bottom(const CnuityArgs A) {
   const double q = div_rn(A.pbot[c], A.p[(long long)A.kdm * sl + c]);
   for (int k = 0; k < A.kdm; k++) {
     double *d = A.dp + ((long long)k + (long long)nn * A.kdm) * sl + c;
-    *d = *d * q;
+    *d = mul_rn(*d, q);
     A.p[(long long)(k + 1) * sl + c] = A.p[(long long)k * sl + c] + *d;
   }
 }
@@ -317,22 +374,22 @@ __global__ void cn_thk_util(const CnuityArgs A, int k) {
   const double *dk = A.dp + ((long long)(k - 1) + (long long)nn * A.kdm) * sl,
                *dkm = A.dp + ((long long)(k - 2) + (long long)nn * A.kdm) * sl, *pk = A.p + (long long)(k - 1) * sl;
   double u1, u2;
-  if (mn(dk[c], dkm[c]) < kOnecm) {
+  if (klt(mn(dk[c], dkm[c]), kOnecm)) {
     u1 = 0.0;
     u2 = 0.0;
   } else {
     const long long ca = nbx(A, c, -1), cb = nbx(A, c, 1), cja = nbx(A, c, -ld), cjb = nbx(A, c, ld);
-    u1 = pk[c] - .5 * (pk[ca] + pk[cb]);
-    u2 = pk[c] - .5 * (pk[cja] + pk[cjb]);
+    u1 = pk[c] - half_of(pk[ca] + pk[cb]);
+    u2 = pk[c] - half_of(pk[cja] + pk[cjb]);
     if (gt0(u1)) {
-      if (mn(dk[ca], dk[cb]) < kOnecm) u1 = 0.0;
+      if (klt(mn(dk[ca], dk[cb]), kOnecm)) u1 = 0.0;
     } else {
-      if (mn(dkm[ca], dkm[cb]) < kOnecm) u1 = 0.0;
+      if (klt(mn(dkm[ca], dkm[cb]), kOnecm)) u1 = 0.0;
     }
     if (gt0(u2)) {
-      if (mn(dk[cja], dk[cjb]) < kOnecm) u2 = 0.0;
+      if (klt(mn(dk[cja], dk[cjb]), kOnecm)) u2 = 0.0;
     } else {
-      if (mn(dkm[cja], dkm[cjb]) < kOnecm) u2 = 0.0;
+      if (klt(mn(dkm[cja], dkm[cjb]), kOnecm)) u2 = 0.0;
     }
   }
   W(A, W_U1)[c] = u1;
@@ -348,7 +405,9 @@ __global__ void cn_thk_util(const CnuityArgs A, int k) {
 // four faces): flxhi = G(i), flxlo = -G(i-1) (negation is exact), and the
 // biharmonic bounds uflux + H, uflux - H of the cells the reference names.
 constexpr int kTX = 32, kTY = 8;  // the block of every cnuity launch
-__global__ void __launch_bounds__(kTX * kTY) cn_thk_flux(const CnuityArgs A, int k, int bih, int iflip) {
+// BIH, IFLIP: compile-time, so that no branch of the other form is predicated in.
+template <bool BIH, bool IFLIP>
+__global__ void __launch_bounds__(kTX * kTY, 6) cn_thk_flux(const CnuityArgs A, int k) {
   __shared__ double sG[kTY + 1][kTX + 1], sH[kTY + 1][kTX + 1];
   Cell x;
   const bool in = cell_of(A, 4, x);
@@ -357,59 +416,65 @@ __global__ void __launch_bounds__(kTX * kTY) cn_thk_flux(const CnuityArgs A, int
   const double *pk = A.p + (long long)(k - 1) * sl, *ptop = A.p + (long long)A.kdm * sl;
   const double *pold = W(A, W_POLD), *scp2 = A.scp2;
   auto terms = [&](long long c, int sy, int sx) {
-    sG[sy][sx] = .25 * (ptop[c] - pk[c]) * scp2[c];
-    if (bih) sH[sy][sx] = iflip == 0 ? .25 * (pk[c] - pold[c]) * scp2[c] : .25 * (pold[c] - pk[c]) * scp2[c];
+    sG[sy][sx] = mul_rn(half_of(half_of(ptop[c] - pk[c])), scp2[c]);
+    if (BIH) sH[sy][sx] = mul_rn(half_of(half_of(IFLIP ? pold[c] - pk[c] : pk[c] - pold[c])), scp2[c]);
   };
-  // the box starts at margin 4, so the west and south neighbours of its
-  // first column and row (margin 5) lie inside the array
-  if (in) {
-    terms(x.c, ty, tx);
-    if (tx == 1) terms(x.c - 1, ty, 0);
-    if (ty == 1) terms(x.c - ld, 0, tx);
-  }
-  __syncthreads();
-  if (!in) return;
+  // every other operand is under way before the terms are exchanged
   const long long c = x.c;
-  const uint8_t mk = A.msk[c];
-  const double dtinv = A.dtinv;
+  const uint8_t mk = in ? A.msk[c] : 0;
   double *uk1 = A.uflx + (long long)(k - 2) * sl, *uk = A.uflx + (long long)(k - 1) * sl;
   double *vk1 = A.vflx + (long long)(k - 2) * sl, *vk = A.vflx + (long long)(k - 1) * sl;
-  const double g = sG[ty][tx];
+  double *uf = W(A, W_UF), *vf = W(A, W_VF);
+  const double *pu = BIH ? W(A, W_U1) : pk, *pv = BIH ? W(A, W_U2) : pk;
+  double tu = 0, uw = 0, uc = 0, uf0 = 0, ul1 = 0, ul0 = 0, tv = 0, vs = 0, vc = 0, vf0 = 0, vl1 = 0, vl0 = 0;
   if (mk & kIU) {
-    double *uf = W(A, W_UF);
-    double flxhi = g, flxlo = -sG[ty][tx - 1];
-    double f;
-    if (bih) {
-      const double hw = sH[ty][tx - 1], h = sH[ty][tx];
-      flxhi = mn(flxhi, uf[c] + (iflip == 0 ? hw : h));
-      flxlo = mx(flxlo, uf[c] - (iflip == 0 ? h : hw));
-      const double thkdfu = A.delt1 * A.thkdfu[c];
-      f = mn(flxhi, mx(flxlo, thkdfu * (W(A, W_U1)[c - 1] - W(A, W_U1)[c])));
-    } else {
-      const double thkdfu = A.delt1 * A.thkdfu[c];
-      f = mn(flxhi, mx(flxlo, thkdfu * (pk[c - 1] - pk[c])));
-    }
-    uf[c] = f;
-    uk1[c] = uk1[c] + f * dtinv;
-    uk[c] = uk[c] - f * dtinv;
+    tu = A.thkdfu[c], uw = pu[c - 1], uc = pu[c], ul1 = uk1[c], ul0 = uk[c];
+    if (BIH) uf0 = uf[c];
   }
   if (mk & kIV) {
-    double *vf = W(A, W_VF);
-    double flxhi = g, flxlo = -sG[ty - 1][tx];
-    double f;
-    if (bih) {
-      const double hs = sH[ty - 1][tx], h = sH[ty][tx];
-      flxhi = mn(flxhi, vf[c] + (iflip == 0 ? hs : h));
-      flxlo = mx(flxlo, vf[c] - (iflip == 0 ? h : hs));
-      const double thkdfv = A.delt1 * A.thkdfv[c];
-      f = mn(flxhi, mx(flxlo, thkdfv * (W(A, W_U2)[c - ld] - W(A, W_U2)[c])));
-    } else {
-      const double thkdfv = A.delt1 * A.thkdfv[c];
-      f = mn(flxhi, mx(flxlo, thkdfv * (pk[c - ld] - pk[c])));
+    tv = A.thkdfv[c], vs = pv[c - ld], vc = pv[c], vl1 = vk1[c], vl0 = vk[c];
+    if (BIH) vf0 = vf[c];
+  }
+  // the box starts at margin 4, so the west and south neighbours of its
+  // first column and row (margin 5) lie inside the array; one warp takes the
+  // block's west column, one its south row
+  if (in) terms(c, ty, tx);
+  const long long c0 = (long long)((int)blockIdx.x * kTX - 3 + A.nb - 1) + (long long)((int)blockIdx.y * kTY - 3 + A.nb - 1) * ld;
+  if (ty == 1 && tx <= kTY && (int)blockIdx.y * kTY + tx - 1 < A.jj + 8) terms(c0 - 1 + (tx - 1) * ld, tx, 0);
+  if (ty == 2 && (int)blockIdx.x * kTX + tx - 1 < A.ii + 8) terms(c0 - ld + tx - 1, 0, tx);
+  __syncthreads();
+  if (!in) return;
+  const double dtinv = A.dtinv;
+  const double g = sG[ty][tx];
+  if (mk & kIU) {
+    double flxhi = g, flxlo = minus(sG[ty][tx - 1]);
+    if (BIH) {
+      const double hw = sH[ty][tx - 1], h = sH[ty][tx];
+      flxhi = mn(flxhi, uf0 + (IFLIP ? h : hw));
+      flxlo = mx(flxlo, uf0 - (IFLIP ? hw : h));
     }
+    const double f = mn(flxhi, mx(flxlo, scaled(mul_rn(A.delt1, tu), uw - uc)));
+    uf[c] = f;
+    if (!is0(f)) {
+      const double ft = mul_rn(f, dtinv);
+      uk1[c] = ul1 + ft;
+      uk[c] = ul0 - ft;
+    }
+  }
+  if (mk & kIV) {
+    double flxhi = g, flxlo = minus(sG[ty - 1][tx]);
+    if (BIH) {
+      const double hs = sH[ty - 1][tx], h = sH[ty][tx];
+      flxhi = mn(flxhi, vf0 + (IFLIP ? h : hs));
+      flxlo = mx(flxlo, vf0 - (IFLIP ? hs : h));
+    }
+    const double f = mn(flxhi, mx(flxlo, scaled(mul_rn(A.delt1, tv), vs - vc)));
     vf[c] = f;
-    vk1[c] = vk1[c] + f * dtinv;
-    vk[c] = vk[c] - f * dtinv;
+    if (!is0(f)) {
+      const double ft = mul_rn(f, dtinv);
+      vk1[c] = vl1 + ft;
+      vk[c] = vl0 - ft;
+    }
   }
 }
 
@@ -422,7 +487,7 @@ __global__ void cn_thk_p(const CnuityArgs A, int k) {
   double *pk = A.p + (long long)(k - 1) * A.slice;
   const double *uf = W(A, W_UF), *vf = W(A, W_VF);
   W(A, W_POLD)[c] = pk[c];
-  pk[c] = pk[c] - ((uf[c + 1] - uf[c]) + (vf[c + ld] - vf[c])) * A.scp2i[c];
+  pk[c] = pk[c] - mul_rn((uf[c + 1] - uf[c]) + (vf[c + ld] - vf[c]), A.scp2i[c]);
 }
 
 // :925-950 at margin 4: interfaces kept ordered, dp(n) from p
@@ -435,7 +500,7 @@ __global__ void cn_thk_final(const CnuityArgs A) {
   for (int k = 0; k < A.kdm; k++) {
     double *p1 = A.p + (long long)(k + 1) * sl + c;
     const double p0 = A.p[(long long)k * sl + c];
-    if (*p1 < p0) *p1 = p0;
+    if (klt(*p1, p0)) *p1 = p0;
     A.dp[((long long)k + (long long)nn * A.kdm) * sl + c] = *p1 - p0;
   }
 }
@@ -488,10 +553,11 @@ __global__ void cn_ra(const CnuityArgs A) {
   const long long c = x.c, sl = A.slice;
   if (!(A.msk[c] & kIP)) return;
   const int mm = A.m - 1, nn = A.n - 1;
+  const double hra = 0.5 * A.ra2fac;
   for (int k = 0; k < A.kdm; k++) {
     const long long om = ((long long)k + (long long)mm * A.kdm) * sl + c, on = ((long long)k + (long long)nn * A.kdm) * sl + c;
     const double dpold = A.dpo[on], dpmid = A.dp[om], dpnew = A.dp[on];
-    const double q = 0.5 * A.ra2fac * (dpold + dpnew - 2.0 * dpmid);
+    const double q = mul_rn(hra, dpold + dpnew - twice_of(dpmid));
     A.dpo[om] = dpmid;
     A.dp[om] = dpmid + q;
   }
@@ -559,7 +625,9 @@ cudaError_t launch_cnuity_rest(const CnuityArgs &a, int *launches, cudaStream_t 
         cn_thk_util<<<grid_for(a, 5), b, 0, s>>>(a, k);
         nl++;
       }
-      cn_thk_flux<<<grid_for(a, 4), b, 0, s>>>(a, k, bih, iflip);
+      if (!bih) cn_thk_flux<false, false><<<grid_for(a, 4), b, 0, s>>>(a, k);
+      else if (iflip) cn_thk_flux<true, true><<<grid_for(a, 4), b, 0, s>>>(a, k);
+      else cn_thk_flux<true, false><<<grid_for(a, 4), b, 0, s>>>(a, k);
       cn_thk_p<<<grid_for(a, 4), b, 0, s>>>(a, k);
       nl += 2;
       if (k == k1) break;
