@@ -9,7 +9,7 @@ namespace hyc {
 constexpr uint8_t kIP = 1, kIU = 2, kIV = 4;  // mask bits: ip, iu, iv
 
 constexpr int kMaxFields = 16;
-// FCT strip kernel (hyc_march.cuh): columns a CTA marches over (6 fewer are
+// strip kernels (hyc_march.cuh): columns a CTA marches over (6 fewer are
 // updated), fields it carries, and so the most groups of fields
 constexpr int kMarchCols = 64, kMarchFields = 2, kMaxMarchGroups = kMaxFields / kMarchFields;
 enum Scheme { kPCM = 0, kMPDATA = 1, kFCT2 = 2, kFCT4 = 4 };

@@ -5,6 +5,7 @@
 #include <climits>
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 
 #include "hyc_ens.h"
 #include "hyc_internal.h"
@@ -58,11 +59,11 @@ static cudaError_t launch_shape(int scheme, const TileArgs &a, int nlayers, cuda
   return cudaErrorInvalidValue;
 }
 
-// FCT2/FCT4 strip kernel.  Rows a CTA: the fewest row steps over the waves of
+// Strip kernels (hyc_march.cuh).  Rows a CTA: the fewest row steps over the waves of
 // CTAs that the chip holds (each CTA takes nrow + 7 steps)
 template <int S, int NT, int NG>
 static cudaError_t launch_march_one(const TileArgs &a, int nlayers, cudaStream_t s) {
-  using G = MarchGeom<NT, NG>;
+  using G = std::conditional_t<S == kFCT2 || S == kFCT4, MarchGeom<NT, NG>, MarchGeom1<NT, NG>>;
   static unsigned long long attr_done = 0;
   auto kern = march_kernel<S, NT, NG>;
   int dev = 0, nsm = 0;
@@ -89,29 +90,42 @@ static cudaError_t launch_march_one(const TileArgs &a, int nlayers, cudaStream_t
   return cudaGetLastError();
 }
 
-// The strip kernel from the size on where its CTAs fill the chip: more 32x16
-// tiles than one wave of the tile kernel (two CTAs an SM), four waves where
-// the launch has one field.  A whole call (FCT2, T and S; tile / strip): 240
-// tiles 65 / 82 us, 351 tiles 88 / 83, 1170 tiles 188 / 150, the 4500x3298x41
-// basin 125 / 78 ms; one field: 551 tiles 71 / 84 us, 1276 tiles 119 / 120,
-// 3243 tiles 245 / 245.  The layer-1 fields of isopycnic mode that need a
-// second pair of fluxes (ufco) stay with the tile kernel.
+// The strip kernel from the size on where its CTAs fill the chip, by the
+// number of 32x16 tiles of all layers: more than two an SM, with one field in
+// the launch four (MPDATA) or eight (FCT); donor cell always.  A whole call,
+// tile / strip, T and S: FCT2 240 tiles 65 / 82 us, 351 tiles 88 / 83, 1170
+// tiles 188 / 150, the 4500x3298x41 basin 125 / 78 ms; MPDATA 240 tiles 107 /
+// 121 us, 351 tiles 140 / 122, 1170 tiles 358 / 231; donor cell 72 tiles 46 /
+// 41, 1170 tiles 163 / 89.  One field: FCT2 551 tiles 71 / 84 us, 1276 tiles
+// 119 / 120, 3243 tiles 245 / 245; MPDATA 551 tiles 114 / 115, 1276 tiles 214
+// / 170; donor cell 117 tiles 39 / 39, 551 tiles 58 / 51.  The layer-1 fields
+// of isopycnic mode that need a second pair of fluxes (ufco) stay with the
+// tile kernel.
 bool march_takes(int scheme, const TileArgs &a, int nlayers) {
-  if ((scheme != kFCT2 && scheme != kFCT4) || a.ufco) return false;
+  if (a.ufco) return false;
   if ((long long)nlayers * ((a.nfld + kMarchFields - 1) / kMarchFields) > 65535) return false;  // grid limit
+  if (scheme == kPCM) return true;
   int dev = 0, nsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const long long tiles = (long long)((a.ii + 31) / 32) * ((a.jj + 15) / 16) * nlayers;
-  return tiles > (a.nfld > 1 ? 1 : 4) * 2LL * nsm;
+  return tiles > (a.nfld > 1 ? 2LL : scheme == kMPDATA ? 4LL : 8LL) * nsm;
+}
+
+template <int S>
+static cudaError_t launch_march_fields(const TileArgs &a, int nlayers, cudaStream_t s) {
+  if (a.nfld == 1) return launch_march_one<S, kMarchCols, 1>(a, nlayers, s);
+  return launch_march_one<S, kMarchCols, kMarchFields>(a, nlayers, s);
 }
 
 cudaError_t launch_march(int scheme, const TileArgs &a, int nlayers, cudaStream_t s) {
-  if (a.nfld == 1)
-    return scheme == kFCT2 ? launch_march_one<kFCT2, kMarchCols, 1>(a, nlayers, s)
-                           : launch_march_one<kFCT4, kMarchCols, 1>(a, nlayers, s);
-  return scheme == kFCT2 ? launch_march_one<kFCT2, kMarchCols, kMarchFields>(a, nlayers, s)
-                         : launch_march_one<kFCT4, kMarchCols, kMarchFields>(a, nlayers, s);
+  switch (scheme) {
+    case kPCM: return launch_march_fields<kPCM>(a, nlayers, s);
+    case kMPDATA: return launch_march_fields<kMPDATA>(a, nlayers, s);
+    case kFCT2: return launch_march_fields<kFCT2>(a, nlayers, s);
+    case kFCT4: return launch_march_fields<kFCT4>(a, nlayers, s);
+  }
+  return cudaErrorInvalidValue;
 }
 
 bool advect_tile_shape_ok(TileShape t) {

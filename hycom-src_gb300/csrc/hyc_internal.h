@@ -23,7 +23,7 @@ size_t advect_tiles_smem(TileShape shape);
 // the tile kernel of this scheme and shape stages its region by TMA when
 // the launch carries tensor maps (box (tx+8) x (ty+6), see TileArgs::tmaps)
 bool advect_tiles_tma(int scheme, TileShape shape);
-// the launch goes to the FCT strip kernel (hyc_march.cuh), which takes no tensor maps
+// the launch goes to a strip kernel (hyc_march.cuh), which takes no tensor maps
 bool march_takes(int scheme, const TileArgs &a, int nlayers);
 bool advect_tile_shape_ok(TileShape shape);
 

@@ -29,6 +29,10 @@
 // The region is staged by TMA (one box per array, one mbarrier, bounded
 // waits) when the launch carries tensor maps and the shape allows it
 // (TileGeom::TMA), else by plain loads.
+//
+// It serves MPDATA launches too small for the strip kernel (hyc_march.cuh)
+// and the isopycnic layer-1 launches with a second pair of fluxes; FCT2 and
+// FCT4 have a tile kernel of their own (hyc_fct.cuh).
 #pragma once
 #include <cuda.h>
 

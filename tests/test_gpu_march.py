@@ -1,4 +1,4 @@
-"""The FCT strip kernel (csrc/hyc_march.cuh) against the oracle, bit for bit,
+"""The strip kernels (csrc/hyc_march.cuh) against the oracle, bit for bit,
 where its geometry ends: strips of 58 columns, short and ragged segments, odd
 counts of fields, and tracers that leave the range of the integer
 multiplication and division or the FP32 limiter test.  The layer counts put
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("nx,ny,kdm,periodic", [(57, 41, 52, False), (58, 33, 56, True), (59, 20, 80, False),
                                                 (117, 18, 40, True), (175, 45, 20, False)])
-@pytest.mark.parametrize("advtyp,ntr", [(2, 0), (2, 1), (4, 3)])
+@pytest.mark.parametrize("advtyp,ntr", [(0, 0), (0, 1), (1, 0), (1, 3), (2, 0), (2, 1), (4, 3)])
 def test_strip_edges(cuda, nx, ny, kdm, periodic, advtyp, ntr):
     b = basin(nx, ny, periodic, seed=nx)
     g = oracle_grid(b)
@@ -29,7 +29,8 @@ def test_strip_edges(cuda, nx, ny, kdm, periodic, advtyp, ntr):
     compare(c, t)
 
 
-def test_fct4_with_oneta(cuda):
+@pytest.mark.parametrize("advtyp", [0, 1, 4])
+def test_with_oneta(cuda, advtyp):
     b = basin(90, 70, True, seed=5)
     g = oracle_grid(b)
     c = np_case(b, g, kdm=24, ntracr=0, seed=5, courant=0.7, delt1=600.0)
@@ -38,13 +39,14 @@ def test_fct4_with_oneta(cuda):
     t = torchify(dict(c, oneta=oneta), cuda)
     ctx = make_ctx(b, g, 24)
     bind_all(ctx, t, extra=("oneta",))
-    oracle_steps(g, c, (1, 2), 4, btrmas=True, oneta=oneta)
-    gpu_steps(ctx, t, (1, 2), 4, btrmas=True)
+    oracle_steps(g, c, (1, 2), advtyp, btrmas=True, oneta=oneta)
+    gpu_steps(ctx, t, (1, 2), advtyp, btrmas=True)
     compare(c, t)
 
 
+@pytest.mark.parametrize("advtyp", [0, 1, 2])
 @pytest.mark.parametrize("scale", [0.0, 1e-306, 1e-40, 1e30, 1e150])
-def test_tracer_ranges(cuda, scale):
+def test_tracer_ranges(cuda, scale, advtyp):
     """Constant, tiny and huge tracers: what the limiter's FP32 test cannot
     decide and what the integer arithmetic hands to the FP64 pipe."""
     b = basin(100, 60, False, seed=9)
@@ -57,12 +59,12 @@ def test_tracer_ranges(cuda, scale):
     ctx = make_ctx(b, g, 26)
     bind_all(ctx, t)
     flg = np.zeros(2, np.int32)
-    oracle_steps(g, c, (1, 2), 2, trcflg=flg)
-    gpu_steps(ctx, t, (1, 2), 2, ntracr=2, trcflg=flg)
+    oracle_steps(g, c, (1, 2), advtyp, trcflg=flg)
+    gpu_steps(ctx, t, (1, 2), advtyp, ntracr=2, trcflg=flg)
     compare(c, t)
 
 
-@pytest.mark.parametrize("advtyp", [2, 4])
+@pytest.mark.parametrize("advtyp", [0, 1, 2, 4])
 def test_one_field_slice(cuda, advtyp):
     """advem on one long slice: the one-field form."""
     b = basin(59, 9800, False, seed=11)
