@@ -168,10 +168,9 @@ int fct2c_batch(const hyc_ctx *c) {
 }
 
 void fct2c_bind(hyc::Fct2cArgs &f, const hyc_ctx *c, int npair) {
-  const size_t sl = (size_t)c->slice;
   f.npair = npair;
   f.work = (double *)c->d_fct2c;
-  f.lcalc = c->d_fct2c + (size_t)npair * sl * 13 * sizeof(double);
+  f.lcalc = c->d_fct2c + (size_t)npair * hyc::fct2c_work_doubles(c->slice) * sizeof(double);
 }
 
 // TMA maps of the FCT tile kernel for the launches of one call (box TX+8 x

@@ -40,6 +40,7 @@ cudaError_t launch_conserve(const TileArgs &a, int nlayers, double *rows, double
 struct Fct2cArgs;
 // advem_fct2c: work bytes per (field, layer) pair; the stages of one call
 size_t fct2c_work_bytes(long long slice);
+size_t fct2c_work_doubles(long long slice);
 cudaError_t launch_fct2c(const Fct2cArgs &a, int nreg, int *launches, cudaStream_t s);
 
 // Lateral diffusion (tsdff_1x/tsdff_2x and the density update); the two
