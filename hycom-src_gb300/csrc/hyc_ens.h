@@ -19,7 +19,6 @@ struct MixBasin {
   long long slice;
   int kdm, ntr;  // ntr: tracers this table's launch advances, from q0 on
   int images;  // periodic-x halo images to write (0 when closed)
-  int seg;     // rows per strip segment
   int kchunk;  // layers per work item
   int q0;      // first tracer of this table's launch
   float *fnew;  // ntr*kdm slices, level t+1
@@ -35,6 +34,9 @@ struct MixBasin {
 // two columns per lane, 64-column strips (56 updated) streamed by TMA
 constexpr int kCol2Strip = 56;
 constexpr int kCol2Box = 64, kCol2Rows = 4;
+// its work item: (basin, strip, first row, rows | layer chunk << kCol2RowBits);
+// segments have at most 2048 rows
+constexpr int kCol2RowBits = 12;
 cudaError_t launch_mix_col2(int scheme, const MixBasin *basins, const int4 *items, int nitems, int *head, int nsm,
                             int nq, bool prep64, bool diff, int *err, cudaStream_t s);
 // grid table of the diffusion epilogue (see MixBasin::c2_gd) from reference-layout FP64

@@ -36,6 +36,12 @@ struct EBasin {
   double temdf2 = 0.0;                          // lateral diffusion after each step (0: none)
   long long work = 0;                           // cells*layers*tracers, for queue ordering
   std::vector<double> posdef;                   // MPDATA offset per tracer (0 unless set)
+  std::vector<uint8_t> sea;                     // strip kernel: [strip][row] has sea among the columns it updates
+};
+
+// rows [j0, j0 + rows) of a strip
+struct Run {
+  int strip, j0, rows;
 };
 
 }  // namespace
@@ -68,6 +74,7 @@ struct hyc_ens {
   int4 *d_items = nullptr;  // the main launch's items, then the one-tracer launch's
   int nitems = 0, nitems_t = 0;
   int items_nq = 0;         // tracers per pass the strip items were built for
+  int kchunk = 1;  // strip kernel: layers per work item
   int items_tx = 0, items_ty = 0, items_layers = -1;
   int *d_head = nullptr;  // two queue counters per step slot (main and one-tracer launch)
   int nhead = 0;
@@ -207,17 +214,44 @@ int encode_strip_maps(hyc_ens *e) {
   return HYC_OK;
 }
 
+// The segments of rows of a basin that the strip kernel works on: each strip's
+// rows from the first to the last with sea among the columns it updates,
+// without gaps of land of more than kLandGap rows (a segment recomputes 6 or
+// 8 rows, and a queue item costs a little), in equal segments of at most seg
+// rows.  Three steps, T and S, against segments that cover every row:
+// 4500x3298x41 (30 % land) 38.3 -> 30.4 ms, 1500x1100x41 (30 % land) 4.64 ->
+// 4.11, 24 closed basins 122.6 -> 119.8 (six steps).  The same test in the
+// kernel, a block of land rows after another skipped, gained as much there but
+// cost the other basins 4-7 %: the kernel has no register to spare.
+constexpr int kLandGap = 24;
+std::vector<Run> strip_runs(const EBasin &b, int seg) {
+  std::vector<Run> out;
+  const int nstrip = (int)(b.sea.size() / b.jdm);
+  for (int st = 0; st < nstrip; st++) {
+    const uint8_t *sea = b.sea.data() + (size_t)st * b.jdm;
+    for (int j = 0; j < b.jdm;) {
+      if (!sea[j]) {
+        j++;
+        continue;
+      }
+      int last = j;
+      for (int r = j + 1; r < b.jdm && r - last <= kLandGap; r++)
+        if (sea[r]) last = r;
+      const int n = last + 1 - j, ns = (n + seg - 1) / seg, len = (n + ns - 1) / ns;
+      for (int r = 0; r < n; r += len) out.push_back({st, 1 + j + r, std::min(len, n - r)});
+      j = last + 1;
+    }
+  }
+  return out;
+}
+
 // Layers per work item of the two-column strip kernel: enough items for
 // about 16 per resident warp over the whole ensemble (so the last wave of
 // the queue is short), and no more than 8 layers per item unless the
 // ensemble is small.
-int col2_kchunk(const hyc_ens *e, const EBasin &) {
+int col2_kchunk(const hyc_ens *e) {
   long long cols = 0;  // (strip, segment, layer) units over the ensemble
-  for (const auto &b : e->b) {
-    const long long nstrip = (b.nbdy + b.idm - 4 + hyc::kCol2Strip - 1) / hyc::kCol2Strip;
-    const long long nseg = (b.jdm + e->shape.ty - 1) / e->shape.ty;
-    cols += nstrip * nseg * b.kdm;
-  }
+  for (const auto &b : e->b) cols += (long long)strip_runs(b, e->shape.ty).size() * b.kdm;
   const long long want = 16LL * e->nsm * 8;  // ~16 items per warp at 8 warps per SM
   long long kc = cols / std::max(want, 1LL);
   return (int)std::max(1LL, std::min(8LL, kc));
@@ -261,8 +295,7 @@ int build_tables(hyc_ens *e, double dt2) {
         m.ntr = b.ntr;
         m.images = b.nreg == 1 ? std::min(5, b.nbdy) : 0;
         m.fnew = (float *)b.lev[ln];
-        m.seg = e->shape.ty;
-        m.kchunk = col2_kchunk(e, b);
+        m.kchunk = e->kchunk;
         m.q0 = 0;
         if (e->items_nq == 2 && b.ntr > 1) m.ntr = b.ntr & ~1;  // pairs; an odd last tracer is the other launch's
         for (int q = 0; q < b.ntr && q < hyc::kMaxFields; q++) m.posdef[q] = (float)b.posdef[q];
@@ -387,6 +420,7 @@ int build_items(hyc_ens *e) {
     int4 it;
   };
   std::vector<W> w, wt;  // main launch, one-tracer launch
+  if (is_col2(e->shape)) e->kchunk = col2_kchunk(e);
   for (int i = 0; i < (int)e->b.size(); i++) {
     const EBasin &b = e->b[i];
     if (is_col2(e->shape)) {  // (basin, 56-column strip, segment, chunk of layers), all tracers
@@ -395,18 +429,16 @@ int build_items(hyc_ens *e) {
       // and from L2 by the other chunks
       // with pairs of tracers per pass, an odd count's last tracer goes to the
       // one-tracer launch instead of a pass that advances it twice
-      const int nstrip = (b.nbdy + b.idm - 4 + hyc::kCol2Strip - 1) / hyc::kCol2Strip;
-      const int nty = (b.jdm + e->shape.ty - 1) / e->shape.ty;
-      const int kc = col2_kchunk(e, b), nkc = (b.kdm + kc - 1) / kc;
+      const int kc = e->kchunk, nkc = (b.kdm + kc - 1) / kc;
       const int trm = nqm == 2 ? (b.ntr & ~1) : b.ntr;
       const bool tail = nqm == 2 && (b.ntr & 1);
-      for (int sg = 0; sg < nty; sg++)
-        for (int kq = 0; kq < nkc; kq++)
-          for (int st = 0; st < nstrip; st++) {
-            const long long lay = std::min(b.kdm, (kq + 1) * kc) - kq * kc;
-            if (trm > 0) w.push_back({lay * trm, make_int4(i, st, sg, kq)});
-            if (tail) wt.push_back({lay, make_int4(i, st, sg, kq)});
-          }
+      for (const Run &r : strip_runs(b, e->shape.ty))
+        for (int kq = 0; kq < nkc; kq++) {
+          const long long lay = std::min(b.kdm, (kq + 1) * kc) - kq * kc, rows = r.rows + 6;
+          const int4 item = make_int4(i, r.strip, r.j0, r.rows | kq << hyc::kCol2RowBits);
+          if (trm > 0) w.push_back({lay * rows * trm, item});
+          if (tail) wt.push_back({lay * rows, item});
+        }
       continue;
     }
     // FP64 form: (basin, strip, segment, layer, group of fields)
@@ -580,6 +612,19 @@ int hyc_ens_create(hyc_ens **out, int32_t nbasin, const hyc_basin_spec *specs, i
     e->b.push_back(b);
     if (!ok) return bail(efail(nullptr, HYC_ERR_NOMEM, "basin %d: device allocation failed", i));
     EBasin &bb = e->b.back();
+    if (precision == HYC_PREC_MIXED) {
+      const int nstrip = (bb.nbdy + bb.idm - 4 + hyc::kCol2Strip - 1) / hyc::kCol2Strip;
+      bb.sea.assign((size_t)nstrip * bb.jdm, 0);
+      for (int j = 0; j < bb.jdm; j++) {
+        const uint8_t *row = m.data() + (long long)(j + bb.nbdy) * bb.ld1;
+        for (int st = 0; st < nstrip; st++) {
+          const int c0 = std::max(bb.nbdy, st * hyc::kCol2Strip + 4), c1 = std::min(bb.nbdy + bb.idm, st * hyc::kCol2Strip + 60);
+          uint8_t any = 0;
+          for (int c = c0; c < c1; c++) any |= row[c];
+          bb.sea[(size_t)st * bb.jdm + j] = any & hyc::kIP;
+        }
+      }
+    }
     bool cp = cudaMemcpy(bb.msk, m.data(), bb.slice, cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(bb.scp2, sc.data(), bb.slice * 8, cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(bb.scp2i, si.data(), bb.slice * 8, cudaMemcpyHostToDevice) == cudaSuccess &&

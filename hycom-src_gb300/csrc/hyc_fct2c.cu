@@ -19,7 +19,8 @@
 // and a face between two such cells no flux.  16 pairs of 900x700: 3.9 -> 1.8
 // ms, of it start 0.20, the first iteration 0.41, the four others 0.17 each,
 // fluxes, ratios and update 0.67.
-//  The stages keep
+//
+// The stages keep
 // the reference's margins and operation order and are built without FMA
 // contraction, so results equal the oracle's bit for bit.
 #include <cuda_runtime.h>

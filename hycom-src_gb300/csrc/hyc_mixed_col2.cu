@@ -2,7 +2,7 @@
 // 64-column strip north through the rows, two columns per lane, with the
 // rows streamed into a per-warp shared-memory ring by TMA.
 //
-// Work item: (basin, strip, segment of rows, chunk of layers), all the
+// Work item: (basin, strip, segment of rows with sea, chunk of layers), all the
 // launch's tracers of the basin (its table entry's q0 .. q0+ntr-1).  The
 // strip starts at padded column s = 56*w (a multiple of 4, so every TMA box
 // starts on a 16-byte boundary), lane l owns columns s+2l and s+2l+1, and
@@ -255,15 +255,15 @@ __global__ void __launch_bounds__(kWarps * 32, NQ == 1 ? 3 : 2)
     if (it >= nitems) break;
     const int4 w = items[it];
     const MixBasin &B = basins[w.x];
-    const int ii = B.ii, jj = B.jj, nb = B.nbdy, ld1 = B.ld1, kdm = B.kdm, images = B.images;
+    const int ii = B.ii, nb = B.nbdy, ld1 = B.ld1, kdm = B.kdm, images = B.images;
     const int q0 = B.q0, ntr = B.ntr;  // this launch's tracers: q0 .. q0+ntr-1
     float *const fnew = B.fnew;
     const long long sl = B.slice;
     const int s0 = 56 * w.y;  // strip start (padded column)
-    const int j0 = 1 + w.z * B.seg, j1 = min(j0 + B.seg, jj + 1);
+    const int j0 = w.z, j1 = j0 + (w.w & ((1 << kCol2RowBits) - 1));
     const int nblk = (j1 - j0 + 2 * kLead + kRB - 1) / kRB;
     const int nqp = (ntr + NQ - 1) / NQ;
-    const int ka = w.w * B.kchunk, kb = min(kdm, ka + B.kchunk);  // this item's layers
+    const int ka = (w.w >> kCol2RowBits) * B.kchunk, kb = min(kdm, ka + B.kchunk);  // this item's layers
     const int T = (kb - ka) * nqp * nblk;
     // this lane's columns: padded a0 = s0 + 2*lane (A) and a0 + 1 (B)
     const int a0 = s0 + 2 * lane;
