@@ -31,6 +31,7 @@
 #include "hyc_args.h"
 #include "hyc_device.cuh"
 #include "hyc_internal.h"
+#include "hyc_pdl.cuh"
 
 namespace hyc {
 
@@ -76,6 +77,7 @@ __device__ __forceinline__ bool finite(double x) { return (__double2hiint(x) & 0
 
 // :112-157 at margin 6
 __global__ void cn_init(const CnuityArgs A) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 6, x)) return;
   const long long c = x.c, sl = A.slice;
@@ -117,6 +119,7 @@ __global__ void cn_init(const CnuityArgs A) {
 // are skipped; the FP64 pipe bounds this kernel.
 template <bool BT>
 __global__ void cn_flux(const CnuityArgs A, int k) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 5, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
@@ -166,6 +169,7 @@ __device__ __forceinline__ void row_min(const CnuityArgs &A, const Cell &x, bool
 // loop 19, :294-315 at margin 4: low-order update of dp(k,n) (BT as cn_flux)
 template <bool BT>
 __global__ void cn_low(const CnuityArgs A, int k) {
+  after_previous();
   Cell x;
   const bool in = cell_of(A, 4, x);
   bool sea = false;
@@ -187,6 +191,7 @@ __global__ void cn_low(const CnuityArgs A, int k) {
 
 // :400-430 at margin 4: the limiter's ratios
 __global__ void cn_ratio(const CnuityArgs A, int k) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 4, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
@@ -236,6 +241,7 @@ __device__ __forceinline__ double clipped(double f2, double clip, double *rest) 
 
 // :442-472 at margin 3: clip the antidiffusive fluxes
 __global__ void cn_clip(const CnuityArgs A, int k) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 3, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
@@ -264,6 +270,7 @@ __global__ void cn_clip(const CnuityArgs A, int k) {
 // loop 15 (:480-498, margin 2) and loop 14 (:650-665, margin 0): flux update
 // of dp(k,n) and p(k+1)
 __global__ void cn_update(const CnuityArgs A, int k, int M, int slot) {
+  after_previous();
   Cell x;
   const bool in = cell_of(A, M, x);
   bool sea = false;
@@ -286,6 +293,7 @@ __global__ void cn_update(const CnuityArgs A, int k, int M, int slot) {
 // not change during loop 77 before its last layer's fluxes are formed, so one
 // reciprocal per cell serves every layer's division dp/p(kk+1).
 __global__ void cn_rpb(const CnuityArgs A) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 2, x)) return;
   const long long c = x.c;
@@ -297,6 +305,7 @@ __global__ void cn_rpb(const CnuityArgs A) {
 // q = dp/p(kk+1) by div_by with the cell's reciprocal.  A face that clipped
 // nothing (most) has no correction flux: uf = 0*q = 0 for its finite q.
 __global__ void cn_btflux(const CnuityArgs A, int k) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 1, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
@@ -329,6 +338,7 @@ __global__ void cn_btflux(const CnuityArgs A, int k) {
 
 // :709-735 at margin 0: bottom-pressure restoring (not btrmas)
 __global__ void cn_bottom(const CnuityArgs A) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 0, x)) return;
   const long long c = x.c, sl = A.slice;
@@ -344,6 +354,7 @@ __global__ void cn_bottom(const CnuityArgs A) {
 
 // :770-785 / :993-1010 at margin 6: start of the interface diffusion
 __global__ void cn_thk_init(const CnuityArgs A, int bih, int iflip) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 6, x)) return;
   const long long c = x.c;
@@ -366,6 +377,7 @@ __device__ __forceinline__ long long nbx(const CnuityArgs &A, long long c, long 
 
 // loop 13, :790-830 at margin 5: biharmonic smoothing operands at interface k (1-based)
 __global__ void cn_thk_util(const CnuityArgs A, int k) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 5, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
@@ -408,6 +420,7 @@ constexpr int kTX = 32, kTY = 8;  // the block of every cnuity launch
 // BIH, IFLIP: compile-time, so that no branch of the other form is predicated in.
 template <bool BIH, bool IFLIP>
 __global__ void __launch_bounds__(kTX * kTY, 6) cn_thk_flux(const CnuityArgs A, int k) {
+  after_previous();
   __shared__ double sG[kTY + 1][kTX + 1], sH[kTY + 1][kTX + 1];
   Cell x;
   const bool in = cell_of(A, 4, x);
@@ -480,6 +493,7 @@ __global__ void __launch_bounds__(kTX * kTY, 6) cn_thk_flux(const CnuityArgs A, 
 
 // :905-920 at margin 4: move interface k (1-based)
 __global__ void cn_thk_p(const CnuityArgs A, int k) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 4, x)) return;
   const long long c = x.c, ld = A.ld1;
@@ -492,6 +506,7 @@ __global__ void cn_thk_p(const CnuityArgs A, int k) {
 
 // :925-950 at margin 4: interfaces kept ordered, dp(n) from p
 __global__ void cn_thk_final(const CnuityArgs A) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 4, x)) return;
   const long long c = x.c, sl = A.slice;
@@ -507,6 +522,7 @@ __global__ void cn_thk_final(const CnuityArgs A) {
 
 // :1326-1348 at margin 0: cumulative fluxes
 __global__ void cn_cumul(const CnuityArgs A) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 0, x)) return;
   const long long c = x.c, sl = A.slice;
@@ -522,6 +538,7 @@ __global__ void cn_cumul(const CnuityArgs A) {
 
 // :1350-1385 at margin 1: btrmas restoring (dp back to dp')
 __global__ void cn_btrmas(const CnuityArgs A) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 1, x)) return;
   const long long c = x.c, sl = A.slice;
@@ -548,6 +565,7 @@ __global__ void cn_btrmas(const CnuityArgs A) {
 
 // :1387-1410 at margin 6: Robert-Asselin filter of dp
 __global__ void cn_ra(const CnuityArgs A) {
+  after_previous();
   Cell x;
   if (!cell_of(A, 6, x)) return;
   const long long c = x.c, sl = A.slice;
@@ -574,19 +592,19 @@ size_t cnuity_work_slices() { return W_N; }
 cudaError_t launch_cnuity_layers(const CnuityArgs &a, int *launches, cudaStream_t s) {
   const dim3 b(kTX, kTY);
   int nl = 0;
-  cn_init<<<grid_for(a, 6), b, 0, s>>>(a);
+  launch_after(cn_init, grid_for(a, 6), b, s, a);
   nl++;
   for (int k = 0; k < a.kdm; k++) {  // loop 76
     if (a.btrmas) {
-      cn_flux<true><<<grid_for(a, 5), b, 0, s>>>(a, k);
-      cn_low<true><<<grid_for(a, 4), b, 0, s>>>(a, k);
+      launch_after(cn_flux<true>, grid_for(a, 5), b, s, a, k);
+      launch_after(cn_low<true>, grid_for(a, 4), b, s, a, k);
     } else {
-      cn_flux<false><<<grid_for(a, 5), b, 0, s>>>(a, k);
-      cn_low<false><<<grid_for(a, 4), b, 0, s>>>(a, k);
+      launch_after(cn_flux<false>, grid_for(a, 5), b, s, a, k);
+      launch_after(cn_low<false>, grid_for(a, 4), b, s, a, k);
     }
-    cn_ratio<<<grid_for(a, 4), b, 0, s>>>(a, k);
-    cn_clip<<<grid_for(a, 3), b, 0, s>>>(a, k);
-    cn_update<<<grid_for(a, 2), b, 0, s>>>(a, k, 2, a.kdm + k);
+    launch_after(cn_ratio, grid_for(a, 4), b, s, a, k);
+    launch_after(cn_clip, grid_for(a, 3), b, s, a, k);
+    launch_after(cn_update, grid_for(a, 2), b, s, a, k, 2, a.kdm + k);
     nl += 5;
   }
   *launches += nl;
@@ -597,14 +615,14 @@ cudaError_t launch_cnuity_rest(const CnuityArgs &a, int *launches, cudaStream_t 
   const dim3 b(kTX, kTY);
   int nl = 0;
   if (!a.btrmas) {
-    cn_rpb<<<grid_for(a, 2), b, 0, s>>>(a);
+    launch_after(cn_rpb, grid_for(a, 2), b, s, a);
     nl++;
     for (int k = 0; k < a.kdm; k++) {  // loop 77
-      cn_btflux<<<grid_for(a, 1), b, 0, s>>>(a, k);
-      cn_update<<<grid_for(a, 0), b, 0, s>>>(a, k, 0, -1);
+      launch_after(cn_btflux, grid_for(a, 1), b, s, a, k);
+      launch_after(cn_update, grid_for(a, 0), b, s, a, k, 0, -1);
       nl += 2;
     }
-    cn_bottom<<<grid_for(a, 0), b, 0, s>>>(a);
+    launch_after(cn_bottom, grid_for(a, 0), b, s, a);
     nl++;
   }
   cudaError_t e = cudaGetLastError();
@@ -617,30 +635,30 @@ cudaError_t launch_cnuity_rest(const CnuityArgs &a, int *launches, cudaStream_t 
     if (e == cudaSuccess) e = launch_xctilr(a.p + a.slice, a.slice, a.kdm, a.ii, a.jj, nb, a.ld1, 6, 6, a.nreg, s);
     if (e != cudaSuccess) return e;
     nl += 2;
-    cn_thk_init<<<grid_for(a, 6), b, 0, s>>>(a, bih, iflip);
+    launch_after(cn_thk_init, grid_for(a, 6), b, s, a, bih, iflip);
     nl++;
     const int k0 = bih ? (iflip ? a.kdm : 2) : 2, k1 = bih ? (iflip ? 2 : a.kdm) : a.kdm, dk = k1 >= k0 ? 1 : -1;
     for (int k = k0;; k += dk) {
       if (bih) {
-        cn_thk_util<<<grid_for(a, 5), b, 0, s>>>(a, k);
+        launch_after(cn_thk_util, grid_for(a, 5), b, s, a, k);
         nl++;
       }
-      if (!bih) cn_thk_flux<false, false><<<grid_for(a, 4), b, 0, s>>>(a, k);
-      else if (iflip) cn_thk_flux<true, true><<<grid_for(a, 4), b, 0, s>>>(a, k);
-      else cn_thk_flux<true, false><<<grid_for(a, 4), b, 0, s>>>(a, k);
-      cn_thk_p<<<grid_for(a, 4), b, 0, s>>>(a, k);
+      if (!bih) launch_after(cn_thk_flux<false, false>, grid_for(a, 4), b, s, a, k);
+      else if (iflip) launch_after(cn_thk_flux<true, true>, grid_for(a, 4), b, s, a, k);
+      else launch_after(cn_thk_flux<true, false>, grid_for(a, 4), b, s, a, k);
+      launch_after(cn_thk_p, grid_for(a, 4), b, s, a, k);
       nl += 2;
       if (k == k1) break;
     }
-    cn_thk_final<<<grid_for(a, 4), b, 0, s>>>(a);
+    launch_after(cn_thk_final, grid_for(a, 4), b, s, a);
     nl++;
   }
   if (a.uflxav && a.vflxav && a.dpav) {
-    cn_cumul<<<grid_for(a, 0), b, 0, s>>>(a);
+    launch_after(cn_cumul, grid_for(a, 0), b, s, a);
     nl++;
   }
   if (a.btrmas) {
-    cn_btrmas<<<grid_for(a, 1), b, 0, s>>>(a);
+    launch_after(cn_btrmas, grid_for(a, 1), b, s, a);
     nl++;
   }
   e = cudaGetLastError();
@@ -648,7 +666,7 @@ cudaError_t launch_cnuity_rest(const CnuityArgs &a, int *launches, cudaStream_t 
   e = launch_xctilr(a.dp + (long long)(a.n - 1) * a.kdm * a.slice, a.slice, a.kdm, a.ii, a.jj, a.nb, a.ld1, 6, 6,
                     a.nreg, s);
   if (e != cudaSuccess) return e;
-  cn_ra<<<grid_for(a, 6), b, 0, s>>>(a);
+  launch_after(cn_ra, grid_for(a, 6), b, s, a);
   nl += 2;
   *launches += nl;
   return cudaGetLastError();

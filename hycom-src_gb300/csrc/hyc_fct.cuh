@@ -24,6 +24,7 @@
 
 #include "hyc_args.h"
 #include "hyc_device.cuh"
+#include "hyc_pdl.cuh"
 #include "hyc_tma.cuh"
 
 namespace hyc {
@@ -389,6 +390,7 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
 
 template <int SCHEME, int TX, int TY>
 __global__ void __launch_bounds__(256, 2) fct_tile_kernel(const TileArgs A) {
+  after_previous();
   extern __shared__ __align__(16) double sm[];
   __shared__ uint64_t bar;
   if (threadIdx.x == 0) {

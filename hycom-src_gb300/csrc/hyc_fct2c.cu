@@ -30,6 +30,7 @@
 #include "hyc_args.h"
 #include "hyc_device.cuh"
 #include "hyc_internal.h"
+#include "hyc_pdl.cuh"
 
 namespace hyc {
 
@@ -100,6 +101,7 @@ __device__ __forceinline__ double local_dt(const Fct2cArgs &A, const double *u, 
 // :1804-1810) and fldlo, and the first local time step.  The other work
 // arrays (:1068-1081) need no initial values: the first iteration writes them.
 __global__ void __launch_bounds__(kBX * kBY) fct2c_start(Fct2cArgs A) {
+  after_previous();
   const int p = blockIdx.y, nb = A.nb;
   long long t;
   int a, b;
@@ -129,6 +131,7 @@ __global__ void __launch_bounds__(kBX * kBY) fct2c_start(Fct2cArgs A) {
 // used up dt2 (lcalc = 0, most cells after the first iteration) gives its
 // faces nothing more.
 __global__ void __launch_bounds__(kBX * kBY) fct2c_dt(Fct2cArgs A) {
+  after_previous();
   const int p = blockIdx.y;
   const uint8_t *lc = A.lcalc + (long long)p * A.slice;
   const double *u = U_(A, p), *v = V_(A, p), *h = W(A, A_HLOC, p);
@@ -165,6 +168,7 @@ __device__ __forceinline__ void face(const Fct2cArgs &A, bool open, long long c,
 // Partial-step donor fluxes and their sums.  A face between two cells with
 // lcalc = 0 is not read any more.
 __global__ void __launch_bounds__(kBX * kBY) fct2c_flux_first(Fct2cArgs A) {
+  after_previous();
   const int p = blockIdx.y;
   long long c;
   if (!cell_of(A, kMb - 1, c)) return;
@@ -174,6 +178,7 @@ __global__ void __launch_bounds__(kBX * kBY) fct2c_flux_first(Fct2cArgs A) {
   face<true>(A, m & kIV, c, c - A.ld1, V_(A, p), dt, lo, W(A, A_VCUM, p), W(A, A_VLOC, p), W(A, A_FLY, p), W(A, A_FYC, p));
 }
 __global__ void __launch_bounds__(kBX * kBY) fct2c_flux(Fct2cArgs A) {
+  after_previous();
   const int p = blockIdx.y, ld = A.ld1;
   const uint8_t *lc = A.lcalc + (long long)p * A.slice;
   const double *u = U_(A, p), *v = V_(A, p), *dt = W(A, A_DTLOC, p), *lo = W(A, A_FLDLO, p);
@@ -204,11 +209,13 @@ __device__ __forceinline__ void low_order(const Fct2cArgs &A, int p, long long c
   lc[c] = more;
 }
 __global__ void __launch_bounds__(kBX * kBY) fct2c_cell_first(Fct2cArgs A) {
+  after_previous();
   const int p = blockIdx.y;
   long long c;
   if (cell_of(A, kMb - 2, c) && (A.msk[c] & kIP)) low_order(A, p, c, A.lcalc + (long long)p * A.slice);
 }
 __global__ void __launch_bounds__(kBX * kBY) fct2c_cell(Fct2cArgs A) {
+  after_previous();
   const int p = blockIdx.y;
   uint8_t *lc = A.lcalc + (long long)p * A.slice;
   active_cells(A, kMb - 2, [&](long long c) { return (A.msk[c] & kIP) && lc[c]; },
@@ -219,6 +226,7 @@ __global__ void __launch_bounds__(kBX * kBY) fct2c_cell(Fct2cArgs A) {
 // cells carry none (the section-edge zeroing :1223-1243 covers every such
 // face a sea cell reads)
 __global__ void __launch_bounds__(kBX * kBY) fct2c_anti(Fct2cArgs A) {
+  after_previous();
   const int p = blockIdx.y;
   long long c;
   if (!cell_of(A, kMb - 2, c)) return;
@@ -236,6 +244,7 @@ __global__ void __launch_bounds__(kBX * kBY) fct2c_anti(Fct2cArgs A) {
 // Zalesak ratios (:1257-1303), true i+1/j+1 neighbours.  FP32 bounds (below
 // qp, above famax, and famax surely above kEps) show most to be 1.
 __global__ void __launch_bounds__(kBX * kBY) fct2c_ratio(Fct2cArgs A) {
+  after_previous();
   const int p = blockIdx.y;
   long long c;
   if (!cell_of(A, kMb - 3, c) || !(A.msk[c] & kIP)) return;
@@ -274,6 +283,7 @@ __global__ void __launch_bounds__(kBX * kBY) fct2c_ratio(Fct2cArgs A) {
 // by both its cells: that is a product where the factor is not 1, against a
 // pass that writes and reads both flux arrays.
 __global__ void __launch_bounds__(kBX * kBY) fct2c_update(Fct2cArgs A) {
+  after_previous();
   const int p = blockIdx.y;
   long long c;
   if (!cell_of(A, 0, c)) return;
@@ -307,8 +317,7 @@ cudaError_t go(K kern, const Fct2cArgs &A, int margin, cudaStream_t s, int rows 
   const unsigned nbx = (unsigned)(A.ii + 2 * margin + kBX - 1) / kBX,
                  nby = (unsigned)(A.jj + 2 * margin + kBY * rows - 1) / (kBY * rows);
   const dim3 grid(nbx * nby, A.npair);
-  kern<<<grid, dim3(kBX, kBY), 0, s>>>(A);
-  return cudaGetLastError();
+  return launch_after(kern, grid, dim3(kBX, kBY), s, A);
 }
 
 }  // namespace

@@ -11,6 +11,7 @@
 #include "hyc_internal.h"
 #include "hyc_fct.cuh"
 #include "hyc_march.cuh"
+#include "hyc_pdl.cuh"
 #include "hyc_tile.cuh"
 
 namespace hyc {
@@ -32,8 +33,7 @@ static cudaError_t launch_kernel(K kern, size_t smem, const TileArgs &a, int nla
     if (dev < 64) attr_done |= 1ULL << dev;
   }
   dim3 grid((unsigned)(a.ntx * a.nty), (unsigned)nlayers);
-  kern<<<grid, 256, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_after_smem(kern, grid, dim3(256), smem, s, a);
 }
 
 template <int S, int TX, int TY>
@@ -86,8 +86,7 @@ static cudaError_t launch_march_one(const TileArgs &a, int nlayers, cudaStream_t
     if (cost < best) best = cost, nrow = r;
   }
   dim3 grid((unsigned)strips, (unsigned)((a.jj + nrow - 1) / nrow), (unsigned)(nlayers * ((a.nfld + NG - 1) / NG)));
-  kern<<<grid, NT * NG, G::smem_bytes, s>>>(a, nrow);
-  return cudaGetLastError();
+  return launch_after_smem(kern, grid, dim3(NT * NG), G::smem_bytes, s, a, nrow);
 }
 
 // The strip kernel from the size on where its CTAs fill the chip, by the
@@ -148,6 +147,27 @@ size_t advect_tiles_smem(TileShape t) {
   return 0;
 }
 
+// The shape of a launch that goes to a tile kernel, and whether its region is
+// staged by TMA, where the caller fixed no shape.  Up to one 32x16 tile an SM
+// a launch is all latency: 16x16 tiles halve a CTA's passes, and plain loads
+// save encoding and copying the tensor maps (advem, a 257x193 slice, FCT2: 51
+// -> 45 us; tsadvc 61x45x10 52 -> 42 us).  MPDATA's kernel, which fits one 32x16
+// CTA an SM, keeps the small tiles up to where its strip kernel takes over
+// (551 tiles: 116 -> 111 us).
+TilePlan tile_plan(int scheme, const TileArgs &a, int nlayers, TileShape shape, bool fixed) {
+  if (march_takes(scheme, a, nlayers)) return {shape, false};
+  bool tma = true;
+  if (!fixed) {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const long long tiles = (long long)((a.ii + 31) / 32) * ((a.jj + 15) / 16) * nlayers;
+    if (tiles <= (scheme == kMPDATA ? 4LL : 1LL) * nsm) shape = TileShape{16, 16};
+    tma = tiles > nsm;
+  }
+  return {shape, tma && advect_tiles_tma(scheme, shape)};
+}
+
 cudaError_t launch_advect_tiles(int scheme, const TileArgs &a, int nlayers, TileShape t, cudaStream_t s) {
   if (march_takes(scheme, a, nlayers)) return launch_march(scheme, a, nlayers, s);
   if (t.tx == 32 && t.ty == 16) return launch_shape<32, 16>(scheme, a, nlayers, s);
@@ -187,6 +207,7 @@ cudaError_t launch_march_queue(int scheme, const TileArgs *basins, const int4 *i
 // grid: (blocks over interior, nlayers, nfld)
 // ---------------------------------------------------------------------------
 __global__ void copy_back_kernel(const TileArgs A) {
+  after_previous();
   const int k = blockIdx.y, fi = blockIdx.z;
   const FieldDesc fd = A.f[fi];
   if (k + 1 > fd.kmax || k + 1 < fd.kmin) return;
@@ -292,8 +313,7 @@ cudaError_t launch_copy_back(const TileArgs &a, int nlayers, cudaStream_t s) {
   int bx = (int)((n + 255) / 256);
   if (bx > 1216) bx = 1216;
   dim3 grid(bx, nlayers, a.nfld);
-  copy_back_kernel<<<grid, 256, 0, s>>>(a);
-  return cudaGetLastError();
+  return launch_after(copy_back_kernel, grid, dim3(256), s, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -344,6 +364,7 @@ cudaError_t launch_iso_smooth(const double *uk, const double *vk, const uint8_t 
 // ---------------------------------------------------------------------------
 __global__ void xctilr_kernel(double *a, long long slice, int ii, int jj, int nb, int ld1, int mhl, int nhl,
                               int nreg) {
+  after_previous();
   double *s = a + (long long)blockIdx.y * slice;
   const bool closed_y = nreg <= 2, closed_x = (nreg == 0 || nreg == 4);
   const long long W = (long long)ii + 2 * mhl;
@@ -390,7 +411,9 @@ cudaError_t launch_xctilr(double *a, long long slice, int nlev, int ii, int jj, 
   if (bx > 512) bx = 512;
   for (int l0 = 0; l0 < nlev; l0 += 65535) {
     int nl = nlev - l0 < 65535 ? nlev - l0 : 65535;
-    xctilr_kernel<<<dim3(bx, nl), 256, 0, s>>>(a + (long long)l0 * slice, slice, ii, jj, nbdy, ld1, mhl, nhl, nreg);
+    const cudaError_t e = launch_after(xctilr_kernel, dim3(bx, nl), dim3(256), s, a + (long long)l0 * slice, slice, ii, jj,
+                                       nbdy, ld1, mhl, nhl, nreg);
+    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }

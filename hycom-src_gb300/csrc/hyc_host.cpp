@@ -83,6 +83,7 @@ struct hyc_ctx {
   double *d_sum = nullptr;      // mass-sum partials + result
   double *h_sum = nullptr;      // pinned
   hyc::TileShape shape{32, 16};
+  bool shape_fixed = false;  // by HYC_TILE
   std::string err;
   // timers (HYC_T_*) and launch accounting
   bool timing = false;
@@ -139,12 +140,20 @@ const int kMbdy[5] = {2, 5, 5, 0, 5};  // mbdy_advtyp, mod_tsadvc.F90:24-29
 
 bool valid_advtyp(int a) { return a == 0 || a == 1 || a == 2 || a == 4; }
 
-hyc::TileShape env_shape(hyc::TileShape def) {
+// the tile shape HYC_TILE asks for, if it does
+bool env_shape(hyc::TileShape &shape) {
   const char *s = getenv("HYC_TILE");
-  if (!s) return def;
   hyc::TileShape t{0, 0};
-  if (sscanf(s, "%dx%d", &t.tx, &t.ty) == 2 && hyc::advect_tile_shape_ok(t)) return t;
-  return def;
+  if (!s || sscanf(s, "%dx%d", &t.tx, &t.ty) != 2 || !hyc::advect_tile_shape_ok(t)) return false;
+  shape = t;
+  return true;
+}
+// the launch's tile shape into its arguments
+hyc::TilePlan plan_tiles(int scheme, hyc::TileArgs &a, int nlayers, hyc::TileShape shape, bool fixed) {
+  const hyc::TilePlan p = hyc::tile_plan(scheme, a, nlayers, shape, fixed);
+  a.ntx = (a.ii + p.shape.tx - 1) / p.shape.tx;
+  a.nty = (a.jj + p.shape.ty - 1) / p.shape.ty;
+  return p;
 }
 
 int ensure_fct2c(hyc_ctx *c, size_t bytes) {
@@ -183,9 +192,9 @@ struct TileMaps {
 };
 
 // append the maps of launch a; returns its first index, or -1 (plain loads)
-long tile_maps_add(const hyc_ctx *c, const hyc::TileArgs &a, int kk, bool flux1, TileMaps &tmv) {
+long tile_maps_add(const hyc_ctx *c, const hyc::TileArgs &a, hyc::TileShape t, int kk, bool flux1, TileMaps &tmv) {
   if (!tmv.use || !hyc::tmap_available()) return -1;
-  const int bx = c->shape.tx + 8, by = c->shape.ty + 6;
+  const int bx = t.tx + 8, by = t.ty + 6;
   const long long w = c->idm + 2LL * c->nbdy, h = c->jdm + 2LL * c->nbdy, ld = c->ld1, sl = c->slice;
   std::vector<CUtensorMap> m(6 + 2 * (size_t)a.nfld);
   bool ok = true;
@@ -454,7 +463,7 @@ int hyc_adv_init(hyc_ctx **out, int32_t idm, int32_t jdm, int32_t kdm, int32_t n
   c->ld2 = jdm + 2 * nbdy;
   c->slice = (long long)c->ld1 * c->ld2;
   c->device = device;
-  c->shape = env_shape(c->shape);
+  c->shape_fixed = env_shape(c->shape);
   // masks: iu/iv must be the bigrid ones (iu = ip(i-1)*ip(i), iv = ip(j-1)*ip(j))
   const int nb = nbdy, ii = idm, jj = jdm;
   std::vector<uint8_t> m((size_t)c->slice, 0);
@@ -705,8 +714,6 @@ int hyc_advem(hyc_ctx *c, int32_t advtyp, double *fld, const double *fldc, const
   a.ld1 = c->ld1;
   a.ld2 = c->ld2;
   a.slice = sl;
-  a.ntx = (c->idm + c->shape.tx - 1) / c->shape.tx;
-  a.nty = (c->jdm + c->shape.ty - 1) / c->shape.ty;
   a.mode = 1;
   a.msk = c->d_msk;
   a.scal = dscal;
@@ -727,9 +734,10 @@ int hyc_advem(hyc_ctx *c, int32_t advtyp, double *fld, const double *fldc, const
   a.out = c->d_scratch;
   a.kdm = 1;
   a.err = c->d_err;
-  if (hyc::advect_tiles_tma(advtyp, c->shape) && !hyc::march_takes(advtyp, a, 1)) {  // the tile kernel stages by TMA
+  const hyc::TilePlan tp = plan_tiles(advtyp, a, 1, c->shape, c->shape_fixed);
+  if (tp.tma) {  // the tile kernel stages by TMA
     TileMaps tmv;
-    const long m0 = tile_maps_add(c, a, 1, true, tmv);
+    const long m0 = tile_maps_add(c, a, tp.shape, 1, true, tmv);
     if (m0 >= 0) {
       if ((rc = tile_maps_upload(c, tmv))) return rc;
       a.tmaps = c->d_tmaps + m0;
@@ -738,7 +746,7 @@ int hyc_advem(hyc_ctx *c, int32_t advtyp, double *fld, const double *fldc, const
   }
   {
     Timed t(c, HYC_T_ADVECT);
-    CK(hyc::launch_advect_tiles(advtyp, a, 1, c->shape, c->stream), "advem kernel");
+    CK(hyc::launch_advect_tiles(advtyp, a, 1, tp.shape, c->stream), "advem kernel");
   }
   if (c->lconserve && (rc = conserve(c, a, 1))) return rc;
   CK(hyc::launch_copy_back(a, 1, c->stream), "advem copy");
@@ -872,8 +880,6 @@ int hyc_tsadvc(hyc_ctx *c, int32_t m, int32_t n, const hyc_tsadvc_params *p, dou
   a.ld1 = c->ld1;
   a.ld2 = c->ld2;
   a.slice = sl;
-  a.ntx = (c->idm + c->shape.tx - 1) / c->shape.tx;
-  a.nty = (c->jdm + c->shape.ty - 1) / c->shape.ty;
   a.mode = 0;
   a.msk = c->d_msk;
   a.scal = c->d_scp2;
@@ -941,16 +947,17 @@ int hyc_tsadvc(hyc_ctx *c, int32_t m, int32_t n, const hyc_tsadvc_params *p, dou
     TileArgs a;
     int nlay;
     long map0;  // first TMA map, -1: plain loads
+    hyc::TilePlan plan;
   };
   std::vector<Launch> launches;
   TileMaps tmv;
-  const bool fct = hyc::advect_tiles_tma(at, c->shape);  // the tile kernel stages by TMA
   auto plan = [&](const std::vector<FieldDesc> &grp, int nlay, bool flux1) {
     for (size_t f0 = 0; f0 < grp.size(); f0 += chunk) {
-      Launch L{a, nlay, -1};
+      Launch L{a, nlay, -1, {}};
       L.a.nfld = (int)(grp.size() - f0) < chunk ? (int)(grp.size() - f0) : chunk;
       for (int q = 0; q < L.a.nfld; q++) L.a.f[q] = grp[f0 + q];
-      if (fct && !hyc::march_takes(at, L.a, nlay)) L.map0 = tile_maps_add(c, L.a, kk, flux1, tmv);
+      L.plan = plan_tiles(at, L.a, nlay, c->shape, c->shape_fixed);
+      if (L.plan.tma) L.map0 = tile_maps_add(c, L.a, L.plan.shape, kk, flux1, tmv);
       launches.push_back(L);
     }
   };
@@ -985,7 +992,7 @@ int hyc_tsadvc(hyc_ctx *c, int32_t m, int32_t n, const hyc_tsadvc_params *p, dou
     }
     {
       Timed t(c, HYC_T_ADVECT);
-      CK(hyc::launch_advect_tiles(at, L.a, L.nlay, c->shape, s), "advect kernel");
+      CK(hyc::launch_advect_tiles(at, L.a, L.nlay, L.plan.shape, s), "advect kernel");
       int rc2;
       if (c->lconserve && (rc2 = conserve(c, L.a, L.nlay))) return rc2;
     }

@@ -25,6 +25,12 @@ size_t advect_tiles_smem(TileShape shape);
 bool advect_tiles_tma(int scheme, TileShape shape);
 // the launch goes to a strip kernel (hyc_march.cuh), which takes no tensor maps
 bool march_takes(int scheme, const TileArgs &a, int nlayers);
+// tile shape of a launch (fixed: the one given) and whether it takes tensor maps
+struct TilePlan {
+  TileShape shape;
+  bool tma;
+};
+TilePlan tile_plan(int scheme, const TileArgs &a, int nlayers, TileShape shape, bool fixed);
 bool advect_tile_shape_ok(TileShape shape);
 
 // Copy the interior of out[(fi*kdm+k)] back into field level n for every

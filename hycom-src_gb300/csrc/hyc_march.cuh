@@ -35,6 +35,7 @@
 
 #include "hyc_args.h"
 #include "hyc_device.cuh"
+#include "hyc_pdl.cuh"
 
 namespace hyc {
 
@@ -659,6 +660,7 @@ __device__ __forceinline__ void march1_body(const TileArgs &A, const FieldDesc *
 // next to each other
 template <int SCHEME, int NT, int NG>
 __global__ void __launch_bounds__(NT *NG, 512 / (NT * NG)) march_kernel(const TileArgs A, int nrow) {
+  after_previous();
   extern __shared__ __align__(16) char smc[];
   const int ngrp = (A.nfld + NG - 1) / NG;
   const int k = blockIdx.z / ngrp, q = blockIdx.z - k * ngrp;

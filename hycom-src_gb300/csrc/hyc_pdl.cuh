@@ -1,0 +1,41 @@
+// hyc_pdl.cuh -- programmatic dependent launch for chains of short kernels.
+//
+// A kernel launched by launch_after may be set up, and its blocks scheduled,
+// while the one before it in the stream still runs; after_previous, the first
+// thing such a kernel does, waits until that one has finished and its writes
+// are visible, and lets the next kernel's blocks come.  Only the launch gap
+// goes (cnuity on 1500x1100x41: 410 kernels of 20-80 us).  After anything but
+// a kernel (a copy, an event) the launch is an ordinary one.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace hyc {
+
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_after_smem(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t s, A &&...args) {
+  return launch_after_smem(kern, grid, block, 0, s, std::forward<A>(args)...);
+}
+
+}  // namespace hyc

@@ -38,6 +38,7 @@
 
 #include "hyc_args.h"
 #include "hyc_device.cuh"
+#include "hyc_pdl.cuh"
 #include "hyc_tma.cuh"
 
 namespace hyc {
@@ -56,6 +57,7 @@ __device__ __forceinline__ void for_rect(int a0, int a1, int b0, int b1, F f) {
 
 template <int SCHEME, int TX, int TY>
 __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
+  after_previous();
   using G = TileGeom<TX, TY>;
   constexpr int RX = G::RX, RW = G::RW, RY = G::RY, N = G::N, NR = G::NR;
   extern __shared__ __align__(16) double sm[];
