@@ -800,6 +800,26 @@ static int move(hyc_ens *e, int32_t basin, int32_t what, int32_t s0, int32_t ns_
     if (what == HYC_E_OLD || what == HYC_E_CUR) e->primed = false;
     return HYC_OK;
   }
+  // get into this device's memory: one kernel on the ensemble's stream
+  // (staging and copying it out would move every value three times); the copy
+  // stream's event follows it, so that waiting works as for a copy
+  cudaPointerAttributes pa;
+  if (where == HYC_DEVICE && cudaPointerGetAttributes(&pa, host) == cudaSuccess && pa.type == cudaMemoryTypeDevice &&
+      pa.device == e->device) {
+    cudaEvent_t t1 = span_open(e, e->stream);
+    c = hyc::launch_repitch(dst, dfp32, b.ld1, b.slice, host, 0, b.ld1r, rsl, b.ld1r, b.ld2, ns, e->stream);
+    if (c != cudaSuccess) return efail(e, HYC_ERR_CUDA, "get: %s", cudaGetErrorString(c));
+    span_close(e, t1, HYC_T_XCTILR, e->stream);
+    ECK(cudaEventRecord(e->ev_staged, e->stream), "event");
+    ECK(cudaStreamWaitEvent(e->copy_stream, e->ev_staged, 0), "wait staged");
+    ECK(cudaEventRecord(e->ev_gdone, e->copy_stream), "event");
+    e->get_pending = true;
+    if (!async_get) {
+      ECK(cudaEventSynchronize(e->ev_gdone), "get sync");
+      e->get_pending = false;
+    }
+    return HYC_OK;
+  }
   // get: repitch into the get staging on the ensemble's stream (after any
   // copy-out still reading it), then copy out
   if (e->gstage_bytes < bytes) {

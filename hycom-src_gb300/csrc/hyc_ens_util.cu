@@ -51,22 +51,61 @@ cudaError_t launch_diff_table(const double *aspux, const double *aspvy, const do
 // format conversion between the reference layout (FP64, pitch ld1) and the
 // ensemble layout (FP32 or FP64, pitch ld1p), nslices slices
 // ---------------------------------------------------------------------------
+// Conversions on the integer pipes: a conversion instruction issues at the
+// FP64 rate.  Values the bit forms do not cover (infinities, NaNs, FP32
+// subnormals and overflow) take it, as a real call: predicated into the loop
+// it would hold the FP64 pipe for every element.
+static __device__ __noinline__ double widen_slow(float x) { return (double)x; }
+static __device__ __noinline__ float narrow_slow(double x) { return (float)x; }
+__device__ __forceinline__ void convert(float x, float &y) { y = x; }
+__device__ __forceinline__ void convert(double x, double &y) { y = x; }
+__device__ __forceinline__ void convert(float x, double &y) {
+  const unsigned b = __float_as_uint(x), e = b & 0x7F800000u;
+  if (e - 0x00800000u < 0x7F000000u)  // normal: exponent rebased by 1023-127
+    y = __hiloint2double((int)(((unsigned)((int)b >> 3) & 0x8FFFFFFFu) + 0x38000000u), (int)(b << 29));
+  else if ((b << 1) == 0)
+    y = __hiloint2double((int)b, 0);
+  else
+    y = widen_slow(x);
+}
+__device__ __forceinline__ void convert(double x, float &y) {  // to nearest, ties to even
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  if ((h & 0x7FFFFFFFu) - 0x38100000u < 0x0FD00000u) {  // 2^-126 .. 2^127: rounds to a finite normal
+    const unsigned t = __funnelshift_l(l, h, 3) + 0x40000000u;
+    y = __uint_as_float((t + (((l & 0x1FFFFFFFu) + 0x0FFFFFFFu + (t & 1u)) >> 29)) | (h & 0x80000000u));
+  } else if (((h << 1) | l) == 0) {
+    y = __uint_as_float(h);
+  } else {
+    y = narrow_slow(x);
+  }
+}
+
+// A warp takes a row at a time, four elements of a lane in flight.  Bound by
+// memory: 4500x3298, 82 slices to FP64, see launch_repitch.
 template <class S, class D>
-__global__ void repitch_kernel(const S *src, long long spitch, long long sslice, D *dst, long long dpitch,
-                               long long dslice, int w, int h) {
-  const long long n = (long long)w * h;
+__global__ void __launch_bounds__(256) repitch_kernel(const S *src, long long spitch, long long sslice, D *dst,
+                                                      long long dpitch, long long dslice, int w, int h) {
   const S *s = src + blockIdx.y * sslice;
   D *d = dst + blockIdx.y * dslice;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int j = (int)(t / w), i = (int)(t - (long long)j * w);
-    d[i + j * dpitch] = (D)s[i + j * spitch];
+  const int lane = threadIdx.x & 31;
+  for (int j = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)); j < h; j += (int)gridDim.x * 8) {
+    const S *sr = s + j * spitch;
+    D *dr = d + j * dpitch;
+    for (int i0 = lane; i0 < w; i0 += 128) {
+      S v[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++)
+        if (i0 + 32 * r < w) v[r] = sr[i0 + 32 * r];
+#pragma unroll
+      for (int r = 0; r < 4; r++)
+        if (i0 + 32 * r < w) convert(v[r], dr[i0 + 32 * r]);
+    }
   }
 }
 
 cudaError_t launch_repitch(const void *src, int src_fp32, long long spitch, long long sslice, void *dst, int dst_fp32,
                            long long dpitch, long long dslice, int w, int h, int nslices, cudaStream_t s) {
-  long long n = (long long)w * h;
-  int bx = (int)((n + 255) / 256);
+  int bx = (h + 7) / 8;
   if (bx > 2048) bx = 2048;
   for (int z0 = 0; z0 < nslices; z0 += 65535) {
     int nz = nslices - z0 < 65535 ? nslices - z0 : 65535;
