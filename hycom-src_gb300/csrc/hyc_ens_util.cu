@@ -80,8 +80,10 @@ __device__ __forceinline__ void convert(double x, float &y) {  // to nearest, ti
   }
 }
 
-// A warp takes a row at a time, four elements of a lane in flight.  Bound by
-// memory: 4500x3298, 82 slices to FP64, see launch_repitch.
+// A warp takes a row at a time, four elements of a lane in flight; bound by
+// memory.  A get of 82 slices of 4500x3298 into device memory with a step of the
+// mixed form: 30.2 -> 26.2 ms for three steps and the get, of it the staging copy
+// and the conversions.
 template <class S, class D>
 __global__ void __launch_bounds__(256) repitch_kernel(const S *src, long long spitch, long long sslice, D *dst,
                                                       long long dpitch, long long dslice, int w, int h) {

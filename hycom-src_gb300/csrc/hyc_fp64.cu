@@ -204,7 +204,9 @@ cudaError_t launch_march_queue(int scheme, const TileArgs *basins, const int4 *i
 
 // ---------------------------------------------------------------------------
 // copy the interior of the output slices back into field level n
-// grid: (blocks over interior, nlayers, nfld)
+// grid: (blocks of 8 rows, nlayers, nfld); a warp takes a row, four elements
+// of a lane in flight.  Bound by memory (17 bytes a cell): 1500x1100x10, T and
+// S: 0.071 ms, 0.138 ms with an index division a cell and one element in flight
 // ---------------------------------------------------------------------------
 __global__ void copy_back_kernel(const TileArgs A) {
   after_previous();
@@ -214,11 +216,25 @@ __global__ void copy_back_kernel(const TileArgs A) {
   const long long sl = A.slice;
   double *dst = fd.nbase + (long long)(k + fd.k_off) * sl;
   const double *src = A.out + ((long long)fi * A.kdm + k) * sl;
-  const long long n = (long long)A.ii * A.jj;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    int j = (int)(t / A.ii), i = (int)(t - (long long)j * A.ii);
-    long long o = (long long)(i + A.nbdy) + (long long)(j + A.nbdy) * A.ld1;
-    if (A.msk[o] & kIP) dst[o] = A.cfac ? src[o] * A.cfac[fi * A.kdm + k] : src[o];  // sea points only
+  const int lane = threadIdx.x & 31;
+  const double fac = A.cfac ? A.cfac[fi * A.kdm + k] : 1.0;
+  for (int j = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)); j < A.jj; j += (int)gridDim.x * 8) {
+    const long long row = (long long)(j + A.nbdy) * A.ld1 + A.nbdy;
+    for (int i0 = lane; i0 < A.ii; i0 += 128) {
+      double v[4];
+      uint8_t m[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const bool in = i0 + 32 * r < A.ii;
+        m[r] = in ? A.msk[row + i0 + 32 * r] : 0;
+        if (in) v[r] = src[row + i0 + 32 * r];
+      }
+      if (A.cfac)
+        for (int r = 0; r < 4; r++) v[r] = v[r] * fac;
+#pragma unroll
+      for (int r = 0; r < 4; r++)
+        if (m[r] & kIP) dst[row + i0 + 32 * r] = v[r];  // sea points only
+    }
   }
 }
 
@@ -309,8 +325,7 @@ cudaError_t launch_conserve(const TileArgs &a, int nlayers, double *rows, double
 }
 
 cudaError_t launch_copy_back(const TileArgs &a, int nlayers, cudaStream_t s) {
-  long long n = (long long)a.ii * a.jj;
-  int bx = (int)((n + 255) / 256);
+  int bx = (a.jj + 7) / 8;
   if (bx > 1216) bx = 1216;
   dim3 grid(bx, nlayers, a.nfld);
   return launch_after(copy_back_kernel, grid, dim3(256), s, a);
