@@ -803,9 +803,17 @@ static int move(hyc_ens *e, int32_t basin, int32_t what, int32_t s0, int32_t ns_
   // get into this device's memory: one kernel on the ensemble's stream
   // (staging and copying it out would move every value three times); the copy
   // stream's event follows it, so that waiting works as for a copy
-  cudaPointerAttributes pa;
-  if (where == HYC_DEVICE && cudaPointerGetAttributes(&pa, host) == cudaSuccess && pa.type == cudaMemoryTypeDevice &&
-      pa.device == e->device) {
+  bool direct = where == HYC_DEVICE && ((uintptr_t)host & 7) == 0;  // a copy needs no alignment, nor its own device
+  if (direct) {
+    cudaPointerAttributes pa;
+    if (cudaPointerGetAttributes(&pa, host) != cudaSuccess) {
+      cudaGetLastError();
+      direct = false;
+    } else {
+      direct = pa.type == cudaMemoryTypeDevice && pa.device == e->device;
+    }
+  }
+  if (direct) {
     cudaEvent_t t1 = span_open(e, e->stream);
     c = hyc::launch_repitch(dst, dfp32, b.ld1, b.slice, host, 0, b.ld1r, rsl, b.ld1r, b.ld2, ns, e->stream);
     if (c != cudaSuccess) return efail(e, HYC_ERR_CUDA, "get: %s", cudaGetErrorString(c));
