@@ -482,7 +482,7 @@ def run_tsadvc_fp64(args, wl, b, masks, nreg, sc, si, case, dev, stream, dist, l
         res["roofline"] = {"bound": "fp64-alu (hbm fraction shown)", "achieved": achieved, "peak": peak,
                            "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                            "kernel": ("fct2c_* stage kernels" if btrmas and advtyp == 2 else
-                                      "fct_tile_kernel" if advtyp in (2, 4) else "advect_tile_kernel"),
+                                      "march_kernel"),
                            "algorithmic_bytes_per_update": bpu,
                            "advect_ms_per_step": adv_ms / ts_calls, "advect_spans_per_step": adv_calls / ts_calls,
                            "share_of_step": adv_ms / max(st["tsadvc"][0], 1e-9),
