@@ -372,15 +372,25 @@ cudaError_t launch_iso_smooth(const double *uk, const double *vk, const uint8_t 
 }
 
 // ---------------------------------------------------------------------------
+// The arrays of one halo launch: levels first[q] .. first[q+1]-1 of the grid are array q's
+struct HaloList {
+  static constexpr int kMax = 16;
+  double *a[kMax];
+  int first[kMax + 1];
+  int n;
+};
+
 // xctilr, mod_xc_sm.h:1337-1428.  Every halo cell is computed directly from
 // interior cells (the reference's N/S pass followed by the E/W pass over
 // rows 1-nhl..jj+nhl gives the same values), so one launch has no ordering
-// hazard.  grid: (blocks, nlev)
+// hazard.  grid: (blocks, levels of every array)
 // ---------------------------------------------------------------------------
-__global__ void xctilr_kernel(double *a, long long slice, int ii, int jj, int nb, int ld1, int mhl, int nhl,
+__global__ void xctilr_kernel(const HaloList L, long long slice, int ii, int jj, int nb, int ld1, int mhl, int nhl,
                               int nreg) {
   after_previous();
-  double *s = a + (long long)blockIdx.y * slice;
+  int q = 0;
+  while (q + 1 < L.n && (int)blockIdx.y >= L.first[q + 1]) q++;
+  double *s = L.a[q] + (long long)((int)blockIdx.y - L.first[q]) * slice;
   const bool closed_y = nreg <= 2, closed_x = (nreg == 0 || nreg == 4);
   const long long W = (long long)ii + 2 * mhl;
   const long long nns = 2LL * nhl * W, new_ = 2LL * mhl * jj;
@@ -413,24 +423,46 @@ __global__ void xctilr_kernel(double *a, long long slice, int ii, int jj, int nb
   }
 }
 
-cudaError_t launch_xctilr(double *a, long long slice, int nlev, int ii, int jj, int nbdy, int ld1, int mh, int nh,
-                          int nreg, cudaStream_t s) {
+cudaError_t launch_xctilr_list(const std::vector<std::pair<double *, int>> &list, long long slice, int ii, int jj, int nbdy, int ld1, int mh, int nh,
+                               int nreg, int *launches, cudaStream_t s) {
   if (nreg < 0) return cudaSuccess;  // HYC_NREG_EXTERNAL: the caller exchanges the halos
   int mhl = mh < nbdy ? mh : nbdy;
   if (mhl < 0) mhl = 0;
   int nhl = nh < nbdy ? nh : nbdy;
   if (nhl < 0) nhl = 0;
-  if (nlev <= 0 || (mhl == 0 && nhl == 0)) return cudaSuccess;
+  if (mhl == 0 && nhl == 0) return cudaSuccess;
   long long n = 2LL * nhl * (ii + 2LL * mhl) + 2LL * mhl * jj;
   int bx = (int)((n + 255) / 256);
   if (bx > 512) bx = 512;
-  for (int l0 = 0; l0 < nlev; l0 += 65535) {
-    int nl = nlev - l0 < 65535 ? nlev - l0 : 65535;
-    const cudaError_t e = launch_after(xctilr_kernel, dim3(bx, nl), dim3(256), s, a + (long long)l0 * slice, slice, ii, jj,
-                                       nbdy, ld1, mhl, nhl, nreg);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaGetLastError();
+  // the levels of all the arrays one after another, at most 65535 (the grid's limit) a launch
+  HaloList part = {};
+  auto flush = [&]() -> cudaError_t {
+    if (part.n == 0) return cudaSuccess;
+    const int nl = part.first[part.n];
+    if (launches) *launches += 1;
+    const cudaError_t e =
+        launch_after(xctilr_kernel, dim3(bx, nl), dim3(256), s, part, slice, ii, jj, nbdy, ld1, mhl, nhl, nreg);
+    part = {};
+    return e;
+  };
+  for (const auto &x : list)
+    for (int l0 = 0; l0 < x.second;) {
+      const int nl = std::min(x.second - l0, 65535 - part.first[part.n]);
+      part.a[part.n] = x.first + (long long)l0 * slice;
+      part.first[part.n + 1] = part.first[part.n] + nl;
+      part.n++;
+      l0 += nl;
+      if (part.first[part.n] == 65535 || part.n == HaloList::kMax) {
+        const cudaError_t e = flush();
+        if (e != cudaSuccess) return e;
+      }
+    }
+  return flush();
+}
+
+cudaError_t launch_xctilr(double *a, long long slice, int nlev, int ii, int jj, int nbdy, int ld1, int mh, int nh,
+                          int nreg, cudaStream_t s) {
+  return launch_xctilr_list({{a, nlev}}, slice, ii, jj, nbdy, ld1, mh, nh, nreg, nullptr, s);
 }
 
 // ---------------------------------------------------------------------------

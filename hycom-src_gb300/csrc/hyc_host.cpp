@@ -802,27 +802,25 @@ int hyc_tsadvc(hyc_ctx *c, int32_t m, int32_t n, const hyc_tsadvc_params *p, dou
 
   // halo refresh, mod_tsadvc.F90:1827-1840 (dp halo is up to date on entry)
   const int l = kMbdy[at];
-  auto halo = [&](int id, int nlev) -> cudaError_t {
-    if (!F[id].dev) return cudaSuccess;
-    c->stats.launches += (nlev + 65534) / 65535;
-    return hyc::launch_xctilr(F[id].dev, sl, nlev, c->idm, c->jdm, c->nbdy, c->ld1, l, l, c->nreg, s);
-  };
   {
-  Timed t_halo(c, HYC_T_XCTILR);
-  CK(halo(HYC_F_SALN, 2 * kk), "xctilr saln");
-  CK(halo(HYC_F_TEMP, 2 * kk), "xctilr temp");
-  CK(halo(HYC_F_TH3D, 2 * kk), "xctilr th3d");
-  CK(halo(HYC_F_UFLX, kk), "xctilr uflx");
-  CK(halo(HYC_F_VFLX, kk), "xctilr vflx");
-  if (p->ntracr > 0) {
-    c->stats.launches += (2 * kk * p->ntracr + 65534) / 65535;
-    CK(hyc::launch_xctilr(F[HYC_F_TRACER].dev, sl, 2 * kk * p->ntracr, c->idm, c->jdm, c->nbdy, c->ld1, l, l,
-                          c->nreg, s), "xctilr tracer");
-  }
-  if (p->mxlmy) {
-    CK(halo(HYC_F_Q2, 2 * kk + 4), "xctilr q2");
-    CK(halo(HYC_F_Q2L, 2 * kk + 4), "xctilr q2l");
-  }
+    Timed t_halo(c, HYC_T_XCTILR);
+    std::vector<std::pair<double *, int>> halos;
+    auto halo = [&](int id, int nlev) {
+      if (F[id].dev) halos.push_back({F[id].dev, nlev});
+    };
+    halo(HYC_F_SALN, 2 * kk);
+    halo(HYC_F_TEMP, 2 * kk);
+    halo(HYC_F_TH3D, 2 * kk);
+    halo(HYC_F_UFLX, kk);
+    halo(HYC_F_VFLX, kk);
+    if (p->ntracr > 0) halo(HYC_F_TRACER, 2 * kk * p->ntracr);
+    if (p->mxlmy) {
+      halo(HYC_F_Q2, 2 * kk + 4);
+      halo(HYC_F_Q2L, 2 * kk + 4);
+    }
+    int nl = 0;
+    CK(hyc::launch_xctilr_list(halos, sl, c->idm, c->jdm, c->nbdy, c->ld1, l, l, c->nreg, &nl, s), "xctilr");
+    c->stats.launches += nl;
   }
 
   // field list in the reference's call order (mod_tsadvc.F90:1969-2048)
@@ -1086,10 +1084,9 @@ int hyc_tsdff(hyc_ctx *c, int32_t m, int32_t n, const hyc_tsadvc_params *p, doub
     halos.push_back({F[HYC_F_TRACER].dev + ((long long)t * 2 * kk + (long long)nn * kk) * sl, kk});
   {
     Timed t(c, HYC_T_XCTILR);
-    for (auto &h : halos) {
-      CK(hyc::launch_xctilr(h.first, sl, h.second, c->idm, c->jdm, c->nbdy, c->ld1, mdf, mdf, c->nreg, s), "xctilr");
-      c->stats.launches += (h.second + 65534) / 65535;
-    }
+    int nl = 0;
+    CK(hyc::launch_xctilr_list(halos, sl, c->idm, c->jdm, c->nbdy, c->ld1, mdf, mdf, c->nreg, &nl, s), "xctilr");
+    c->stats.launches += nl;
   }
   // the diffused fields, layer 1 of level n; temp and saln first (they give th3d)
   std::vector<double *> fl = {F[HYC_F_TEMP].dev + (long long)nn * kk * sl, F[HYC_F_SALN].dev + (long long)nn * kk * sl};
@@ -1308,20 +1305,17 @@ int hyc_cnuity(hyc_ctx *c, int32_t m, int32_t n, const hyc_cnuity_params *p, dou
   Timed t_all(c, HYC_T_CNUITY);
   const int mm = m - 1;
   // halos, cnuity.F90:100-107 (dpmixl is not carried)
-  struct H {
-    double *a;
-    int nlev;
-  } halos[] = {{F[HYC_F_DP].dev, 2 * kk},
-               {F[HYC_F_DPU].dev + (long long)mm * kk * sl, kk},
-               {F[HYC_F_DPV].dev + (long long)mm * kk * sl, kk},
-               {F[HYC_F_U].dev + (long long)mm * kk * sl, kk},
-               {F[HYC_F_V].dev + (long long)mm * kk * sl, kk},
-               {F[HYC_F_UBAVG].dev + (long long)mm * sl, 1},
-               {F[HYC_F_VBAVG].dev + (long long)mm * sl, 1}};
-  for (auto &h : halos) {
-    CK(hyc::launch_xctilr(h.a, sl, h.nlev, c->idm, c->jdm, c->nbdy, c->ld1, 6, 6, c->nreg, s), "xctilr");
-    c->stats.launches += 1;
-  }
+  const std::vector<std::pair<double *, int>> halos = {
+      {F[HYC_F_DP].dev, 2 * kk},
+      {F[HYC_F_DPU].dev + (long long)mm * kk * sl, kk},
+      {F[HYC_F_DPV].dev + (long long)mm * kk * sl, kk},
+      {F[HYC_F_U].dev + (long long)mm * kk * sl, kk},
+      {F[HYC_F_V].dev + (long long)mm * kk * sl, kk},
+      {F[HYC_F_UBAVG].dev + (long long)mm * sl, 1},
+      {F[HYC_F_VBAVG].dev + (long long)mm * sl, 1}};
+  int nhalo = 0;
+  CK(hyc::launch_xctilr_list(halos, sl, c->idm, c->jdm, c->nbdy, c->ld1, 6, 6, c->nreg, &nhalo, s), "xctilr");
+  c->stats.launches += nhalo;
   hyc::CnuityArgs a;
   memset(&a, 0, sizeof a);
   a.ii = c->idm;

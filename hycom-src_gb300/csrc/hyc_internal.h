@@ -5,6 +5,9 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include <utility>
+#include <vector>
+
 namespace hyc {
 
 struct FieldDesc;
@@ -69,6 +72,10 @@ cudaError_t launch_cnuity_rest(const CnuityArgs &a, int *launches, cudaStream_t 
 cudaError_t launch_iso_smooth(const double *uk, const double *vk, const uint8_t *msk, long long slice, int ii, int jj,
                               int nb, int ld1, int margin, double *us, double *vs, cudaStream_t s);
 
+// xctilr on several arrays of (levels) slices in one launch (a small tsadvc's
+// five took 15 us of 160); launches, if given, counts them
+cudaError_t launch_xctilr_list(const std::vector<std::pair<double *, int>> &list, long long slice, int ii, int jj,
+                               int nbdy, int ld1, int mh, int nh, int nreg, int *launches, cudaStream_t s);
 // xctilr on nlev slices (mod_xc_sm.h:1337-1428).
 cudaError_t launch_xctilr(double *a, long long slice, int nlev, int ii, int jj, int nbdy, int ld1, int mh,
                           int nh, int nreg, cudaStream_t s);
