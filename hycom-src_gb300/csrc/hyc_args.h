@@ -137,6 +137,7 @@ struct CnuityArgs {
   double delt1, ra2fac;
   double dtinv;                     // 1/delt1, divided once on the host
   double *w;                        // work slices
+  int nbatch, k0;                   // layers per launch, first layer (0-based) of this one
   long long *keys;                  // 2*kdm dpkmin keys, or null
 };
 

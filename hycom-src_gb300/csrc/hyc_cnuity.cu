@@ -6,11 +6,13 @@
 //
 // The reference is a sequence of sweeps over the slice whose margins shrink
 // from 6 to 0 within a layer, with a vertical recurrence (util3 = depth of
-// the layer's top, p = interface pressures) from one layer to the next.  The
-// first GPU form keeps that structure: one kernel per sweep over the same
-// margin, layer after layer, so every value the reference computes (halo
-// cells included) is computed here, in the same operation order, FP64
-// without FMA contraction: the results equal the oracle's bit for bit.
+// the layer's top, p = interface pressures) from one layer to the next.  Here
+// one kernel does a sweep over the same margin for a batch of layers: util3 is
+// a running sum of the thicknesses as they came, p one of the results, and
+// neither is read by another layer's sweeps in between, so both are formed by
+// kernels of their own.  Every value the reference computes (halo cells
+// included) is computed, in the same operation order, FP64 without FMA
+// contraction: the results equal the oracle's bit for bit.
 //
 // What bounds them: at the start the FP64 pipe (71-82 % busy in every sweep);
 // with products and divisions on the integer pipes (hyc_div.cuh) the pipe, the
@@ -21,8 +23,9 @@
 // cn_thk_flux 112 / 82, cn_thk_p 21 / 19.  The sweeps move about 55 slices per
 // cell and layer against 11 for a fused form.
 //
-// Work slices (CnuityArgs::w): uflux, vflux, uflux2, vflux2, utotn, vtotn,
-// util1, util2, util3, pold, oneta_u, oneta_v, onetamas(:,:,1:2).
+// Work slices (CnuityArgs::w): utotn, vtotn, util3 below the batch, pold, the
+// reciprocal of p(kk+1), oneta_u, oneta_v, onetamas(:,:,1:2); then for each layer
+// of a batch uflux, vflux, uflux2, vflux2, util1, util2, util3.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -37,7 +40,9 @@ namespace hyc {
 
 namespace {
 
-enum { W_UF, W_VF, W_UF2, W_VF2, W_UTN, W_VTN, W_U1, W_U2, W_U3, W_POLD, W_OU, W_OV, W_OM, W_N = W_OM + 2 };
+// one slice each, then A.nbatch slices each (layer k0 + l of a batch in slice l)
+enum { W_UTN, W_VTN, W_U3T, W_POLD, W_RPB, W_OU, W_OV, W_OM, W_FIX = W_OM + 2 };
+enum { B_UF, B_VF, B_UF2, B_VF2, B_U1, B_U2, B_U3, B_N };
 
 constexpr double kOnem = 9.806 / (1.0 / 1000.0);  // onem = g/svref, mod_cb_arrays.F90:843-846
 constexpr double kOnecm = kOnem * 0.01;
@@ -60,6 +65,9 @@ __device__ __forceinline__ bool cell_of(const CnuityArgs &A, int M, Cell &x) {
 }
 
 __device__ __forceinline__ double *W(const CnuityArgs &A, int s) { return A.w + (long long)s * A.slice; }
+__device__ __forceinline__ double *WB(const CnuityArgs &A, int s, int l) {
+  return A.w + ((long long)W_FIX + (long long)s * A.nbatch + l) * A.slice;
+}
 
 // the reference's max/min of two reals (ordered as written; signs of zero
 // never reach a result of this path)
@@ -106,11 +114,40 @@ __global__ void cn_init(const CnuityArgs A) {
   }
   W(A, W_UTN)[c] = 0.0;
   W(A, W_VTN)[c] = 0.0;
-  W(A, W_U3)[c] = 0.0;
+  W(A, W_U3T)[c] = 0.0;
   for (int k = 0; k < A.kdm; k++) {
     const long long o = ((long long)k + (long long)nn * A.kdm) * sl + c;
     A.dpo[o] = A.dp[o];
   }
+}
+
+// util3, the depth of each layer's top, of the batch's layers: the running sum
+// of dp(:,:,k,n) before the layers' own updates (:300-306), at the sea cells of
+// margin 4, where the reference forms it layer after layer; 0 elsewhere
+__global__ void cn_top(const CnuityArgs A, int nl) {
+  after_previous();
+  Cell x;
+  if (!cell_of(A, 4, x)) return;
+  const long long c = x.c, sl = A.slice;
+  if (!(A.msk[c] & kIP)) return;
+  const double *dk = A.dp + ((long long)A.k0 + (long long)(A.n - 1) * A.kdm) * sl + c;
+  double t = W(A, W_U3T)[c];
+  int l = 0;
+  for (; l + 4 <= nl; l += 4) {
+    double d[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) d[r] = dk[(long long)(l + r) * sl];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      WB(A, B_U3, l + r)[c] = t;
+      t = t + d[r];
+    }
+  }
+  for (; l < nl; l++) {
+    WB(A, B_U3, l)[c] = t;
+    t = t + dk[(long long)l * sl];
+  }
+  W(A, W_U3T)[c] = t;
 }
 
 // loop 76, :240-285 at margin 5: low-order and antidiffusive fluxes of layer k.
@@ -118,15 +155,16 @@ __global__ void cn_init(const CnuityArgs A) {
 // (:142-145), and x*1.0 == x exactly, so those products (and their loads)
 // are skipped; the FP64 pipe bounds this kernel.
 template <bool BT>
-__global__ void cn_flux(const CnuityArgs A, int k) {
+__global__ void cn_flux(const CnuityArgs A) {
   after_previous();
+  const int l = blockIdx.z, k = A.k0 + l;
   Cell x;
   if (!cell_of(A, 5, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
   const int mm = A.m - 1, nn = A.n - 1;
   const uint8_t mk = A.msk[c];
   const double *dk = A.dp + ((long long)k + (long long)nn * A.kdm) * sl;
-  const double *u3 = W(A, W_U3), *omn = W(A, W_OM) + nn * sl;
+  const double *u3 = WB(A, B_U3, l), *omn = W(A, W_OM) + nn * sl;
   const long long lm = ((long long)k + (long long)mm * A.kdm) * sl;
   if (!(mk & (kIU | kIV))) return;
   // every operand is loaded before the first is used: the upwind cell is
@@ -139,9 +177,9 @@ __global__ void cn_flux(const CnuityArgs A, int k) {
     const bool up = ge0(utotm);
     const double q0 = mn(up ? dw : d0, mx(0., du - (up ? tw : t0)));
     const double uf = mul_rn(utotm, BT ? mul_rn(q0, omn[up ? c - 1 : c]) : q0);
-    W(A, W_UF)[c] = uf;
+    WB(A, B_UF, l)[c] = uf;
     const double ud = mul_rn(utotm, hu);
-    W(A, W_UF2)[c] = (BT ? mul_rn(ud, W(A, W_OU)[c]) : ud) - uf;
+    WB(A, B_UF2, l)[c] = (BT ? mul_rn(ud, W(A, W_OU)[c]) : ud) - uf;
     A.uflx[(long long)k * sl + c] = uf;
   }
   if (mk & kIV) {
@@ -149,9 +187,9 @@ __global__ void cn_flux(const CnuityArgs A, int k) {
     const bool up = ge0(vtotm);
     const double q0 = mn(up ? ds : d0, mx(0., dv - (up ? ts : t0)));
     const double vf = mul_rn(vtotm, BT ? mul_rn(q0, omn[up ? c - ld : c]) : q0);
-    W(A, W_VF)[c] = vf;
+    WB(A, B_VF, l)[c] = vf;
     const double vd = mul_rn(vtotm, hv);
-    W(A, W_VF2)[c] = (BT ? mul_rn(vd, W(A, W_OV)[c]) : vd) - vf;
+    WB(A, B_VF2, l)[c] = (BT ? mul_rn(vd, W(A, W_OV)[c]) : vd) - vf;
     A.vflx[(long long)k * sl + c] = vf;
   }
 }
@@ -168,8 +206,9 @@ __device__ __forceinline__ void row_min(const CnuityArgs &A, const Cell &x, bool
 
 // loop 19, :294-315 at margin 4: low-order update of dp(k,n) (BT as cn_flux)
 template <bool BT>
-__global__ void cn_low(const CnuityArgs A, int k) {
+__global__ void cn_low(const CnuityArgs A) {
   after_previous();
+  const int l = blockIdx.z, k = A.k0 + l;
   Cell x;
   const bool in = cell_of(A, 4, x);
   bool sea = false;
@@ -178,8 +217,7 @@ __global__ void cn_low(const CnuityArgs A, int k) {
     const long long c = x.c, sl = A.slice, ld = A.ld1;
     const int mm = A.m - 1, nn = A.n - 1;
     double *dk = A.dp + ((long long)k + (long long)nn * A.kdm) * sl;
-    const double *uf = W(A, W_UF), *vf = W(A, W_VF);
-    W(A, W_U3)[c] = W(A, W_U3)[c] + dk[c];
+    const double *uf = WB(A, B_UF, l), *vf = WB(A, B_VF, l);
     d = (BT ? mul_rn(dk[c], W(A, W_OM)[nn * sl + c]) : dk[c]) -
         mul_rn(mul_rn((uf[c + 1] - uf[c]) + (vf[c + ld] - vf[c]), A.delt1), A.scp2i[c]);
     dk[c] = d;
@@ -190,8 +228,9 @@ __global__ void cn_low(const CnuityArgs A, int k) {
 }
 
 // :400-430 at margin 4: the limiter's ratios
-__global__ void cn_ratio(const CnuityArgs A, int k) {
+__global__ void cn_ratio(const CnuityArgs A) {
   after_previous();
+  const int l = blockIdx.z, k = A.k0 + l;
   Cell x;
   if (!cell_of(A, 4, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
@@ -205,7 +244,7 @@ __global__ void cn_ratio(const CnuityArgs A, int k) {
   const double d = dk[c];
   const double u1 = mx(mx(mx(mx(d, dk[ca]), dk[cb]), dk[cja]), dk[cjb]);
   const double u2 = mx(0., mn(mn(mn(mn(d, dk[ca]), dk[cb]), dk[cja]), dk[cjb]));
-  const double *f2u = W(A, W_UF2), *f2v = W(A, W_VF2);
+  const double *f2u = WB(A, B_UF2, l), *f2v = WB(A, B_VF2, l);
   const double fu0 = f2u[c], fu1 = f2u[c + 1], fv0 = f2v[c], fv1 = f2v[c + ld];
   // The ratios are used as min(1, ratio) only.  FP32 bounds (below the
   // numerator, above the denominator) show most of them to be at least 1, and
@@ -228,8 +267,8 @@ __global__ void cn_ratio(const CnuityArgs A, int k) {
     if (!(fine && is0(n2)))
       r2 = div_rn(n2, mul_rn(mul_rn(((pos0(fu1) - neg0(fu0)) + (pos0(fv1) - neg0(fv0))) + kEpsilCb, A.delt1), A.scp2i[c]));
   }
-  W(A, W_U1)[c] = r1;
-  W(A, W_U2)[c] = r2;
+  WB(A, B_U1, l)[c] = r1;
+  WB(A, B_U2, l)[c] = r2;
 }
 
 // f2*clip; the part clipped off is added to rest (nothing where clip = 1)
@@ -239,38 +278,42 @@ __device__ __forceinline__ double clipped(double f2, double clip, double *rest) 
   return mul_rn(f2, clip);
 }
 
-// :442-472 at margin 3: clip the antidiffusive fluxes
-__global__ void cn_clip(const CnuityArgs A, int k) {
+// :442-472 at margin 3: clip the antidiffusive fluxes of the batch's layers.
+// A thread takes its faces through the layers, since utotn adds up in their order.
+__global__ void cn_clip(const CnuityArgs A, int nl) {
   after_previous();
   Cell x;
   if (!cell_of(A, 3, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
   const uint8_t mk = A.msk[c];
   if (!(mk & (kIU | kIV))) return;
-  const double *u1 = W(A, W_U1), *u2 = W(A, W_U2);
-  double *ul = A.uflx + (long long)k * sl + c, *vl = A.vflx + (long long)k * sl + c;
-  const double a1 = u1[c], a2 = u2[c], w1 = u1[c - 1], w2 = u2[c - 1], s1 = u1[c - ld], s2 = u2[c - ld];
-  const double f2 = W(A, W_UF2)[c], g2 = W(A, W_VF2)[c], ul0 = *ul, vl0 = *vl;
-  if (mk & kIU) {
-    const bool up = ge0(f2);
-    const double clip = mn(mn(1., up ? a1 : a2), up ? w2 : w1);
-    const double uf = clipped(f2, clip, W(A, W_UTN) + c);
-    W(A, W_UF)[c] = uf;
-    *ul = ul0 + uf;
-  }
-  if (mk & kIV) {
-    const bool up = ge0(g2);
-    const double clip = mn(mn(1., up ? a1 : a2), up ? s2 : s1);
-    const double vf = clipped(g2, clip, W(A, W_VTN) + c);
-    W(A, W_VF)[c] = vf;
-    *vl = vl0 + vf;
+  double *ul = A.uflx + (long long)A.k0 * sl + c, *vl = A.vflx + (long long)A.k0 * sl + c;
+  for (int l = 0; l < nl; l++, ul += sl, vl += sl) {
+    const double *u1 = WB(A, B_U1, l), *u2 = WB(A, B_U2, l);
+    const double a1 = u1[c], a2 = u2[c], w1 = u1[c - 1], w2 = u2[c - 1], s1 = u1[c - ld], s2 = u2[c - ld];
+    const double f2 = WB(A, B_UF2, l)[c], g2 = WB(A, B_VF2, l)[c], ul0 = *ul, vl0 = *vl;
+    if (mk & kIU) {
+      const bool up = ge0(f2);
+      const double clip = mn(mn(1., up ? a1 : a2), up ? w2 : w1);
+      const double uf = clipped(f2, clip, W(A, W_UTN) + c);
+      WB(A, B_UF, l)[c] = uf;
+      *ul = ul0 + uf;
+    }
+    if (mk & kIV) {
+      const bool up = ge0(g2);
+      const double clip = mn(mn(1., up ? a1 : a2), up ? s2 : s1);
+      const double vf = clipped(g2, clip, W(A, W_VTN) + c);
+      WB(A, B_VF, l)[c] = vf;
+      *vl = vl0 + vf;
+    }
   }
 }
 
 // loop 15 (:480-498, margin 2) and loop 14 (:650-665, margin 0): flux update
-// of dp(k,n) and p(k+1)
-__global__ void cn_update(const CnuityArgs A, int k, int M, int slot) {
+// of dp(k,n); slot: dpkmin slot of layer 1, -1: none
+__global__ void cn_update(const CnuityArgs A, int M, int slot) {
   after_previous();
+  const int l = blockIdx.z, k = A.k0 + l;
   Cell x;
   const bool in = cell_of(A, M, x);
   bool sea = false;
@@ -279,40 +322,67 @@ __global__ void cn_update(const CnuityArgs A, int k, int M, int slot) {
     const long long c = x.c, sl = A.slice, ld = A.ld1;
     const int nn = A.n - 1;
     double *dk = A.dp + ((long long)k + (long long)nn * A.kdm) * sl;
-    const double *uf = W(A, W_UF), *vf = W(A, W_VF);
+    const double *uf = WB(A, B_UF, l), *vf = WB(A, B_VF, l);
     d = dk[c] - mul_rn(mul_rn((uf[c + 1] - uf[c]) + (vf[c + ld] - vf[c]), A.delt1), A.scp2i[c]);
     dk[c] = d;
-    A.p[(long long)(k + 1) * sl + c] = A.p[(long long)k * sl + c] + d;
     sea = true;
   }
-  if (A.keys && slot >= 0) row_min(A, x, in && sea, d, slot);
+  if (A.keys && slot >= 0) row_min(A, x, in && sea, d, slot + k);
+}
+
+// p(k+1) = p(k) + dp(k,n) of every layer at margin M (:494-496, :661-663).  The
+// layers' updates do not read it but for p(kk+1), which loop 77 takes as it was.
+__global__ void cn_p(const CnuityArgs A, int M) {
+  after_previous();
+  Cell x;
+  if (!cell_of(A, M, x)) return;
+  const long long c = x.c, sl = A.slice;
+  if (!(A.msk[c] & kIP)) return;
+  const double *dk = A.dp + (long long)(A.n - 1) * A.kdm * sl + c;
+  double *p = A.p + c, t = *p;
+  int k = 0;
+  for (; k + 4 <= A.kdm; k += 4) {
+    double d[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) d[r] = dk[(long long)(k + r) * sl];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      t = t + d[r];
+      p[(long long)(k + r + 1) * sl] = t;
+    }
+  }
+  for (; k < A.kdm; k++) {
+    t = t + dk[(long long)k * sl];
+    p[(long long)(k + 1) * sl] = t;
+  }
 }
 
 // loop 77: the 32-bit reciprocal (recip_of) of p(kk+1) of every sea cell at
-// margin 2, into util1 (free until the interface diffusion).  p(kk+1) does
-// not change during loop 77 before its last layer's fluxes are formed, so one
-// reciprocal per cell serves every layer's division dp/p(kk+1).
+// margin 2.  p(kk+1) does not change during loop 77 before its last layer's
+// fluxes are formed, so one reciprocal per cell serves every layer's division
+// dp/p(kk+1).
 __global__ void cn_rpb(const CnuityArgs A) {
   after_previous();
   Cell x;
   if (!cell_of(A, 2, x)) return;
   const long long c = x.c;
   if (!(A.msk[c] & kIP)) return;
-  W(A, W_U1)[c] = __longlong_as_double(recip_of(A.p[(long long)A.kdm * A.slice + c]));
+  W(A, W_RPB)[c] = __longlong_as_double(recip_of(A.p[(long long)A.kdm * A.slice + c]));
 }
 
 // loop 77, :595-645 at margin 1: the barotropic correction fluxes of layer k.
 // q = dp/p(kk+1) by div_by with the cell's reciprocal.  A face that clipped
 // nothing (most) has no correction flux: uf = 0*q = 0 for its finite q.
-__global__ void cn_btflux(const CnuityArgs A, int k) {
+__global__ void cn_btflux(const CnuityArgs A) {
   after_previous();
+  const int l = blockIdx.z, k = A.k0 + l;
   Cell x;
   if (!cell_of(A, 1, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
   const uint8_t mk = A.msk[c];
   const int nn = A.n - 1;
   const double *dk = A.dp + ((long long)k + (long long)nn * A.kdm) * sl, *pb = A.p + (long long)A.kdm * sl;
-  const double *rpb = W(A, W_U1);
+  const double *rpb = W(A, W_RPB);
   if (!(mk & (kIU | kIV))) return;
   double *ul = A.uflx + (long long)k * sl + c, *vl = A.vflx + (long long)k * sl + c;
   const double ut = W(A, W_UTN)[c], vt = W(A, W_VTN)[c], d0 = dk[c], dw = dk[c - 1], ds = dk[c - ld], p0 = pb[c],
@@ -328,11 +398,11 @@ __global__ void cn_btflux(const CnuityArgs A, int k) {
   };
   if (mk & kIU) {
     const bool up = ge0(ut);
-    W(A, W_UF)[c] = flux(ut, up ? dw : d0, up ? pw : p0, up ? rw : r0, ul0, ul);
+    WB(A, B_UF, l)[c] = flux(ut, up ? dw : d0, up ? pw : p0, up ? rw : r0, ul0, ul);
   }
   if (mk & kIV) {
     const bool up = ge0(vt);
-    W(A, W_VF)[c] = flux(vt, up ? ds : d0, up ? ps : p0, up ? rs : r0, vl0, vl);
+    WB(A, B_VF, l)[c] = flux(vt, up ? ds : d0, up ? ps : p0, up ? rs : r0, vl0, vl);
   }
 }
 
@@ -359,10 +429,10 @@ __global__ void cn_thk_init(const CnuityArgs A, int bih, int iflip) {
   if (!cell_of(A, 6, x)) return;
   const long long c = x.c;
   const uint8_t mk = A.msk[c];
-  if (mk & kIU) W(A, W_UF)[c] = 0.;
-  if (mk & kIV) W(A, W_VF)[c] = 0.;
+  if (mk & kIU) WB(A, B_UF, 0)[c] = 0.;
+  if (mk & kIV) WB(A, B_VF, 0)[c] = 0.;
   if (mk & kIP) {
-    if (!bih) W(A, W_VF)[c] = 0.;
+    if (!bih) WB(A, B_VF, 0)[c] = 0.;
     W(A, W_POLD)[c] = iflip == 1 ? A.p[(long long)A.kdm * A.slice + c] : 0.;
   }
 }
@@ -375,9 +445,12 @@ __device__ __forceinline__ long long nbx(const CnuityArgs &A, long long c, long 
   return c;
 }
 
-// loop 13, :790-830 at margin 5: biharmonic smoothing operands at interface k (1-based)
-__global__ void cn_thk_util(const CnuityArgs A, int k) {
+// loop 13, :790-830 at margin 5: biharmonic smoothing operands at the
+// interfaces k = kf, kf + dir, .. (1-based) of a batch; they read only their own
+// interface, which moves after them
+__global__ void cn_thk_util(const CnuityArgs A, int kf, int dir) {
   after_previous();
+  const int l = blockIdx.z, k = kf + dir * l;
   Cell x;
   if (!cell_of(A, 5, x)) return;
   const long long c = x.c, sl = A.slice, ld = A.ld1;
@@ -404,8 +477,8 @@ __global__ void cn_thk_util(const CnuityArgs A, int k) {
       if (klt(mn(dkm[cja], dkm[cjb]), kOnecm)) u2 = 0.0;
     }
   }
-  W(A, W_U1)[c] = u1;
-  W(A, W_U2)[c] = u2;
+  WB(A, B_U1, l)[c] = u1;
+  WB(A, B_U2, l)[c] = u2;
 }
 
 // :838-900 (biharmonic) / :1030-1060 (Laplacian) at margin 4: limited
@@ -419,7 +492,7 @@ __global__ void cn_thk_util(const CnuityArgs A, int k) {
 constexpr int kTX = 32, kTY = 8;  // the block of every cnuity launch
 // BIH, IFLIP: compile-time, so that no branch of the other form is predicated in.
 template <bool BIH, bool IFLIP>
-__global__ void __launch_bounds__(kTX * kTY, 6) cn_thk_flux(const CnuityArgs A, int k) {
+__global__ void __launch_bounds__(kTX * kTY, 6) cn_thk_flux(const CnuityArgs A, int k, int l) {
   after_previous();
   __shared__ double sG[kTY + 1][kTX + 1], sH[kTY + 1][kTX + 1];
   Cell x;
@@ -437,8 +510,8 @@ __global__ void __launch_bounds__(kTX * kTY, 6) cn_thk_flux(const CnuityArgs A, 
   const uint8_t mk = in ? A.msk[c] : 0;
   double *uk1 = A.uflx + (long long)(k - 2) * sl, *uk = A.uflx + (long long)(k - 1) * sl;
   double *vk1 = A.vflx + (long long)(k - 2) * sl, *vk = A.vflx + (long long)(k - 1) * sl;
-  double *uf = W(A, W_UF), *vf = W(A, W_VF);
-  const double *pu = BIH ? W(A, W_U1) : pk, *pv = BIH ? W(A, W_U2) : pk;
+  double *uf = WB(A, B_UF, 0), *vf = WB(A, B_VF, 0);
+  const double *pu = BIH ? WB(A, B_U1, l) : pk, *pv = BIH ? WB(A, B_U2, l) : pk;
   double tu = 0, uw = 0, uc = 0, uf0 = 0, ul1 = 0, ul0 = 0, tv = 0, vs = 0, vc = 0, vf0 = 0, vl1 = 0, vl0 = 0;
   if (mk & kIU) {
     tu = A.thkdfu[c], uw = pu[c - 1], uc = pu[c], ul1 = uk1[c], ul0 = uk[c];
@@ -499,7 +572,7 @@ __global__ void cn_thk_p(const CnuityArgs A, int k) {
   const long long c = x.c, ld = A.ld1;
   if (!(A.msk[c] & kIP)) return;
   double *pk = A.p + (long long)(k - 1) * A.slice;
-  const double *uf = W(A, W_UF), *vf = W(A, W_VF);
+  const double *uf = WB(A, B_UF, 0), *vf = WB(A, B_VF, 0);
   W(A, W_POLD)[c] = pk[c];
   pk[c] = pk[c] - mul_rn((uf[c + 1] - uf[c]) + (vf[c + ld] - vf[c]), A.scp2i[c]);
 }
@@ -581,49 +654,68 @@ __global__ void cn_ra(const CnuityArgs A) {
   }
 }
 
-dim3 grid_for(const CnuityArgs &a, int M) {
-  return dim3((unsigned)((a.ii + 2 * M + kTX - 1) / kTX), (unsigned)((a.jj + 2 * M + kTY - 1) / kTY));
+dim3 grid_for(const CnuityArgs &a, int M, int layers = 1) {
+  return dim3((unsigned)((a.ii + 2 * M + kTX - 1) / kTX), (unsigned)((a.jj + 2 * M + kTY - 1) / kTY), (unsigned)layers);
 }
 
 }  // namespace
 
-size_t cnuity_work_slices() { return W_N; }
+size_t cnuity_work_slices(int nbatch) { return W_FIX + (size_t)B_N * nbatch; }
 
-cudaError_t launch_cnuity_layers(const CnuityArgs &a, int *launches, cudaStream_t s) {
+// Layers per launch of loops 76 and 77 (their layers are independent but for
+// util3 and p, which are running sums) and interfaces per launch of the
+// interface diffusion's operands: as many as 1 GiB of work slices holds.  One
+// layer a launch and as many as 8 GiB holds: 257x193x22 1361 / 696 us (1 GiB:
+// 696), 600x450x41 3737 / 2784 (2786), 1500x1100x41 16.9 / 14.9 ms (14.9),
+// 3000x2200x10 15.1 / 14.2 (14.5).
+int cnuity_batch(long long slice, int kdm) {
+  const long long n = (1LL << 30) / (B_N * 8 * slice);
+  return (int)(n < 1 ? 1 : n > kdm ? kdm : n);
+}
+
+cudaError_t launch_cnuity_layers(const CnuityArgs &a0, int *launches, cudaStream_t s) {
   const dim3 b(kTX, kTY);
+  CnuityArgs a = a0;
   int nl = 0;
   launch_after(cn_init, grid_for(a, 6), b, s, a);
   nl++;
-  for (int k = 0; k < a.kdm; k++) {  // loop 76
+  for (a.k0 = 0; a.k0 < a.kdm; a.k0 += a.nbatch) {  // loop 76
+    const int n = a.kdm - a.k0 < a.nbatch ? a.kdm - a.k0 : a.nbatch;
+    launch_after(cn_top, grid_for(a, 4), b, s, a, n);
     if (a.btrmas) {
-      launch_after(cn_flux<true>, grid_for(a, 5), b, s, a, k);
-      launch_after(cn_low<true>, grid_for(a, 4), b, s, a, k);
+      launch_after(cn_flux<true>, grid_for(a, 5, n), b, s, a);
+      launch_after(cn_low<true>, grid_for(a, 4, n), b, s, a);
     } else {
-      launch_after(cn_flux<false>, grid_for(a, 5), b, s, a, k);
-      launch_after(cn_low<false>, grid_for(a, 4), b, s, a, k);
+      launch_after(cn_flux<false>, grid_for(a, 5, n), b, s, a);
+      launch_after(cn_low<false>, grid_for(a, 4, n), b, s, a);
     }
-    launch_after(cn_ratio, grid_for(a, 4), b, s, a, k);
-    launch_after(cn_clip, grid_for(a, 3), b, s, a, k);
-    launch_after(cn_update, grid_for(a, 2), b, s, a, k, 2, a.kdm + k);
-    nl += 5;
+    launch_after(cn_ratio, grid_for(a, 4, n), b, s, a);
+    launch_after(cn_clip, grid_for(a, 3), b, s, a, n);
+    launch_after(cn_update, grid_for(a, 2, n), b, s, a, 2, a.kdm);
+    nl += 6;
   }
+  launch_after(cn_p, grid_for(a, 2), b, s, a, 2);
+  nl++;
   *launches += nl;
   return cudaGetLastError();
 }
 
-cudaError_t launch_cnuity_rest(const CnuityArgs &a, int *launches, cudaStream_t s) {
+cudaError_t launch_cnuity_rest(const CnuityArgs &a0, int *launches, cudaStream_t s) {
   const dim3 b(kTX, kTY);
+  CnuityArgs a = a0;
   int nl = 0;
   if (!a.btrmas) {
     launch_after(cn_rpb, grid_for(a, 2), b, s, a);
     nl++;
-    for (int k = 0; k < a.kdm; k++) {  // loop 77
-      launch_after(cn_btflux, grid_for(a, 1), b, s, a, k);
-      launch_after(cn_update, grid_for(a, 0), b, s, a, k, 0, -1);
+    for (a.k0 = 0; a.k0 < a.kdm; a.k0 += a.nbatch) {  // loop 77
+      const int n = a.kdm - a.k0 < a.nbatch ? a.kdm - a.k0 : a.nbatch;
+      launch_after(cn_btflux, grid_for(a, 1, n), b, s, a);
+      launch_after(cn_update, grid_for(a, 0, n), b, s, a, 0, -1);
       nl += 2;
     }
+    launch_after(cn_p, grid_for(a, 0), b, s, a, 0);
     launch_after(cn_bottom, grid_for(a, 0), b, s, a);
-    nl++;
+    nl += 2;
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -638,17 +730,18 @@ cudaError_t launch_cnuity_rest(const CnuityArgs &a, int *launches, cudaStream_t 
     launch_after(cn_thk_init, grid_for(a, 6), b, s, a, bih, iflip);
     nl++;
     const int k0 = bih ? (iflip ? a.kdm : 2) : 2, k1 = bih ? (iflip ? 2 : a.kdm) : a.kdm, dk = k1 >= k0 ? 1 : -1;
-    for (int k = k0;; k += dk) {
-      if (bih) {
-        launch_after(cn_thk_util, grid_for(a, 5), b, s, a, k);
+    const int ni = a.kdm < 2 ? 0 : (k1 - k0) * dk + 1;  // interior interfaces
+    for (int q = 0; q < ni; q++) {
+      const int k = k0 + dk * q, l = q % a.nbatch;
+      if (bih && l == 0) {
+        launch_after(cn_thk_util, grid_for(a, 5, ni - q < a.nbatch ? ni - q : a.nbatch), b, s, a, k, dk);
         nl++;
       }
-      if (!bih) launch_after(cn_thk_flux<false, false>, grid_for(a, 4), b, s, a, k);
-      else if (iflip) launch_after(cn_thk_flux<true, true>, grid_for(a, 4), b, s, a, k);
-      else launch_after(cn_thk_flux<true, false>, grid_for(a, 4), b, s, a, k);
+      if (!bih) launch_after(cn_thk_flux<false, false>, grid_for(a, 4), b, s, a, k, l);
+      else if (iflip) launch_after(cn_thk_flux<true, true>, grid_for(a, 4), b, s, a, k, l);
+      else launch_after(cn_thk_flux<true, false>, grid_for(a, 4), b, s, a, k, l);
       launch_after(cn_thk_p, grid_for(a, 4), b, s, a, k);
       nl += 2;
-      if (k == k1) break;
     }
     launch_after(cn_thk_final, grid_for(a, 4), b, s, a);
     nl++;

@@ -1291,7 +1291,8 @@ int hyc_cnuity(hyc_ctx *c, int32_t m, int32_t n, const hyc_cnuity_params *p, dou
     return rc;
   DeviceGuard g(c->device);
   cudaStream_t s = c->stream;
-  const size_t nw = hyc::cnuity_work_slices();
+  const int nbatch = hyc::cnuity_batch(sl, kk);
+  const size_t nw = hyc::cnuity_work_slices(nbatch);
   if (!c->d_cnw) {
     CK(cudaMalloc(&c->d_cnw, nw * sl * sizeof(double)), "malloc cnuity work");
     CK(cudaMemsetAsync(c->d_cnw, 0, nw * sl * sizeof(double), s), "cnuity work");
@@ -1363,6 +1364,7 @@ int hyc_cnuity(hyc_ctx *c, int32_t m, int32_t n, const hyc_cnuity_params *p, dou
   a.dtinv = 1. / p->delt1;  // cnuity.F90:758, :987 (the same IEEE quotient as on the device)
   a.ra2fac = p->ra2fac;
   a.w = c->d_cnw;
+  a.nbatch = nbatch;
   a.keys = want_keys ? c->d_cnkeys : nullptr;
   int nl = 0;
   CK(hyc::launch_cnuity_layers(a, &nl, s), "cnuity loop 76");
