@@ -80,7 +80,7 @@ static cudaError_t launch_march_one(const TileArgs &a, int nlayers, cudaStream_t
   const int resident = nsm * std::min<int>(228 * 1024 / (G::smem_bytes + 1024), 512 / (NT * NG));
   int nrow = 0;
   long long best = LLONG_MAX;
-  for (int r = 4; r <= 256; r += r < 32 ? 1 : 4) {
+  for (int r = 4; r <= 512; r += r < 32 ? 1 : 4) {
     if ((a.jj + r - 1) / r > 65535) continue;
     const long long cost = ((per * ((a.jj + r - 1) / r) + resident - 1) / resident) * (r + 7);
     if (cost < best) best = cost, nrow = r;
