@@ -81,3 +81,32 @@ def test_one_field_slice(cuda, advtyp):
     g.advem(advtyp, ref, fldc, u, v, fco, fcn, 0.0, c["scp2"], c["scp2i"], 600.0)
     make_ctx(b, g, 1).advem(advtyp, got, fldc, u, v, fco, fcn, 0.0, c["scp2"], c["scp2i"], 600.0)
     assert same(got, ref) and not np.array_equal(got, fld)
+
+
+@pytest.mark.parametrize("advtyp", [0, 1, 2, 4])
+@pytest.mark.parametrize("mode", ["hybrid", "isopycnic", "conserve"])
+def test_field_lists(cuda, advtyp, mode):
+    """Fields with layer ranges of their own: th3d above nhybrd, q2/q2l with a
+    layer offset, the isopycnic layer 1; and the conserving rescale."""
+    b = basin(83, 61, True, seed=131)
+    g = oracle_grid(b)
+    kdm = 28
+    c = np_case(b, g, kdm=kdm, ntracr=2, seed=131, courant=0.7, delt1=600.0)
+    c["delt1"] = 600.0
+    kw = {"hybrid": dict(advflg=1, nhybrd=11, mxlmy=True), "isopycnic": dict(isopyc=True, nhybrd=0, mxlmy=True),
+          "conserve": {}}[mode]
+    q2 = {}
+    if kw:
+        rng = np.random.default_rng(131)
+        q2 = dict(q2=0.01 + rng.random((2, kdm + 2, b.ld2, b.ld1)) * 0.1, q2l=0.1 + rng.random((2, kdm + 2, b.ld2, b.ld1)))
+    c.update(q2)
+    t = torchify(c, cuda)
+    ctx = make_ctx(b, g, kdm)
+    bind_all(ctx, t, extra=tuple(q2))
+    flg = np.array([0, 2], np.int32)
+    if mode == "conserve":
+        ctx.set_conserve(True)
+        g.set_conserve(True)
+    oracle_steps(g, c, (1, 2), advtyp, trcflg=flg, **q2, **kw)
+    gpu_steps(ctx, t, (1, 2), advtyp, ntracr=2, trcflg=flg, **kw)
+    compare(c, t, keys=("temp", "saln", "th3d", "tracer") + tuple(q2))
