@@ -74,7 +74,8 @@ struct hyc_ens {
   int4 *d_items = nullptr;  // the main launch's items, then the one-tracer launch's
   int nitems = 0, nitems_t = 0;
   int items_nq = 0;         // tracers per pass the strip items were built for
-  int kchunk = 1;  // strip kernel: layers per work item
+  int kchunk = 1;      // mixed strip kernel: layers per work item
+  int march_rows = 1;  // FP64 strip kernel: most rows per segment
   int items_tx = 0, items_ty = 0, items_layers = -1;
   int *d_head = nullptr;  // two queue counters per step slot (main and one-tracer launch)
   int nhead = 0;
@@ -257,17 +258,32 @@ int col2_kchunk(const hyc_ens *e) {
   return (int)std::max(1LL, std::min(8LL, kc));
 }
 
-// FP64 FCT strip kernel: strips of a basin and rows per segment.  About 12
-// work items per resident CTA over the ensemble, so that the queue's last wave
-// is short, in segments of 24 rows (7 more are recomputed) to 400 (to 192:
-// six basins, three steps 96.6 ms against 95.6).
+// FP64 FCT strip kernel: strips of a basin and rows per segment.  About eight
+// work items per resident CTA (four an SM) over the ensemble, so that the
+// queue's last wave is short, in segments of 24 rows (7 more are recomputed) to
+// 400; where that leaves CTAs idle, the shortest segments, from 6 rows on, that
+// still make one wave.  One step with a get: 150x100x10, two tracers, 185 us
+// with 24 rows, 110 with 6; four basins of 300x200x22, five tracers, 1.69 ms with
+// twelve items a CTA, 1.66 with eight; 700x500x22, three tracers, 2.57 and 2.52.
 int march_strips(const EBasin &b) { return (b.idm + hyc::kMarchCols - 7) / (hyc::kMarchCols - 6); }
+int march_rows(const hyc_ens *e) {
+  const long long resident = 4LL * e->nsm;
+  auto items = [&](int rows) {
+    long long n = 0;
+    for (const auto &x : e->b)
+      n += (long long)march_strips(x) * ((x.jdm + rows - 1) / rows) * x.kdm *
+           ((x.ntr + hyc::kMarchFields - 1) / hyc::kMarchFields);
+    return n;
+  };
+  int rows = 24;
+  if (items(rows) < resident) {
+    while (rows > 6 && items(rows - 1) <= resident) rows--;
+    return rows;
+  }
+  return (int)std::max(24LL, std::min(400LL, items(1) / (8 * resident)));
+}
 int march_seg(const hyc_ens *e, const EBasin &b) {
-  long long rows = 0;
-  for (const auto &x : e->b)
-    rows += (long long)march_strips(x) * x.jdm * x.kdm * ((x.ntr + hyc::kMarchFields - 1) / hyc::kMarchFields);
-  const long long want = std::max(24LL, std::min(400LL, rows / (12LL * e->nsm * 4)));
-  const int nseg = (int)((b.jdm + want - 1) / want);
+  const int nseg = (b.jdm + e->march_rows - 1) / e->march_rows;
   return (b.jdm + nseg - 1) / nseg;
 }
 
@@ -422,6 +438,7 @@ int build_items(hyc_ens *e) {
   };
   std::vector<W> w, wt;  // main launch, one-tracer launch
   if (is_col2(e->shape)) e->kchunk = col2_kchunk(e);
+  else e->march_rows = march_rows(e);
   for (int i = 0; i < (int)e->b.size(); i++) {
     const EBasin &b = e->b[i];
     if (is_col2(e->shape)) {  // (basin, 56-column strip, segment, chunk of layers), all tracers
@@ -802,8 +819,7 @@ static int move(hyc_ens *e, int32_t basin, int32_t what, int32_t s0, int32_t ns_
     return HYC_OK;
   }
   // get into this device's memory: one kernel on the ensemble's stream
-  // (staging and copying it out would move every value three times); the copy
-  // stream's event follows it, so that waiting works as for a copy
+  // (staging and copying it out would move every value three times)
   bool direct = where == HYC_DEVICE && ((uintptr_t)host & 7) == 0;  // a copy needs no alignment, nor its own device
   if (direct) {
     cudaPointerAttributes pa;
@@ -820,13 +836,10 @@ static int move(hyc_ens *e, int32_t basin, int32_t what, int32_t s0, int32_t ns_
     if (c != cudaSuccess) return efail(e, HYC_ERR_CUDA, "get: %s", cudaGetErrorString(c));
     span_close(e, t1, HYC_T_XCTILR, e->stream);
     ECK(cudaEventRecord(e->ev_staged, e->stream), "event");
-    ECK(cudaStreamWaitEvent(e->copy_stream, e->ev_staged, 0), "wait staged");
-    ECK(cudaEventRecord(e->ev_gdone, e->copy_stream), "event");
-    e->get_pending = true;
-    if (!async_get) {
-      ECK(cudaEventSynchronize(e->ev_gdone), "get sync");
-      e->get_pending = false;
-    }
+    if (async_get)  // hyc_ens_wait waits for the copy stream
+      ECK(cudaStreamWaitEvent(e->copy_stream, e->ev_staged, 0), "wait staged");
+    else
+      ECK(cudaEventSynchronize(e->ev_staged), "get sync");
     return HYC_OK;
   }
   // get: repitch into the get staging on the ensemble's stream (after any
