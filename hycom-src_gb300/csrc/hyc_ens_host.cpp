@@ -150,6 +150,13 @@ size_t esz(const hyc_ens *e) { return e->prec == HYC_PREC_MIXED ? 4 : 8; }
 bool is_col2(hyc::TileShape t) { return t.tx == hyc::kCol2Strip; }
 constexpr int kMaps = 8;  // strip kernel maps per basin
 
+// The recorded steps hold the addresses of the queue and its counters: they go
+// wherever one of these is replaced, and with every option they were recorded under.
+void drop_graph(hyc_ens *e) {
+  if (e->gexec) cudaGraphExecDestroy(e->gexec);
+  e->gexec = nullptr;
+}
+
 void free_all(hyc_ens *e) {
   for (auto &b : e->b) {
     cudaFree(b.msk);
@@ -186,7 +193,7 @@ void free_all(hyc_ens *e) {
   cudaFree(e->d_cmaps);
   cudaFree(e->d_fmaps);
   cudaFree(e->d_err);
-  if (e->gexec) cudaGraphExecDestroy(e->gexec);
+  drop_graph(e);
   for (auto &p : e->pending) {
     cudaEventDestroy(p.a);
     cudaEventDestroy(p.z);
@@ -475,6 +482,7 @@ int build_items(hyc_ens *e) {
   it.reserve(w.size() + wt.size());
   for (const auto &x : w) it.push_back(x.it);
   for (const auto &x : wt) it.push_back(x.it);
+  drop_graph(e);
   cudaFree(e->d_items);
   e->d_items = nullptr;
   ECK(cudaMalloc(&e->d_items, std::max<size_t>(1, it.size()) * sizeof(int4)), "items");
@@ -490,8 +498,11 @@ int build_items(hyc_ens *e) {
 
 int ensure_heads(hyc_ens *e, int n) {
   if (e->nhead >= n) return HYC_OK;
+  ECK(cudaStreamSynchronize(e->stream), "queue heads sync");  // steps in flight count in them
+  drop_graph(e);
   cudaFree(e->d_head);
   e->d_head = nullptr;
+  e->nhead = 0;
   ECK(cudaMalloc(&e->d_head, 2 * n * sizeof(int)), "queue heads");
   e->nhead = n;
   return HYC_OK;
@@ -698,10 +709,7 @@ int hyc_ens_set_stream(hyc_ens *e, void *stream) {
   }
   e->stream = (cudaStream_t)stream;
   e->own_stream = false;
-  if (e->gexec) {
-    cudaGraphExecDestroy(e->gexec);
-    e->gexec = nullptr;
-  }
+  drop_graph(e);
   return HYC_OK;
 }
 
@@ -923,10 +931,7 @@ int hyc_ens_set_tile(hyc_ens *e, int32_t tx, int32_t ty) {
   if (t.tx != e->shape.tx || t.ty != e->shape.ty) {
     e->shape = t;
     e->tbl_dt2 = -1.0;
-    if (e->gexec) {
-      cudaGraphExecDestroy(e->gexec);
-      e->gexec = nullptr;
-    }
+    drop_graph(e);
   }
   return HYC_OK;
 }
@@ -935,20 +940,14 @@ int hyc_ens_set_option(hyc_ens *e, int32_t option, int32_t value) {
   if (!e) return efail(nullptr, HYC_ERR_ARG, "null ensemble");
   if (option == HYC_OPT_PREP64) {
     if (e->prec != HYC_PREC_MIXED) return efail(e, HYC_ERR_ARG, "HYC_OPT_PREP64 applies to the mixed form");
-    if (e->prep64 != (value != 0) && e->gexec) {
-      cudaGraphExecDestroy(e->gexec);
-      e->gexec = nullptr;
-    }
+    if (e->prep64 != (value != 0)) drop_graph(e);
     e->prep64 = value != 0;
     return HYC_OK;
   }
   if (option == HYC_OPT_STRIP_TRACERS) {
     if (e->prec != HYC_PREC_MIXED || value < 1 || value > 2)
       return efail(e, HYC_ERR_ARG, "HYC_OPT_STRIP_TRACERS: 1 or 2, mixed form");
-    if (e->strip_nq != value && e->gexec) {
-      cudaGraphExecDestroy(e->gexec);
-      e->gexec = nullptr;
-    }
+    if (e->strip_nq != value) drop_graph(e);
     e->strip_nq = value;
     return HYC_OK;
   }
@@ -963,10 +962,7 @@ int hyc_ens_set_posdef(hyc_ens *e, int32_t basin, int32_t tracer, double posdef)
     if (e->stream) cudaStreamSynchronize(e->stream);  // steps in flight read the tables
     e->b[basin].posdef[tracer] = posdef;
     e->tbl_dt2 = -1.0;
-    if (e->gexec) {
-      cudaGraphExecDestroy(e->gexec);
-      e->gexec = nullptr;
-    }
+    drop_graph(e);
   }
   return HYC_OK;
 }
@@ -1026,10 +1022,7 @@ int hyc_ens_set_diffusion(hyc_ens *e, int32_t basin, double temdf2, const double
     int rc = encode_strip_maps(e);
     if (rc) return rc;
     e->tbl_dt2 = -1.0;
-    if (e->gexec) {
-      cudaGraphExecDestroy(e->gexec);
-      e->gexec = nullptr;
-    }
+    drop_graph(e);
   }
   return HYC_OK;
 }
@@ -1100,10 +1093,7 @@ int hyc_ens_step(hyc_ens *e, int32_t advtyp, double delt1, int32_t nsteps, int32
     const bool reuse = e->gexec && e->g_nsteps == nsteps && e->g_advtyp == advtyp && e->g_dt == delt1 &&
                        e->g_rot == e->rot && e->g_tx == e->shape.tx && e->g_ty == e->shape.ty;
     if (!reuse) {
-      if (e->gexec) {
-        cudaGraphExecDestroy(e->gexec);
-        e->gexec = nullptr;
-      }
+      drop_graph(e);
       // recorded on a private stream (the caller's may be the legacy default
       // stream, which cannot be captured), launched on the caller's stream
       if (!e->cap_stream) ECK(cudaStreamCreateWithFlags(&e->cap_stream, cudaStreamNonBlocking), "capture stream");
@@ -1206,10 +1196,7 @@ int hyc_ens_tune(hyc_ens *e, int32_t advtyp, double delt1, int32_t *tx, int32_t 
   e->strip_nq = is_col2(best) ? best_nq : keep_nq;
   e->tbl_dt2 = -1.0;
   e->items_tx = 0;  // force the queue for the chosen shape
-  if (e->gexec) {
-    cudaGraphExecDestroy(e->gexec);
-    e->gexec = nullptr;
-  }
+  drop_graph(e);
   if (tx) *tx = best.tx;
   if (ty) *ty = best.ty;
   if (ms_out) *ms_out = best_ms;
