@@ -64,6 +64,7 @@ struct hyc_ctx {
   double *d_cngrid = nullptr;   // scuy, scvx, depthu, depthv, thkdfu, thkdfv (6 slices), hyc_set_cnuity_grid
   bool cn_thkdf = false;        // thkdfu/thkdfv were given
   double *d_cnw = nullptr;      // cnuity work slices
+  int cn_batch = 0;             // layers per launch that they hold
   long long *d_cnkeys = nullptr;  // cnuity dpkmin keys (2*kdm)
   Field fields[HYC_NFIELDS];
   double *d_scratch = nullptr;  // advem output slices (fields x layers)
@@ -180,6 +181,29 @@ void fct2c_bind(hyc::Fct2cArgs &f, const hyc_ctx *c, int npair) {
   f.npair = npair;
   f.work = (double *)c->d_fct2c;
   f.lcalc = c->d_fct2c + (size_t)npair * hyc::fct2c_work_doubles(c->slice) * sizeof(double);
+}
+
+// cnuity's work slices, kept by the context: those of as many layers a launch
+// as cnuity_batch asks for, if they are no more than a sixteenth of the free
+// memory (other contexts and the caller's arrays come after this one) and can
+// be had; else of fewer, down to one layer, which costs 13 % at 1500x1100x41
+// and twice the time at 257x193x22 (hyc_cnuity.cu).
+int ensure_cnuity(hyc_ctx *c) {
+  if (c->d_cnw) return HYC_OK;
+  auto bytes = [&](int n) { return hyc::cnuity_work_slices(n) * (size_t)c->slice * sizeof(double); };
+  int n = hyc::cnuity_batch(c->slice, c->kdm);
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess)
+    while (n > 1 && bytes(n) > free_bytes / 16) n--;
+  while (cudaMalloc(&c->d_cnw, bytes(n)) != cudaSuccess) {
+    c->d_cnw = nullptr;
+    cudaGetLastError();  // or the next launch would report it
+    if (n == 1) return fail(c, HYC_ERR_NOMEM, "cannot allocate %zu bytes of cnuity work slices", bytes(1));
+    n /= 2;
+  }
+  c->cn_batch = n;
+  CK(cudaMemsetAsync(c->d_cnw, 0, bytes(n), c->stream), "cnuity work");
+  return HYC_OK;
 }
 
 // TMA maps of the FCT tile kernel for the launches of one call (box TX+8 x
@@ -1291,12 +1315,7 @@ int hyc_cnuity(hyc_ctx *c, int32_t m, int32_t n, const hyc_cnuity_params *p, dou
     return rc;
   DeviceGuard g(c->device);
   cudaStream_t s = c->stream;
-  const int nbatch = hyc::cnuity_batch(sl, kk);
-  const size_t nw = hyc::cnuity_work_slices(nbatch);
-  if (!c->d_cnw) {
-    CK(cudaMalloc(&c->d_cnw, nw * sl * sizeof(double)), "malloc cnuity work");
-    CK(cudaMemsetAsync(c->d_cnw, 0, nw * sl * sizeof(double), s), "cnuity work");
-  }
+  if ((rc = ensure_cnuity(c))) return rc;
   const bool want_keys = dpkmin || p->nstep % 3 == 0;
   if (want_keys) {
     if (!c->d_cnkeys) CK(cudaMalloc(&c->d_cnkeys, 2 * kk * sizeof(long long)), "malloc keys");
@@ -1364,7 +1383,7 @@ int hyc_cnuity(hyc_ctx *c, int32_t m, int32_t n, const hyc_cnuity_params *p, dou
   a.dtinv = 1. / p->delt1;  // cnuity.F90:758, :987 (the same IEEE quotient as on the device)
   a.ra2fac = p->ra2fac;
   a.w = c->d_cnw;
-  a.nbatch = nbatch;
+  a.nbatch = c->cn_batch;
   a.keys = want_keys ? c->d_cnkeys : nullptr;
   int nl = 0;
   CK(hyc::launch_cnuity_layers(a, &nl, s), "cnuity loop 76");

@@ -63,7 +63,7 @@ cudaError_t launch_asselin(const AsselinArgs &a, bool filter, cudaStream_t s);
 
 // Continuity equation: work slices, loop 76 (all layers), then the rest
 struct CnuityArgs;
-int cnuity_batch(long long slice, int kdm);  // layers per launch
+int cnuity_batch(long long slice, int kdm);  // layers per launch, where memory is plenty
 size_t cnuity_work_slices(int nbatch);
 cudaError_t launch_cnuity_layers(const CnuityArgs &a, int *launches, cudaStream_t s);
 cudaError_t launch_cnuity_rest(const CnuityArgs &a, int *launches, cudaStream_t s);

@@ -12,6 +12,7 @@ namespace {
 
 std::map<const char *, size_t> live;  // base -> bytes
 size_t in_use = 0, limit = (size_t)1 << 40;
+bool hidden = false;
 int dead = 0, ncapture = 0, nlaunch = 0;
 cudaError_t last = cudaSuccess;
 cudaStream_t capturing = nullptr;
@@ -41,6 +42,7 @@ T handle() {
 
 namespace fake {
 void set_free_bytes(size_t n) { limit = in_use + n; }
+void hide_free(bool on) { hidden = on; }
 size_t bytes_in_use() { return in_use; }
 int dead_uses() { return dead; }
 int captures() { return ncapture; }
@@ -71,7 +73,7 @@ cudaError_t cudaFree(void *p) {  // the memory stays: a dead pointer is never ha
   return cudaSuccess;
 }
 cudaError_t cudaMemGetInfo(size_t *f, size_t *t) {
-  *f = limit - in_use;
+  *f = hidden ? (size_t)1 << 40 : limit - in_use;
   *t = limit;
   return cudaSuccess;
 }

@@ -11,6 +11,8 @@ namespace fake {
 
 // device bytes that may be allocated from now on, beyond those in use
 void set_free_bytes(size_t n);
+// cudaMemGetInfo reports far more than that
+void hide_free(bool on);
 size_t bytes_in_use();
 // uses of pointers into freed or unknown memory
 int dead_uses();
