@@ -155,7 +155,7 @@ size_t advect_tiles_smem(TileShape t) {
 // CTA an SM, keeps the small tiles up to where its strip kernel takes over
 // (551 tiles: 116 -> 111 us).
 TilePlan tile_plan(int scheme, const TileArgs &a, int nlayers, TileShape shape, bool fixed) {
-  if (march_takes(scheme, a, nlayers)) return {shape, false};
+  if (!fixed && march_takes(scheme, a, nlayers)) return {shape, false, true};
   bool tma = true;
   if (!fixed) {
     int dev = 0, nsm = 0;
@@ -165,11 +165,12 @@ TilePlan tile_plan(int scheme, const TileArgs &a, int nlayers, TileShape shape, 
     if (tiles <= (scheme == kMPDATA ? 4LL : 1LL) * nsm) shape = TileShape{16, 16};
     tma = tiles > nsm;
   }
-  return {shape, tma && advect_tiles_tma(scheme, shape)};
+  return {shape, tma && advect_tiles_tma(scheme, shape), false};
 }
 
-cudaError_t launch_advect_tiles(int scheme, const TileArgs &a, int nlayers, TileShape t, cudaStream_t s) {
-  if (march_takes(scheme, a, nlayers)) return launch_march(scheme, a, nlayers, s);
+cudaError_t launch_advect_tiles(int scheme, const TileArgs &a, int nlayers, TileShape t, cudaStream_t s,
+                                bool fixed) {
+  if (!fixed && march_takes(scheme, a, nlayers)) return launch_march(scheme, a, nlayers, s);
   if (t.tx == 32 && t.ty == 16) return launch_shape<32, 16>(scheme, a, nlayers, s);
   if (t.tx == 32 && t.ty == 32) return launch_shape<32, 32>(scheme, a, nlayers, s);
   if (t.tx == 16 && t.ty == 16) return launch_shape<16, 16>(scheme, a, nlayers, s);

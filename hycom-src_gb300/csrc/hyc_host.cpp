@@ -141,7 +141,8 @@ const int kMbdy[5] = {2, 5, 5, 0, 5};  // mbdy_advtyp, mod_tsadvc.F90:24-29
 
 bool valid_advtyp(int a) { return a == 0 || a == 1 || a == 2 || a == 4; }
 
-// the tile shape HYC_TILE asks for, if it does
+// the tile shape HYC_TILE asks for, if it does: 16x16, 32x16 or 32x32.  Every
+// launch of a context created under it takes the tile kernel of that shape.
 bool env_shape(hyc::TileShape &shape) {
   const char *s = getenv("HYC_TILE");
   hyc::TileShape t{0, 0};
@@ -770,7 +771,7 @@ int hyc_advem(hyc_ctx *c, int32_t advtyp, double *fld, const double *fldc, const
   }
   {
     Timed t(c, HYC_T_ADVECT);
-    CK(hyc::launch_advect_tiles(advtyp, a, 1, tp.shape, c->stream), "advem kernel");
+    CK(hyc::launch_advect_tiles(advtyp, a, 1, tp.shape, c->stream, c->shape_fixed), "advem kernel");
   }
   if (c->lconserve && (rc = conserve(c, a, 1))) return rc;
   CK(hyc::launch_copy_back(a, 1, c->stream), "advem copy");
@@ -1014,7 +1015,7 @@ int hyc_tsadvc(hyc_ctx *c, int32_t m, int32_t n, const hyc_tsadvc_params *p, dou
     }
     {
       Timed t(c, HYC_T_ADVECT);
-      CK(hyc::launch_advect_tiles(at, L.a, L.nlay, L.plan.shape, s), "advect kernel");
+      CK(hyc::launch_advect_tiles(at, L.a, L.nlay, L.plan.shape, s, c->shape_fixed), "advect kernel");
       int rc2;
       if (c->lconserve && (rc2 = conserve(c, L.a, L.nlay))) return rc2;
     }

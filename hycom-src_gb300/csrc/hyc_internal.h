@@ -18,20 +18,23 @@ struct TileShape {
   int tx, ty;
 };
 
-// Fused advem/tsadvc tile kernel; scheme in {0,1,2,4}.  out receives every
-// interior cell of each (field, layer) slice it processes.
+// Fused advem/tsadvc kernel, strip or tile; scheme in {0,1,2,4}.  out receives
+// the interior sea cells of each (field, layer) slice it processes, and with
+// PCM and MPDATA the old value of its land cells.  fixed: the tile kernel of
+// this shape, whatever the size.
 cudaError_t launch_advect_tiles(int scheme, const TileArgs &a, int nlayers, TileShape shape,
-                                cudaStream_t s);
+                                cudaStream_t s, bool fixed = false);
 size_t advect_tiles_smem(TileShape shape);
 // the tile kernel of this scheme and shape stages its region by TMA when
 // the launch carries tensor maps (box (tx+8) x (ty+6), see TileArgs::tmaps)
 bool advect_tiles_tma(int scheme, TileShape shape);
-// the launch goes to a strip kernel (hyc_march.cuh), which takes no tensor maps
+// a launch of no fixed shape goes to a strip kernel (hyc_march.cuh), which takes no tensor maps
 bool march_takes(int scheme, const TileArgs &a, int nlayers);
-// tile shape of a launch (fixed: the one given) and whether it takes tensor maps
+// a launch's kernel: a strip kernel, or the tile kernel of a shape (fixed: the
+// one given) that takes tensor maps or not
 struct TilePlan {
   TileShape shape;
-  bool tma;
+  bool tma, strip;
 };
 TilePlan tile_plan(int scheme, const TileArgs &a, int nlayers, TileShape shape, bool fixed);
 bool advect_tile_shape_ok(TileShape shape);

@@ -133,6 +133,10 @@ int hyc_bigrid(int32_t idm, int32_t jdm, int32_t nbdy, double *depth, int32_t *i
  * are copied to the device and stay resident.  Replaces the module state
  * that tsadvc reads through `use mod_dimensions, mod_cb_arrays`
  * (mod_tsadvc.F90:15, :1709).
+ * The environment variable HYC_TILE (16x16, 32x16 or 32x32), read here,
+ * fixes the advection kernels of the context: the tile kernels in that
+ * shape at every size.  Unset, the size of a launch chooses.  The results
+ * are the same bits.
  */
 int hyc_adv_init(hyc_ctx **ctx, int32_t idm, int32_t jdm, int32_t kdm, int32_t nbdy, int32_t nreg,
                  const int32_t *ip, const int32_t *iu, const int32_t *iv, const double *scp2,
