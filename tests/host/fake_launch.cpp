@@ -33,7 +33,7 @@ cudaError_t launch_mix_col2(int, const MixBasin *basins, const int4 *items, int,
   for (const void *p : {(const void *)basins, (const void *)items, (const void *)head, (const void *)err}) fake::use(p, s);
   return cudaSuccess;
 }
-cudaError_t launch_advect_tiles(int, const TileArgs &a, int, TileShape, cudaStream_t s) {
+cudaError_t launch_advect_tiles(int, const TileArgs &a, int, TileShape, cudaStream_t s, bool) {
   if (fake_fail_launches > 0 && --fake_fail_launches == 0) return cudaErrorInvalidValue;
   fake::use(a.out, s);
   return cudaSuccess;
