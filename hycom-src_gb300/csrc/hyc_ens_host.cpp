@@ -60,7 +60,7 @@ struct hyc_ens {
   int strip_nq = 2;      // strip kernel: tracers per pass (1 or 2)
   bool diff = false;     // some basin diffuses its tracers after each step (mixed form)
   CUtensorMap *d_cmaps = nullptr;  // [nbasin][kMaps]: strip kernel maps (levels 0-2, u, v, dp, cell words)
-  CUtensorMap *d_fmaps = nullptr;  // FP64 form: the FCT tile kernel's maps, 3 rotations x basins
+  CUtensorMap *d_fmaps = nullptr;  // FP64 MPDATA on basins of the tile kernel: its maps, 3 rotations x basins
   size_t fmaps_cap = 0;
   int *d_err = nullptr;            // device error flag (bounded waits that gave up)
   // device tables, one per rotation
@@ -69,8 +69,9 @@ struct hyc_ens {
   // count's last tracer when the main launch takes the tracers in pairs
   MixBasin *d_mixt[3] = {nullptr, nullptr, nullptr};
   TileArgs *d_targs[3] = {nullptr, nullptr, nullptr};
-  std::vector<TileArgs> h_targs[3];  // host copies (FP64 PCM/MPDATA run the plain tile kernel per basin)
+  std::vector<TileArgs> h_targs[3];  // host copies (FP64 PCM/MPDATA run the plain form's kernels per basin)
   double tbl_dt2 = -1.0;
+  bool tbl_maps = false;  // the tables point to tensor maps
   int4 *d_items = nullptr;  // the main launch's items, then the one-tracer launch's
   int nitems = 0, nitems_t = 0;
   int items_nq = 0;         // tracers per pass the strip items were built for
@@ -294,9 +295,26 @@ int march_seg(const hyc_ens *e, const EBasin &b) {
   return (b.jdm + nseg - 1) / nseg;
 }
 
+// Some launch of this scheme goes to a tile kernel, which has a shape and takes
+// tensor maps: FP64 PCM and MPDATA on basins that the strip kernels leave.
+// FP64 FCT2 and FCT4 have the strip kernel's queue at every size.
+bool takes_tiles(const hyc_ens *e, int advtyp) {
+  if (e->prec == HYC_PREC_MIXED || advtyp >= 2) return false;
+  for (const auto &b : e->b) {
+    TileArgs a;
+    memset(&a, 0, sizeof a);
+    a.ii = b.idm;
+    a.jj = b.jdm;
+    a.nfld = b.ntr;
+    if (!hyc::march_takes(advtyp, a, b.kdm)) return true;
+  }
+  return false;
+}
+
 // device tables for the three rotations (rebuilt when delt1 changes)
-int build_tables(hyc_ens *e, double dt2) {
-  if (e->tbl_dt2 == dt2) return HYC_OK;
+int build_tables(hyc_ens *e, double dt2, int advtyp) {
+  const bool maps = takes_tiles(e, advtyp);
+  if (e->tbl_dt2 == dt2 && (e->tbl_maps || !maps)) return HYC_OK;
   ECK(cudaStreamSynchronize(e->stream), "tables sync");  // earlier steps may still read the tables
   const int nb = (int)e->b.size();
   if (e->prec == HYC_PREC_MIXED)
@@ -376,9 +394,9 @@ int build_tables(hyc_ens *e, double dt2) {
         a.kdm = b.kdm;
         a.images = b.nreg == 1 ? std::min(5, b.nbdy) : 0;
       }
-      // TMA maps of the FCT tile kernel (box tx+8 x ty+6): uflx, vflx, dp,
+      // TMA maps of the tile kernel (box tx+8 x ty+6): uflx, vflx, dp,
       // (no onetamas), scp2, scp2i, then levels t-1 and t of each tracer
-      if (r == 0) {
+      if (maps && r == 0) {
         size_t need = 0;
         for (const auto &b : e->b) need += 3 * (6 + 2 * (size_t)b.ntr);
         if (e->fmaps_cap < need) {
@@ -389,7 +407,7 @@ int build_tables(hyc_ens *e, double dt2) {
           e->fmaps_cap = need;
         }
       }
-      {
+      if (maps) {
         std::vector<CUtensorMap> h;
         size_t base = 0;  // the rotations' maps one after another
         for (int rr = 0; rr < r; rr++)
@@ -429,6 +447,7 @@ int build_tables(hyc_ens *e, double dt2) {
     }
   }
   e->tbl_dt2 = dt2;
+  e->tbl_maps = maps;
   return HYC_OK;
 }
 
@@ -535,7 +554,7 @@ int enqueue_step(hyc_ens *e, int advtyp, int r, int h, cudaStream_t st) {
       launches = (e->nitems > 0) + 1;
     }
   } else if (e->prec != HYC_PREC_MIXED && (advtyp == 0 || advtyp == 1)) {
-    // FP64 PCM/MPDATA: the plain form's tile kernel per basin, then the periodic halo
+    // FP64 PCM/MPDATA: the plain form's kernels per basin, then the periodic halo
     c = cudaSuccess;
     for (size_t i = 0; i < e->b.size() && c == cudaSuccess; i++) {
       const EBasin &b = e->b[i];
@@ -552,8 +571,8 @@ int enqueue_step(hyc_ens *e, int advtyp, int r, int h, cudaStream_t st) {
   return HYC_OK;
 }
 
-// Schemes per form and kernel: FP64 FCT2/FCT4 (queue kernel) and PCM/MPDATA
-// (plain tile kernel); FP32-mixed FCT2, FCT4 and MPDATA (strip kernel).
+// Schemes per form and kernel: FP64 FCT2/FCT4 (the strip kernel's queue) and
+// PCM/MPDATA (strip or tile kernel, basin by basin); FP32-mixed FCT2, FCT4 and MPDATA (strip kernel).
 bool scheme_ok(const hyc_ens *e, int advtyp) {
   if (e->prec == HYC_PREC_MIXED) return advtyp == 1 || advtyp == 2 || advtyp == 4;
   return advtyp == 0 || advtyp == 1 || advtyp == 2 || advtyp == 4;
@@ -1076,7 +1095,7 @@ int hyc_ens_step(hyc_ens *e, int32_t advtyp, double delt1, int32_t nsteps, int32
   Dev g(e->device);
   int rc;
   if ((rc = build_items(e)) ||
-      (rc = build_tables(e, delt1)) || (rc = ensure_heads(e, nsteps)) || (rc = prime(e)))
+      (rc = build_tables(e, delt1, advtyp)) || (rc = ensure_heads(e, nsteps)) || (rc = prime(e)))
     return rc;
   cudaEvent_t a = nullptr, z = nullptr;
   if (e->timing) {
@@ -1153,6 +1172,8 @@ int hyc_ens_tune(hyc_ens *e, int32_t advtyp, double delt1, int32_t *tx, int32_t 
   std::vector<std::pair<hyc::TileShape, int>> trials;
   for (const auto &c : cands) {
     if (!shape_ok(e, c) || !scheme_ok(e, advtyp)) continue;
+    // where no kernel has a shape there is one trial, of the shape as it is
+    if (e->prec != HYC_PREC_MIXED && !takes_tiles(e, advtyp) && (c.tx != keep.tx || c.ty != keep.ty)) continue;
     if (is_col2(c) && e->maxntr > 1) trials.push_back({c, 1});
     trials.push_back({c, 2});
   }
@@ -1162,7 +1183,7 @@ int hyc_ens_tune(hyc_ens *e, int32_t advtyp, double delt1, int32_t *tx, int32_t 
     e->shape = c;
     e->tbl_dt2 = -1.0;
     if ((rc = build_items(e)) ||
-        (rc = build_tables(e, delt1)) || (rc = ensure_heads(e, 1)))
+        (rc = build_tables(e, delt1, advtyp)) || (rc = ensure_heads(e, 1)))
       break;
     // the step kernel writes only the spare level: the state is unchanged
     if ((rc = enqueue_step(e, advtyp, e->rot, 0, e->stream))) break;  // warm-up

@@ -444,12 +444,16 @@ int hyc_ens_get_slices(hyc_ens *ens, int32_t basin, int32_t what, int32_t s0, in
 /* Tile shape of the step kernel; hyc_ens_tune picks one.  Mixed form:
  * tx = 56, the strip kernel (64-column strips streamed by TMA, 56 columns
  * updated), ty = rows per segment, 32 to 2048 (powers of 2).  FP64 form: 32 x 16
- * or 16 x 16 cell tiles. */
+ * or 16 x 16 cell tiles, of the tile kernel that advances small basins with
+ * MPDATA; the FP64 strip kernels (FCT2, FCT4, PCM, larger basins with MPDATA)
+ * have no tile shape, and take it without effect. */
 int hyc_ens_set_tile(hyc_ens *ens, int32_t tx, int32_t ty);
 /*
  * Autotuner: time every supported tile shape on this ensemble (the kernel
  * writes only the spare leapfrog level, so the state does not change),
  * keep the fastest and return it (tx, ty, ms of the best step; may be NULL).
+ * Where no kernel of the scheme has a shape (hyc_ens_set_tile), the shape as
+ * it is, timed once.
  */
 int hyc_ens_tune(hyc_ens *ens, int32_t advtyp, double delt1, int32_t *tx, int32_t *ty, double *ms);
 /*

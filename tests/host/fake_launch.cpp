@@ -10,31 +10,40 @@
 #include "fake_cuda.h"
 #include "fake_launch.h"
 
-int fake_fail_launches = 0;
+int fake_fail_launches = 0, fake_step_launches = 0, fake_maps = 0;
+bool fake_strip = true;
+
+static bool step_launch() {  // counted; false where it is to fail
+  fake_step_launches++;
+  return !(fake_fail_launches > 0 && --fake_fail_launches == 0);
+}
 
 namespace hyc {
 
 bool tmap_available() { return true; }
-bool tmap_encode3(CUtensorMap *, const void *, int, long long, long long, long long, long long, long long, int, int) { return true; }
+bool tmap_encode3(CUtensorMap *, const void *, int, long long, long long, long long, long long, long long, int, int) {
+  fake_maps++;
+  return true;
+}
 void set_library_error(const char *) {}
-bool march_takes(int, const TileArgs &, int) { return true; }
+bool march_takes(int, const TileArgs &, int) { return fake_strip; }
 cudaError_t launch_xctilr(double *a, long long, int, int, int, int, int, int, int, int, cudaStream_t s) {
   fake::use(a, s);
   return cudaSuccess;
 }
 cudaError_t launch_march_queue(int, const TileArgs *basins, const int4 *items, int, int *head, int, cudaStream_t s) {
-  if (fake_fail_launches > 0 && --fake_fail_launches == 0) return cudaErrorInvalidValue;
+  if (!step_launch()) return cudaErrorInvalidValue;
   for (const void *p : {(const void *)basins, (const void *)items, (const void *)head}) fake::use(p, s);
   return cudaSuccess;
 }
 cudaError_t launch_mix_col2(int, const MixBasin *basins, const int4 *items, int, int *head, int, int, bool, bool, int *err,
                             cudaStream_t s) {
-  if (fake_fail_launches > 0 && --fake_fail_launches == 0) return cudaErrorInvalidValue;
+  if (!step_launch()) return cudaErrorInvalidValue;
   for (const void *p : {(const void *)basins, (const void *)items, (const void *)head, (const void *)err}) fake::use(p, s);
   return cudaSuccess;
 }
 cudaError_t launch_advect_tiles(int, const TileArgs &a, int, TileShape, cudaStream_t s, bool) {
-  if (fake_fail_launches > 0 && --fake_fail_launches == 0) return cudaErrorInvalidValue;
+  if (!step_launch()) return cudaErrorInvalidValue;
   fake::use(a.out, s);
   return cudaSuccess;
 }

@@ -38,7 +38,8 @@ int main(int, char **argv) {
     OK(hyc_ens_step(e, 2, 1800.0, 3, 1));
     int tx, ty;
     double ms;
-    fake_fail_launches = 6;  // the second shape's
+    fake_strip = false;      // MPDATA in the tile kernel: two shapes
+    fake_fail_launches = 6;  // the second one's
     if (hyc_ens_tune(e, 1, 1800.0, &tx, &ty, &ms) == HYC_OK) return 3;
     OK(hyc_ens_step(e, 2, 1800.0, 3, 1));
   } else if (!strcmp(argv[1], "no-memory")) {  // the queue counters cannot grow
