@@ -56,10 +56,11 @@ struct TileArgs {
   int nfld;
   int seg;  // rows per segment of the strip kernel's queue
   // output: out + (fi*kdm + k)*slice; sea cells of the interior are written
+  // (PCM and MPDATA: land cells too, with their old value)
   double *out;
   int kdm;
-  // >0: also write the periodic-x halo images of output cells with
-  // i <= images or i > ii-images (an ensemble level is its own halo source)
+  // >0, FCT strip kernel: also write the periodic-x halo images of output cells
+  // with i <= images or i > ii-images (an ensemble level is its own halo source)
   int images;
   FieldDesc f[kMaxFields];  // last: the strip kernel's queue stages what is before it
 };

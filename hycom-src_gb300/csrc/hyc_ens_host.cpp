@@ -34,7 +34,6 @@ struct EBasin {
   double *cell = nullptr;                       // strip kernel per-cell words (mixed form)
   float2 *gd = nullptr;                         // diffusion grid table of the strip kernel (mixed form)
   double temdf2 = 0.0;                          // lateral diffusion after each step (0: none)
-  long long work = 0;                           // cells*layers*tracers, for queue ordering
   std::vector<double> posdef;                   // MPDATA offset per tracer (0 unless set)
   std::vector<uint8_t> sea;                     // strip kernel: [strip][row] has sea among the columns it updates
 };
@@ -630,7 +629,6 @@ int hyc_ens_create(hyc_ens **out, int32_t nbasin, const hyc_basin_spec *specs, i
     b.ld1 = (b.ld1r + align - 1) / align * align;
     b.ld2 = s.jdm + 2 * s.nbdy;
     b.slice = (long long)b.ld1 * b.ld2;
-    b.work = (long long)s.idm * s.jdm * s.kdm * s.ntr;
     b.posdef.assign(s.ntr, 0.0);
     maxk = std::max(maxk, s.kdm);
     e->maxntr = std::max(e->maxntr, s.ntr);

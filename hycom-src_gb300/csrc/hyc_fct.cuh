@@ -376,12 +376,7 @@ __device__ __forceinline__ bool fct_tile_body(const TileArgs &A, const int tile,
       if (i > ii || j > jj || !(MSK[e] & kIP)) return;
       const double fdv = mul_rn(mul_rn((FX[e + 1] - FX[e]) + (FY[e + RX] - FY[e]), dt2), SCI[e]);
       const double res = from_dkey(max(qn[it], min(qx[it], dkey(FLO[e] - div_by(fdv, HN[e], RC[e])))));
-      const long long o = (long long)(i + nb - 1) + (long long)(j + nb - 1) * ld1;
-      out[o] = res;
-      if (A.images) {  // periodic in x: the xctilr copy (mod_xc_sm.h:1415-1421) written here
-        if (i <= A.images) out[o + ii] = res;
-        if (i > ii - A.images) out[o - ii] = res;
-      }
+      out[(long long)(i + nb - 1) + (long long)(j + nb - 1) * ld1] = res;
     });
     __syncthreads();
   }

@@ -140,13 +140,6 @@ bool advect_tiles_tma(int scheme, TileShape t) {
   return TileGeom<16, 16>::TMA;
 }
 
-size_t advect_tiles_smem(TileShape t) {
-  if (t.tx == 32 && t.ty == 16) return TileGeom<32, 16>::smem_bytes;
-  if (t.tx == 32 && t.ty == 32) return TileGeom<32, 32>::smem_bytes;
-  if (t.tx == 16 && t.ty == 16) return TileGeom<16, 16>::smem_bytes;
-  return 0;
-}
-
 // The shape of a launch that goes to a tile kernel, and whether its region is
 // staged by TMA, where the caller fixed no shape.  Up to one 32x16 tile an SM
 // a launch is all latency: 16x16 tiles halve a CTA's passes, and plain loads

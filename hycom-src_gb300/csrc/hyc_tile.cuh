@@ -1,22 +1,22 @@
 // hyc_tile.cuh -- fused shared-memory tile kernel for advem's schemes (FP64).
 //
 // One CTA owns an output tile of TX x TY cells of one layer and stages a
-// region of (TX+6) x (TY+6) cells in shared memory: every scheme here (PCM,
-// MPDATA, FCT2, FCT4) needs inputs at most 3 cells from the cells it
-// updates (fld_new(i) <- limiter ratios at i+-1 <- low-order bounds at i+-2
-// <- 5-point extrema of fld at i+-3).  All stages of a scheme then run out
+// region of (TX+6) x (TY+6) cells in shared memory: PCM and MPDATA need inputs
+// at most 3 cells from the cells they update (fld_new(i) <- limiter ratios at
+// i+-1 <- low-order bounds at i+-2 <- 5-point extrema of fld at i+-3).  All stages of a scheme then run out
 // of shared memory with a shrinking valid region, and only the updated
 // field goes back to HBM.  The per-layer quantities (fluxes, thicknesses,
 // reciprocal thickness, metrics, masks) are staged once and reused by every
 // tracer of the layer.
 //
-// Stage-to-reference map (FCT2, mod_tsadvc.F90:645-997):
-//   S1  upwind face fluxes                         :686-720 (+ :738-758)
-//   S2  5-pt extrema, low-order fldlo, fmxlo/fmnlo :778-797
-//   S3  high-order minus low-order flux fax/fay    :817-855
-//   S4  Zalesak bounds, famax/famin, rp/rm         :863-909
-//   S5  flux limiting                              :922-946
-//   S6  corrected update, clip to [fqmin,fqmax]    :962-982
+// Stage-to-reference map (MPDATA, mod_tsadvc.F90:207-493; PCM ends with S2,
+// :610-630):
+//   S1  upwind face fluxes, tx1/ty1                :248-270
+//   S2  5-pt extrema, divergence, low-order fldlo  :277-352
+//   S3  antidiffusive fluxes                       :377-387
+//   S4  limiter ratios rp/rm                       :411-419
+//   S5  flux limiting                              :440-441
+//   S6  corrected update, clip to the extrema      :465-486
 // Face fluxes are stored as zero on faces that are not between two sea
 // cells; this is what the reference's section-edge zeroing
 // (mod_tsadvc.F90:738-758) produces for every face its stencils read.
@@ -30,9 +30,10 @@
 // waits) when the launch carries tensor maps and the shape allows it
 // (TileGeom::TMA), else by plain loads.
 //
-// It serves MPDATA launches too small for the strip kernel (hyc_march.cuh)
-// and the isopycnic layer-1 launches with a second pair of fluxes; FCT2 and
-// FCT4 have a tile kernel of their own (hyc_fct.cuh).
+// It serves MPDATA launches too small for the strip kernel (hyc_march.cuh), the
+// isopycnic layer-1 launches with a second pair of fluxes, and both schemes in
+// a shape that the caller fixes; FCT2 and FCT4 have a tile kernel of their own
+// (hyc_fct.cuh).
 #pragma once
 #include <cuda.h>
 
@@ -57,6 +58,7 @@ __device__ __forceinline__ void for_rect(int a0, int a1, int b0, int b1, F f) {
 
 template <int SCHEME, int TX, int TY>
 __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
+  static_assert(SCHEME == kPCM || SCHEME == kMPDATA, "fct_tile_kernel has the others");
   after_previous();
   using G = TileGeom<TX, TY>;
   constexpr int RX = G::RX, RW = G::RW, RY = G::RY, N = G::N, NR = G::NR;
@@ -181,15 +183,12 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
     const FieldDesc fd = A.f[fi];
     if (k + 1 > fd.kmax || k + 1 < fd.kmin) continue;  // uniform across the CTA
     const double *fn = fd.nbase + (long long)(k + fd.k_off) * sl;
-    const double *fm = fd.mbase + (long long)(k + fd.k_off) * sl;
     const double posdef = fd.posdef;
-    constexpr bool CENTRE = SCHEME != kPCM && SCHEME != kMPDATA;
     if (tm) {  // the previous field's readers passed the barrier that ends its loop
       if (threadIdx.x == 0) {
         tma::fence_proxy_async();
-        tma::expect_tx(&bar, (CENTRE ? 2u : 1u) * G::BOX);
+        tma::expect_tx(&bar, G::BOX);
         tma::load3(FLD - off, tm + 6 + 2 * fi, &bar, x0 - off, y0, k + fd.k_off);
-        if (CENTRE) tma::load3(FLDC - off, tm + 7 + 2 * fi, &bar, x0 - off, y0, k + fd.k_off);
       }
     }
     for (int t = threadIdx.x; t < NR; t += blockDim.x) {
@@ -199,7 +198,6 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
         bool in = (i >= 1 - nb) && (i <= A.ii + nb) && (j >= 1 - nb) && (j <= A.jj + nb);
         long long o = in ? (long long)(i + nb - 1) + (long long)(j + nb - 1) * ld1 : 0;
         FLD[t] = in ? fn[o] : 0.0;
-        if (CENTRE) FLDC[t] = in ? fm[o] : 0.0;
       }
       FX[t] = 0.0;
       FY[t] = 0.0;
@@ -276,22 +274,13 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
       double fmx = kmax(kmax(kmax(kmax(c, w), ea), s), nn);
       double fmn = kmin(kmin(kmin(kmin(c, w), ea), s), nn);
       double fdv = ((FX[e + 1] - FX[e]) + (FY[e + RX] - FY[e])) * dt2 * SCI[e];
-      if (SCHEME == kMPDATA) {
-        fmx = fmx + posdef;  // :277-280
-        fmn = fmn + posdef;
-        double q = (c + posdef) * (FCO[e] + kOnemu) - fdv;  // :350
-        FLO[e] = kmax(fmn, kmin(fmx, div_rcp(q, HN[e], RH[e])));
-        FLDC[e] = fdv;  // flxdiv, read by neighbours in S3
-        QX[e] = fmx;
-        QN[e] = fmn;
-      } else {
-        double q = c * (FCO[e] + kOnemu) - fdv;  // :788
-        double lo = kmax(fmn, kmin(fmx, div_rcp(q, HN[e], RH[e])));
-        FLO[e] = lo;
-        double cc = FLDC[e];
-        FXL[e] = kmax(kmax(c, cc), lo);  // fmxlo, :792
-        FNL[e] = kmin(kmin(c, cc), lo);  // fmnlo, :793
-      }
+      fmx = fmx + posdef;  // :277-280
+      fmn = fmn + posdef;
+      double q = (c + posdef) * (FCO[e] + kOnemu) - fdv;  // :350
+      FLO[e] = kmax(fmn, kmin(fmx, div_rcp(q, HN[e], RH[e])));
+      FLDC[e] = fdv;  // flxdiv, read by neighbours in S3
+      QX[e] = fmx;
+      QN[e] = fmn;
     });
     __syncthreads();
 
@@ -301,35 +290,17 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
       uint8_t m = MSK[e];
       if (!(m & kIU)) return;
       double uu = U[e];
-      if (SCHEME == kMPDATA) {  // :377-381
-        double fco2 = FCO[e] + FCO[e - 1];
-        double fcn2 = FCN[e] + FCN[e - 1];
-        FX[e] = FXL[e] - div_rn(uu * (FLDC[e] + FLDC[e - 1]), (fco2 + fcn2) + kOnemu);
-      } else if (SCHEME == kFCT4 && (MSK[e - 1] & kIU) && (MSK[e + 1] & kIU)) {  // :1540-1541
-        const double ft14 = 7.0 / 12.0, ft24 = -1.0 / 12.0;
-        double fhx = uu * (ft14 * (FLDC[e] + FLDC[e - 1]) + ft24 * (FLDC[e + 1] + FLDC[e - 2]));
-        FX[e] = fhx - FX[e];
-      } else {  // :824-825
-        double fhx = uu * 0.5 * (FLDC[e] + FLDC[e - 1]);
-        FX[e] = fhx - FX[e];
-      }
+      double fco2 = FCO[e] + FCO[e - 1];  // :377-381
+      double fcn2 = FCN[e] + FCN[e - 1];
+      FX[e] = FXL[e] - div_rn(uu * (FLDC[e] + FLDC[e - 1]), (fco2 + fcn2) + kOnemu);
     });
     for_rect<RX>(2, RW - 2, 2, RY - 1, [&](int a, int b, int e) {
       uint8_t m = MSK[e];
       if (!(m & kIV)) return;
       double vv = V[e];
-      if (SCHEME == kMPDATA) {  // :383-387
-        double fco2 = FCO[e] + FCO[e - RX];
-        double fcn2 = FCN[e] + FCN[e - RX];
-        FY[e] = FNL[e] - div_rn(vv * (FLDC[e] + FLDC[e - RX]), (fco2 + fcn2) + kOnemu);
-      } else if (SCHEME == kFCT4 && (MSK[e - RX] & kIV) && (MSK[e + RX] & kIV)) {  // :1551-1552
-        const double ft14 = 7.0 / 12.0, ft24 = -1.0 / 12.0;
-        double fhy = vv * (ft14 * (FLDC[e] + FLDC[e - RX]) + ft24 * (FLDC[e + RX] + FLDC[e - 2 * RX]));
-        FY[e] = fhy - FY[e];
-      } else {
-        double fhy = vv * 0.5 * (FLDC[e] + FLDC[e - RX]);
-        FY[e] = fhy - FY[e];
-      }
+      double fco2 = FCO[e] + FCO[e - RX];  // :383-387
+      double fcn2 = FCN[e] + FCN[e - RX];
+      FY[e] = FNL[e] - div_rn(vv * (FLDC[e] + FLDC[e - RX]), (fco2 + fcn2) + kOnemu);
     });
     __syncthreads();
 
@@ -337,50 +308,15 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
     for_rect<RX>(2, RW - 2, 2, RY - 2, [&](int a, int b, int e) {
       uint8_t m = MSK[e];
       if (!(m & kIP)) return;
-      if (SCHEME == kMPDATA) {  // :411-419
-        double fx0 = FX[e], fx1 = FX[e + 1], fy0 = FY[e], fy1 = FY[e + RX];
-        double flxdp = neg0(fx1) - pos0(fx0);
-        double flxdn = pos0(fx1) - neg0(fx0);
-        double flydp = neg0(fy1) - pos0(fy0);
-        double flydn = pos0(fy1) - neg0(fy0);
-        double lo = FLO[e];
-        double fs = FCN[e] * SCL[e];
-        RP[e] = div_rn((QX[e] - lo) * fs, (kOnemu - (flxdp + flydp)) * dt2);
-        RM[e] = div_rn((lo - QN[e]) * fs, (kOnemu + (flxdn + flydn)) * dt2);
-        return;
-      }
-      const bool mw = MSK[e - 1] & kIP, me = MSK[e + 1] & kIP, ms = MSK[e - RX] & kIP, mn = MSK[e + RX] & kIP;
-      double fqmax = FXL[e], fqmin = FNL[e];
-      // fqmax = max(fmxlo(i,j),fmxlo(ia,j),fmxlo(ib,j),fmxlo(i,ja),fmxlo(i,jb)), :876-879
-      fqmax = kmax(fqmax, mw ? FXL[e - 1] : FXL[e]);
-      fqmax = kmax(fqmax, me ? FXL[e + 1] : FXL[e]);
-      fqmax = kmax(fqmax, ms ? FXL[e - RX] : FXL[e]);
-      fqmax = kmax(fqmax, mn ? FXL[e + RX] : FXL[e]);
-      fqmin = kmin(fqmin, mw ? FNL[e - 1] : FNL[e]);
-      fqmin = kmin(fqmin, me ? FNL[e + 1] : FNL[e]);
-      fqmin = kmin(fqmin, ms ? FNL[e - RX] : FNL[e]);
-      fqmin = kmin(fqmin, mn ? FNL[e + RX] : FNL[e]);
-      // ib=ipip1, jb=ipjp1: a sea cell with land to the E (N) reads its own
-      // west (south) face twice, mod_tsadvc.F90:880-883.
-      double fxa = FX[e], fxb = me ? FX[e + 1] : FX[e];
-      double fya = FY[e], fyb = mn ? FY[e + RX] : FY[e];
-      double famax = pos0(fxa) - neg0(fxb) + pos0(fya) - neg0(fyb);
-      double famin = pos0(fxb) - neg0(fxa) + pos0(fyb) - neg0(fya);
+      double fx0 = FX[e], fx1 = FX[e + 1], fy0 = FY[e], fy1 = FY[e + RX];  // :411-419
+      double flxdp = neg0(fx1) - pos0(fx0);
+      double flxdn = pos0(fx1) - neg0(fx0);
+      double flydp = neg0(fy1) - pos0(fy0);
+      double flydn = pos0(fy1) - neg0(fy0);
       double lo = FLO[e];
-      double qdt2 = A.qdt2;
-      double rp = 0.0, rm = 0.0;
-      if (gt0(famax)) {
-        double qp = (fqmax - lo) * FCN[e] * SCL[e] * qdt2;
-        rp = klt(qp, famax) ? div_rn(qp, famax) : 1.0;
-      }
-      if (gt0(famin)) {
-        double qm = (lo - fqmin) * FCN[e] * SCL[e] * qdt2;
-        rm = klt(qm, famin) ? div_rn(qm, famin) : 1.0;
-      }
-      RP[e] = rp;
-      RM[e] = rm;
-      QX[e] = fqmax;
-      QN[e] = fqmin;
+      double fs = FCN[e] * SCL[e];
+      RP[e] = div_rn((QX[e] - lo) * fs, (kOnemu - (flxdp + flydp)) * dt2);
+      RM[e] = div_rn((lo - QN[e]) * fs, (kOnemu + (flxdn + flydn)) * dt2);
     });
     __syncthreads();
 
@@ -388,26 +324,17 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
     for_rect<RX>(3, RW - 2, 3, RY - 3, [&](int a, int b, int e) {
       if (!(MSK[e] & kIU)) return;
       double f = FX[e];
-      if (SCHEME == kMPDATA) {  // :440-441
-        FX[e] = pos0(f) * kmin(kmin(1.0, RP[e]), RM[e - 1]) + neg0(f) * kmin(kmin(1.0, RP[e - 1]), RM[e]);
-      } else {  // :929-934
-        double fact = lt0(f) ? kmin(RP[e - 1], RM[e]) : kmin(RP[e], RM[e - 1]);
-        FX[e] = fact * f;
-      }
+      // :440-441
+      FX[e] = pos0(f) * kmin(kmin(1.0, RP[e]), RM[e - 1]) + neg0(f) * kmin(kmin(1.0, RP[e - 1]), RM[e]);
     });
     for_rect<RX>(3, RW - 3, 3, RY - 2, [&](int a, int b, int e) {
       if (!(MSK[e] & kIV)) return;
       double f = FY[e];
-      if (SCHEME == kMPDATA) {
-        FY[e] = pos0(f) * kmin(kmin(1.0, RP[e]), RM[e - RX]) + neg0(f) * kmin(kmin(1.0, RP[e - RX]), RM[e]);
-      } else {
-        double fact = lt0(f) ? kmin(RP[e - RX], RM[e]) : kmin(RP[e], RM[e - RX]);
-        FY[e] = fact * f;
-      }
+      FY[e] = pos0(f) * kmin(kmin(1.0, RP[e]), RM[e - RX]) + neg0(f) * kmin(kmin(1.0, RP[e - RX]), RM[e]);
     });
     __syncthreads();
 
-    // S6: corrected update on the output cells, :962-982 (MPDATA :465-486)
+    // S6: corrected update on the output cells, :465-486
     for_rect<RX>(3, RW - 3, 3, RY - 3, [&](int a, int b, int e) {
       int i = ib0 + a, j = jb0 + b;
       if (i > A.ii || j > A.jj) return;
@@ -415,7 +342,7 @@ __global__ void __launch_bounds__(256, 1) advect_tile_kernel(const TileArgs A) {
       if (MSK[e] & kIP) {
         double fdv = ((FX[e + 1] - FX[e]) + (FY[e + RX] - FY[e])) * dt2 * SCI[e];
         res = kmax(QN[e], kmin(QX[e], FLO[e] - div_rcp(fdv, HN[e], RH[e])));
-        if (SCHEME == kMPDATA) res = res - posdef;
+        res = res - posdef;
       }
       A.out[((long long)fi * A.kdm + k) * sl + (long long)(i + nb - 1) + (long long)(j + nb - 1) * ld1] = res;
     });
