@@ -669,8 +669,8 @@ size_t cnuity_work_slices(int nbatch) { return W_FIX + (size_t)B_N * nbatch; }
 // 696), 600x450x41 3737 / 2784 (2786), 1500x1100x41 16.9 / 14.9 ms (14.9),
 // 3000x2200x10 15.1 / 14.2 (14.5).
 int cnuity_batch(long long slice, int kdm) {
-  const long long n = (1LL << 30) / (B_N * 8 * slice);
-  return (int)(n < 1 ? 1 : n > kdm ? kdm : n);
+  const long long n = (1LL << 30) / (B_N * 8 * slice), most = kdm < 65535 ? kdm : 65535;  // the grid's limit
+  return (int)(n < 1 ? 1 : n > most ? most : n);
 }
 
 cudaError_t launch_cnuity_layers(const CnuityArgs &a0, int *launches, cudaStream_t s) {
