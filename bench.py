@@ -344,8 +344,9 @@ def run_ensemble_forms(args, wl, b, masks, spec, case, dev, stream, dist, local,
         tkey = TRAFFIC_KEY.get(form)
         out[form] = {"value": ws * ups_step / (ms / 1e3), "unit": UNIT, "ms_per_step": ms, "advtyp": adv,
                      "traffic_bytes_per_launch": profile_traffic(f"{tkey}_{args.workload}") if tkey else None,
-                     "tile": [tx, ty],
-                     "tracers_per_pass": nq, "kernel": KERNEL_OF_FORM.get(form, "fct tile/queue kernel (FP64)"),
+                     "tile": [tx, ty],  # (without effect on the FP64 strip kernels)
+                     "tracers_per_pass": nq, "kernel": KERNEL_OF_FORM.get(
+                         form, "march_queue_kernel (FP64)" if adv in (2, 4) else "march_kernel, a basin a launch (FP64)"),
                      "algorithmic_bytes_per_update": bpu, "achieved_GBs": ach, "frac_of_measured_hbm": ach / peak,
                      "graph_steps": args.steps, "clocks": clk.summary(),
                      "content_change_one_step": {n: abs(c_new[q] - c_old[q]) / abs(c_old[q])
@@ -1272,9 +1273,15 @@ def main():
         peak, peak_kind = peak_hbm()
         prec = ENS_FORMS[args.form][0]
         key = TRAFFIC_KEY.get(args.form)
-        roof = {"bound": "hbm", "achieved": head["achieved_GBs"], "peak": peak, "unit": "GB/s",
-                "frac": head["frac_of_measured_hbm"],
-                "traffic": profile_traffic(f"{key}_{args.workload}") if key else None,
+        # value counts every interior cell, land among them; the strip kernel leaves out rows of land, so
+        # only the sea cells' bytes are ones the launch cannot do without
+        sea = sea_cells / (wl["nx"] * wl["ny"])
+        traffic = profile_traffic(f"{key}_{args.workload}") if key else None
+        roof = {"bound": "hbm", "achieved": head["achieved_GBs"] * sea, "peak": peak, "unit": "GB/s",
+                "frac": head["frac_of_measured_hbm"] * sea, "counts": "bytes of the sea cells' updates",
+                "sea_fraction": sea, "frac_of_every_cell": head["frac_of_measured_hbm"],
+                "traffic": traffic,
+                "dram_frac": traffic / head["ms_per_step"] / 1e6 / peak if traffic else None,
                 "peak_kind": peak_kind, "kernel": head["kernel"],
                 "algorithmic_bytes_per_update": head["algorithmic_bytes_per_update"],
                 "avg_launch_ms": head["ms_per_step"], "tile": head["tile"],
