@@ -52,15 +52,17 @@ __device__ __forceinline__ bool klt(double a, double b) { return dkey(a) < dkey(
 
 // FP32 bounds of a double for tests that need no exact value (integer pipes:
 // a conversion instruction would issue at the FP64 rate).  Both truncate
-// (relative error below 2^-23).  f32_below: of a value >= 0, at most x, and 0
-// where x is negative, NaN or outside FP32's normal range.
+// towards zero (relative error below 2^-23).  f32_below: of a value >= 0, at
+// most x, and 0 where x is negative, NaN or outside FP32's normal range.
 __device__ __forceinline__ float f32_below(double x) {
   const uint32_t h = (uint32_t)__double2hiint(x);
   const uint32_t f = __funnelshift_l((uint32_t)__double2loint(x), h, 3) + 0x40000000u;
   return h - 0x38100000u < 0x0FE00000u ? __uint_as_float(f) : 0.0f;
 }
-// f32_away: 0 only where x is 0; below FP32's normal range the smallest
-// normal, above it (and for NaN) infinity
+// f32_away: away from zero where it matters, not in the last bit: 0 only where
+// x is 0, below FP32's normal range the smallest normal, above it (and for NaN)
+// infinity; in the range the truncation leaves it up to 2^-23 short, which the
+// tests' factors (1.000004) cover
 __device__ __forceinline__ float f32_away(double x) {
   const uint32_t h = (uint32_t)__double2hiint(x), l = (uint32_t)__double2loint(x), m = h & 0x7FFFFFFFu;
   uint32_t f = __funnelshift_l(l, h, 3) + 0x40000000u;
